@@ -40,6 +40,9 @@ namespace {
 
 constexpr int kThreads = brick::kThreads;
 
+// Hit words per lane of the traversal for a tile's list depth (64 as the single-box kernel).
+__host__ __device__ constexpr int hit_words(int list_cap) { return list_cap == 32 ? 16 : brick::kHitWords; }
+
 // Per-box entry of the device table.
 struct BatchBox {
 	brick::Box bx;
@@ -387,12 +390,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch_step(StepArgs a) {
 
 	if (!a.skin) {
 		// ---- B: pair forces of every brick (filter and evaluation) ----------------------------
-		const brick::SmemLayout L = brick::layout(a.pc.s_cap, kFP64, kCap);
+		const brick::SmemLayout L = brick::layout(a.pc.s_cap, true, hit_words(kCap));
 		brick::load_params(smem, L, a.pp, a.pc.ns);
 		__syncthreads();
 		for_bricks(2, [&](int item) {
 			const BatchBox& B = a.boxes[box_of(item)];
-			brick::pairs<kFP64, kSingle, kLjIsRc, kCap, false>(a.pc, B.bx, item - B.brick0, item, smem, a.dst.rx, a.dst.ry,
+			brick::pairs<kSingle, kLjIsRc, hit_words(kCap)>(a.pc, B.bx, item - B.brick0, item, smem, a.dst.rx, a.dst.ry,
 			                                            a.dst.rz, a.dst.cid, a.cstart, a.dst.fx, a.dst.fy, a.dst.fz,
 			                                            a.partials, a.status);
 			__syncthreads();
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch_step(StepArgs a) {
 		});
 		if (!grid_barrier(a.bar, a.status, a.timeout_ns, &s_flag)) return;
 		// ---- B2: list evaluation of every brick -----------------------------------------------
-		const brick::SmemLayout L = brick::layout(a.lc.s_cap, kFP64, 0, false);
+		const brick::SmemLayout L = brick::layout(a.lc.s_cap, kFP64);
 		brick::load_params(smem, L, a.pp, a.lc.ns);
 		if (threadIdx.x == 0)
 			reinterpret_cast<float4*>(smem + L.hi)[a.lc.s_cap] =
@@ -438,6 +441,7 @@ using StepKernel = void (*)(StepArgs);
 
 template <int kCap>
 StepKernel pick(bool fp64, bool single, bool ljrc) {
+	if (fp64 && ljrc) return single ? k_batch_step<true, true, true, kCap> : k_batch_step<true, false, true, kCap>;
 	if (fp64) return single ? k_batch_step<true, true, false, kCap> : k_batch_step<true, false, false, kCap>;
 	if (ljrc) return single ? k_batch_step<false, true, true, kCap> : k_batch_step<false, false, true, kCap>;
 	return single ? k_batch_step<false, true, false, kCap> : k_batch_step<false, false, false, kCap>;
@@ -650,16 +654,16 @@ int plan(Batch* b, const Tiles& t, Launch& L) {
 	size_t budget = t.ctas == 1 ? 220 * 1024 : 110 * 1024;
 	if (budget > (size_t) b->max_optin) budget = (size_t) b->max_optin;
 	if (b->max_bin_bytes > budget) return bfail(b, MDGPU_ERR_CAPACITY, "a box is too large for this tile shape");
-	const int s_cap = brick::capacity_for(budget, fp64, t.cap);
+	const int s_cap = brick::capacity_for(budget, true, hit_words(t.cap));
 	L.pc = brick::make_const(b->sp.n, s_cap, b->rc, b->rc_lj);
-	L.smem = std::max(brick::layout(s_cap, fp64, t.cap).total, b->max_bin_bytes);
+	L.smem = std::max(brick::layout(s_cap, true, hit_words(t.cap)).total, b->max_bin_bytes);
 	if (b->skin > 0.0) {
-		const int lcap = brick::capacity_for(budget, fp64, 0, false);
+		const int lcap = brick::capacity_for(budget, fp64);
 		L.lc = brick::make_const(b->sp.n, lcap, b->rc, b->rc_lj);
 		int bcap = 256;
 		while (brick::build_bytes(bcap + 64) <= budget) bcap += 64;
 		L.build_cap = bcap;
-		L.smem = std::max({brick::layout(lcap, fp64, 0, false).total, brick::build_bytes(bcap), b->max_bin_bytes});
+		L.smem = std::max({brick::layout(lcap, fp64).total, brick::build_bytes(bcap), b->max_bin_bytes});
 	}
 	B_CUDA(cudaFuncSetAttribute(L.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) L.smem));
 	int per_sm = 0;

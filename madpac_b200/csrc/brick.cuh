@@ -1,28 +1,27 @@
 // Pair traversal of one brick of 2x2x2 linked cells staged in shared memory (device function used
-// by the single-box pair kernel and by the persistent multi-box step kernel).
+// by the single-box pair kernels and by the persistent multi-box step kernel).
 //
-// One CTA (8 warps) owns a brick of 2x2x2 cells; each warp owns one of its cells and computes the
-// full force on that cell's molecules from every molecule of the 27 surrounding cells (periodic
-// images at +-L, r_j + L / r_j - L as DomainDecompDummy::exchangeMolecules places halo images,
-// parallel/DomainDecompDummy.cpp:64-70, 93-99; paths relative to madpac/mardyn/). Per brick:
+// One CTA (8 warps) owns a brick of 2x2x2 cells and computes the full force on its molecules from every
+// molecule of the 27 cells around theirs (periodic images at +-L, r_j + L / r_j - L as
+// DomainDecompDummy::exchangeMolecules places halo images, parallel/DomainDecompDummy.cpp:64-70, 93-99;
+// paths relative to madpac/mardyn/). Two ways lead there:
 //
-//  staging  The 4x4x4 cells around the brick are copied to shared memory cell by cell (x fastest),
-//           so the 3 cells of each neighbour row of a cell form one contiguous slot range.
-//           Positions are stored in a local frame
-//           X = x + shift - c_brick + C, C = 1.5 * 2^k with all X of the region in [2^k, 2^(k+1)]:
-//           differences of their float "hi" parts are exact (Sterbenz), and the "lo" part X - hi
-//           is kept as 9-bit fixed point (steps of 1/512 ulp of the binade) in the 4th word of the
-//           same float4, with the component id: (hi_i - hi_j) + (lo_i - lo_j) is X_i - X_j to
-//           about 2e-9 absolute, one 16-byte shared load per candidate. The FP64 mode also stages
-//           the double image position x + shift.
-//  filter   Each lane holds one molecule i; every pair of consecutive staged molecules j of the 9
-//           neighbour rows is broadcast to all lanes, which test r^2 in packed half precision
-//           against rc^2 plus a margin covering the rounding, and append hits to their own list.
-//  compute  When a list fills (or at the end), every lane evaluates its list: the exact cutoff test
-//           (dd < rc^2, strict as BlockTraverse.cpp:155) and PotForceLJ (molecules/potforce.h:41-53)
-//           -- in FP64 with the reference's operation order, or in FP32 with FP64 accumulation.
-//  fallback A brick whose region holds more molecules than the shared-memory capacity computes
-//           its cells by gathering straight from global memory (same per-pair arithmetic).
+//  pairs       the drop-in traversal, every call: staging of the 4x4x4 cells around the brick, a packed
+//              half-precision filter over the rows of 3 cells around each molecule's cell (rc plus a
+//              margin covering the rounding) and the exact evaluation of its hits in FP64.
+//  list_pairs  the Verlet-skin steps: the lists that build_lists made with the same filter are evaluated
+//              at the current positions, in FP64 or (mixed form) in FP32 with FP64 accumulation.
+//
+// Staging copies the region's molecules to shared memory cell by cell (x fastest), so the 3 cells of each
+// neighbour row of a cell form one contiguous slot range. The FP64 evaluations read the double image
+// position x + shift. The FP32 lists read a local frame X = x + shift - c_brick + C, C = 1.5 * 2^k with
+// all X of the region in [2^k, 2^(k+1)]: differences of their float "hi" parts are exact (Sterbenz), and
+// the "lo" part X - hi is kept as 9-bit fixed point (steps of 1/512 ulp of the binade) in the 4th word
+// of the same float4, with the component id: (hi_i - hi_j) + (lo_i - lo_j) is X_i - X_j to about 2e-9
+// absolute, one 16-byte shared load per candidate.
+// The exact cutoff test is dd < rc^2, strict as BlockTraverse.cpp:155, decided in FP64 as the reference
+// decides it; the force law is PotForceLJ's (molecules/potforce.h:41-53). A brick whose region holds more
+// molecules than the shared-memory capacity gathers straight from global memory instead.
 //
 // Each unordered pair is evaluated from both sides; energy and virial are halved on readout.
 // Orders of staging, enumeration and accumulation are fixed: results are deterministic and do not
@@ -71,7 +70,7 @@ struct Box {
 };
 
 struct SmemLayout {
-	size_t hi, lo, img, h16, cstart, lists, ccount, gstart, cell_k, cell_shift, params, total;
+	size_t hi, img, comp, h16, cstart, lists, ccount, gstart, cell_k, cell_shift, params, total;
 };
 
 // Two consecutive staged molecules in half precision, relative to the brick centre: the packed
@@ -82,30 +81,34 @@ struct __align__(16) HalfPair {
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
-// list_cap: per-lane candidate list depth of the filter (0 for the list kernel, which reads its
-// lists from global memory); half: whether the packed half-precision copy is staged.
-__host__ __device__ inline SmemLayout layout(int s_cap, bool fp64, int list_cap, bool half = true) {
+// Shared memory of the list kernels (they read their lists from global memory): the hi/lo positions
+// with the far-away sentinel slot past the capacity, and in the FP64 form the double images.
+// With words > 0 that of the traversal (pairs, fp64): the packed half-precision copy for its filter, the
+// double images, the component ids and `words` hit words per lane.
+__host__ __device__ inline SmemLayout layout(int s_cap, bool fp64, int words = 0) {
 	SmemLayout L;
 	size_t o = 0;
+	const bool traverse = words > 0;
 	L.hi = o;
-	o = align16(o + sizeof(float4) * (s_cap + 1));   // + the far-away sentinel slot of the list kernel
-	L.lo = o;
+	if (!traverse) o = align16(o + sizeof(float4) * (s_cap + 1));
 	L.img = o;
 	if (fp64) o = align16(o + sizeof(double) * 3 * s_cap);
+	L.comp = o;
+	if (traverse) o = align16(o + s_cap);
 	L.h16 = o;
-	if (half) o = align16(o + sizeof(HalfPair) * (s_cap / 2 + 20));  // 32-slot blocks may read past the end
+	if (traverse) o = align16(o + sizeof(HalfPair) * (s_cap / 2 + 20));  // 16-slot blocks may read past the end
 	L.cstart = o;
 	o = align16(o + sizeof(int) * 65);
 	L.lists = o;
-	o = align16(o + sizeof(unsigned short) * kWarps * list_cap * 32);
+	if (traverse) o = align16(o + sizeof(unsigned) * kThreads * (words + 1));   // one past the last is read
 	L.ccount = o;
 	o = align16(o + sizeof(int) * 64);
 	L.gstart = o;
 	o = align16(o + sizeof(int) * 64);
 	L.cell_k = o;
-	o = align16(o + sizeof(double) * 3 * 64);
+	if (!traverse) o = align16(o + sizeof(double) * 3 * 64);
 	L.cell_shift = o;
-	o = align16(o + sizeof(double) * 3 * 64);
+	if (!traverse) o = align16(o + sizeof(double) * 3 * 64);
 	L.params = o;
 	o = align16(o + sizeof(double) * 3 * KK + sizeof(float) * 3 * KK);
 	L.total = o;
@@ -113,9 +116,9 @@ __host__ __device__ inline SmemLayout layout(int s_cap, bool fp64, int list_cap,
 }
 
 // Largest staged capacity (a multiple of 64) whose layout fits in `budget` bytes.
-inline int capacity_for(size_t budget, bool fp64, int list_cap, bool half = true) {
+inline int capacity_for(size_t budget, bool fp64, int words = 0) {
 	int s_cap = 256;
-	while (layout(s_cap + 64, fp64, list_cap, half).total <= budget) s_cap += 64;
+	while (layout(s_cap + 64, fp64, words).total <= budget) s_cap += 64;
 	return s_cap > 65535 ? 65535 : s_cap;
 }
 
@@ -184,13 +187,14 @@ __device__ __forceinline__ void load_params(unsigned char* smem, const SmemLayou
 struct Smem {
 	float4* hi;
 	double* img;
+	unsigned char* comp;  // component ids (traversal)
 	HalfPair* h16;
 	__half* h;
 	int* cs;              // staged slot of each staged cell (65)
-	unsigned short* list;
+	unsigned* words;      // hit words of the traversal (a column per thread)
 	int* cnt;
 	int* gst;
-	double* ck;
+	double* ck;           // frame offset and image shift of each staged cell (list kernels)
 	double* csh;
 	double* pd;           // eps24, sig2, shift6 (double)
 	float* pf;            // the same as float
@@ -200,10 +204,11 @@ __device__ __forceinline__ Smem views(unsigned char* smem, const SmemLayout& L) 
 	Smem S;
 	S.hi = reinterpret_cast<float4*>(smem + L.hi);
 	S.img = reinterpret_cast<double*>(smem + L.img);
+	S.comp = smem + L.comp;
 	S.h16 = reinterpret_cast<HalfPair*>(smem + L.h16);
 	S.h = reinterpret_cast<__half*>(S.h16);
 	S.cs = reinterpret_cast<int*>(smem + L.cstart);
-	S.list = reinterpret_cast<unsigned short*>(smem + L.lists);
+	S.words = reinterpret_cast<unsigned*>(smem + L.lists);
 	S.cnt = reinterpret_cast<int*>(smem + L.ccount);
 	S.gst = reinterpret_cast<int*>(smem + L.gstart);
 	S.ck = reinterpret_cast<double*>(smem + L.cell_k);
@@ -246,46 +251,82 @@ __device__ __forceinline__ float3 unpack_lo(unsigned w, const Box& bx) {
 
 __device__ __forceinline__ int unpack_cid(unsigned w) { return (int) ((w >> 27) & 7u); }
 
-// Stages molecule e of staged cell c at double position (x, y, z), component q: the hi/lo frame
-// position, and the half-precision copy or the double image as the staging mode asks.
-// The same with the cell's frame offset (kx, ky, kz) and image shift (shx, shy, shz) given, at slot
-// slot_s.
-template <bool kFP64, bool kHalf>
-__device__ __forceinline__ void stage_at(const Const& p, const Box& bx, const Smem& S, int slot_s, double x, double y,
-                                         double z, int q, double kx, double ky, double kz, double shx, double shy,
-                                         double shz) {
+// What a staging stores: the list kernels' hi/lo frame positions, with the double images in the FP64
+// form, or the traversal's half-precision copy, double images and component ids.
+enum Staging { kStageList32, kStageList64, kStageTraverse };
+
+// Stages a molecule at double position (x, y, z), component q, at slot slot_s, with its cell's frame
+// offset (kx, ky, kz) and image shift (shx, shy, shz). For the traversal the offset is that of the
+// brick's centre, without the frame constant.
+template <Staging kMode>
+__device__ __forceinline__ void stage_at(const Box& bx, const Smem& S, int slot_s, double x, double y, double z, int q,
+                                         double kx, double ky, double kz, double shx, double shy, double shz) {
 	const double Xd = __dadd_rn(x, kx), Yd = __dadd_rn(y, ky), Zd = __dadd_rn(z, kz);
 	const float X = __double2float_rn(Xd), Y = __double2float_rn(Yd), Z = __double2float_rn(Zd);
-	const unsigned w = pack_lo(__double2float_rn(Xd - (double) X), __double2float_rn(Yd - (double) Y),
-	                           __double2float_rn(Zd - (double) Z), q, bx);
-	S.hi[slot_s] = make_float4(X, Y, Z, __uint_as_float(w));
-	if (kHalf) {
+	if (kMode == kStageTraverse) {
 		// half-precision copy relative to the brick centre (slot pairs share one HalfPair)
 		__half* hp = S.h + 8 * (slot_s >> 1) + (slot_s & 1);
-		hp[0] = __float2half_rn(X - bx.frame_c[0]);
-		hp[2] = __float2half_rn(Y - bx.frame_c[1]);
-		hp[4] = __float2half_rn(Z - bx.frame_c[2]);
+		hp[0] = __float2half_rn(X);
+		hp[2] = __float2half_rn(Y);
+		hp[4] = __float2half_rn(Z);
+		S.comp[slot_s] = (unsigned char) q;
+	} else {
+		const unsigned w = pack_lo(__double2float_rn(Xd - (double) X), __double2float_rn(Yd - (double) Y),
+		                           __double2float_rn(Zd - (double) Z), q, bx);
+		S.hi[slot_s] = make_float4(X, Y, Z, __uint_as_float(w));
 	}
-	if (kFP64) {
-		S.img[slot_s] = __dadd_rn(x, shx);
-		S.img[p.s_cap + slot_s] = __dadd_rn(y, shy);
-		S.img[2 * p.s_cap + slot_s] = __dadd_rn(z, shz);
+	if (kMode != kStageList32) {
+		S.img[3 * slot_s] = __dadd_rn(x, shx);
+		S.img[3 * slot_s + 1] = __dadd_rn(y, shy);
+		S.img[3 * slot_s + 2] = __dadd_rn(z, shz);
 	}
 }
 
-template <bool kFP64, bool kHalf>
-__device__ __forceinline__ void stage_one(const Const& p, const Box& bx, const Smem& S, int c, int e, double x,
-                                          double y, double z, int q) {
-	stage_at<kFP64, kHalf>(p, bx, S, S.cs[c] + e, x, y, z, q, S.ck[3 * c], S.ck[3 * c + 1], S.ck[3 * c + 2],
-	                       S.csh[3 * c], S.csh[3 * c + 1], S.csh[3 * c + 2]);
+// Staged coordinate l (0..3) of dimension d of a brick at coordinate b: the grid coordinate (periodic
+// wrap), the image shift of its molecules and their frame offset, X = x + k, k = shift - c_brick + C.
+__device__ __forceinline__ int staged_coord(const Box& bx, int d, int b, int l, double& sh, double& k) {
+	int gc = 2 * b - 1 + l;
+	sh = 0.0;
+	if (gc < 0) {
+		gc += bx.g.nc[d];
+		sh = -bx.g.L[d];
+	} else if (gc >= bx.g.nc[d]) {
+		gc -= bx.g.nc[d];
+		sh = bx.g.L[d];
+	}
+	k = (sh - (2 * b + 1) * bx.g.cell_length[d]) + (double) bx.frame_c[d];
+	return gc;
 }
 
-// Stages the 4x4x4 cells around brick `brick` (positions in the local frame; double images in the
-// FP64 mode). Returns false when the region exceeds the staged capacity (nothing staged then; the
-// cell ranges s_gst/s_cnt are set either way). Ends with a CTA barrier.
-template <bool kFP64, bool kHalf = true, bool kWide = true>
-__device__ __forceinline__ bool stage(const Const& p, const Box& bx, int brick, const Smem& S, const double* rx,
-                                      const double* ry, const double* rz, const int32_t* cid, const int32_t* cstart) {
+// Prefix sums (9) of the counts of a brick's own cells (cells beyond the grid count as empty) and their
+// staged cells (8), by one warp; the counts of staged cells 2 l and 2 l + 1 are in lane l's na and nb.
+__device__ __forceinline__ void own_prefix(const Box& bx, int brick, int na, int nb, int* s_own, int* s_ocell) {
+	const int lane = threadIdx.x & 31;
+	int ic = 0;
+	const bool ok = lane < kWarps && own_cell(bx, brick, lane, ic);
+	const int a = __shfl_sync(kFull, na, ic >> 1), b = __shfl_sync(kFull, nb, ic >> 1);
+	const int c = ok ? ((ic & 1) ? b : a) : 0;
+	int own = c;
+	for (int o = 1; o < kWarps; o <<= 1) {
+		const int y = __shfl_up_sync(kFull, own, o);
+		if (lane >= o) own += y;
+	}
+	if (lane < kWarps) {
+		s_own[lane] = own - c;
+		s_ocell[lane] = ic;
+		if (lane == kWarps - 1) s_own[kWarps] = own;
+	}
+}
+
+// Staging of the list kernels: the 4x4x4 cells around brick `brick`, cell by cell (their cells hold
+// about 28 molecules, a warp's width). Returns false when the region exceeds the staged capacity
+// (nothing staged then; the cell ranges S.gst/S.cnt are set either way). s_own and s_ocell: own_prefix.
+// Ends with a CTA barrier.
+template <bool kFP64, bool kWide>
+__device__ __forceinline__ bool stage_cells(const Const& p, const Box& bx, int brick, const Smem& S, const double* rx,
+                                            const double* ry, const double* rz, const int32_t* cid,
+                                            const int32_t* cstart, int* s_own, int* s_ocell) {
+	constexpr Staging kMode = kFP64 ? kStageList64 : kStageList32;
 	const Grid& g = bx.g;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int bc[3] = {brick % bx.nb[0], (brick / bx.nb[0]) % bx.nb[1], brick / (bx.nb[0] * bx.nb[1])};
@@ -293,22 +334,7 @@ __device__ __forceinline__ bool stage(const Const& p, const Box& bx, int brick, 
 	if (tid < 64) {
 		const int l[3] = {tid & 3, (tid >> 2) & 3, tid >> 4};
 		int gc[3];
-		for (int d = 0; d < 3; d++) {
-			int gcd = 2 * bc[d] - 1 + l[d];
-			double sh = 0.0;
-			if (gcd < 0) {
-				gcd += g.nc[d];
-				sh = -g.L[d];
-			} else if (gcd >= g.nc[d]) {
-				gcd -= g.nc[d];
-				sh = g.L[d];
-			}
-			gc[d] = gcd;
-			S.csh[3 * tid + d] = sh;
-			// frame: X = x + K, K = shift - c_brick + C
-			const double cbr = (2 * bc[d] + 1) * g.cell_length[d];
-			S.ck[3 * tid + d] = (sh - cbr) + (double) bx.frame_c[d];
-		}
+		for (int d = 0; d < 3; d++) gc[d] = staged_coord(bx, d, bc[d], l[d], S.csh[3 * tid + d], S.ck[3 * tid + d]);
 		const int gcell = bx.coff + (gc[2] * g.nc[1] + gc[1]) * g.nc[0] + gc[0];
 		const int st = cstart[gcell];
 		S.gst[tid] = st;
@@ -316,17 +342,21 @@ __device__ __forceinline__ bool stage(const Const& p, const Box& bx, int brick, 
 	}
 	__syncthreads();
 	// exclusive scan of the 64 staged-cell counts (warp 0, two per lane)
-	if (warp == 0) {
+	if (warp < 2) {
 		const int a = S.cnt[2 * lane], b = S.cnt[2 * lane + 1];
-		int inc = a + b;
-		for (int o = 1; o < 32; o <<= 1) {
-			const int y = __shfl_up_sync(kFull, inc, o);
-			if (lane >= o) inc += y;
+		if (warp == 0) {
+			int inc = a + b;
+			for (int o = 1; o < 32; o <<= 1) {
+				const int y = __shfl_up_sync(kFull, inc, o);
+				if (lane >= o) inc += y;
+			}
+			const int excl = inc - (a + b);
+			S.cs[2 * lane] = excl;
+			S.cs[2 * lane + 1] = excl + a;
+			if (lane == 31) S.cs[64] = inc;
+		} else {
+			own_prefix(bx, brick, a, b, s_own, s_ocell);
 		}
-		const int excl = inc - (a + b);
-		S.cs[2 * lane] = excl;
-		S.cs[2 * lane + 1] = excl + a;
-		if (lane == 31) S.cs[64] = inc;
 	}
 	__syncthreads();
 	const bool staged = S.cs[64] <= p.s_cap;
@@ -341,11 +371,15 @@ __device__ __forceinline__ bool stage(const Const& p, const Box& bx, int brick, 
 			const double shx = S.csh[3 * c], shy = S.csh[3 * c + 1], shz = S.csh[3 * c + 2];
 			for (int e = lane; e < cnt; e += 32) {
 				const int gi = st + e;
-				stage_at<kFP64, kHalf>(p, bx, S, base + e, rx[gi], ry[gi], rz[gi], cid[gi], kx, ky, kz, shx, shy, shz);
+				stage_at<kMode>(bx, S, base + e, rx[gi], ry[gi], rz[gi], cid[gi], kx, ky, kz, shx, shy, shz);
 			}
 		}
 	}
 	if (staged && kWide) {
+		auto one = [&](int c, int e, double x, double y, double z, int q) {
+			stage_at<kMode>(bx, S, S.cs[c] + e, x, y, z, q, S.ck[3 * c], S.ck[3 * c + 1], S.ck[3 * c + 2], S.csh[3 * c],
+			                S.csh[3 * c + 1], S.csh[3 * c + 2]);
+		};
 		for (int c0 = warp; c0 < 64; c0 += 4 * kWarps) {
 			double x[4], y[4], z[4];
 			int q[4];
@@ -363,10 +397,100 @@ __device__ __forceinline__ bool stage(const Const& p, const Box& bx, int brick, 
 			for (int u = 0; u < 4; u++) {
 				const int c = c0 + u * kWarps;
 				const int cnt = S.cnt[c];
-				if (lane < cnt) stage_one<kFP64, kHalf>(p, bx, S, c, lane, x[u], y[u], z[u], q[u]);
+				if (lane < cnt) one(c, lane, x[u], y[u], z[u], q[u]);
 				for (int e = lane + 32; e < cnt; e += 32) {
 					const int gi = S.gst[c] + e;
-					stage_one<kFP64, kHalf>(p, bx, S, c, e, rx[gi], ry[gi], rz[gi], cid[gi]);
+					one(c, e, rx[gi], ry[gi], rz[gi], cid[gi]);
+				}
+			}
+		}
+	}
+	__syncthreads();
+	return staged;
+}
+
+// Staging of the traversal, whose cells hold few molecules (12 of a warp's 32 lanes at rc = 2.5 in a
+// liquid): the 16 rows of four cells, which are contiguous slots, two rows per warp. Return value and
+// arguments as stage_cells. Its CTA barrier at the end is its only one: every warp loads all cell starts
+// and scans the counts itself (two cells per lane) instead of waiting for one warp's scan.
+__device__ __forceinline__ bool stage_rows(const Const& p, const Box& bx, int brick, const Smem& S, const double* rx,
+                                           const double* ry, const double* rz, const int32_t* cid,
+                                           const int32_t* cstart, int* s_own, int* s_ocell) {
+	const Grid& g = bx.g;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int bc[3] = {brick % bx.nb[0], (brick / bx.nb[0]) % bx.nb[1], brick / (bx.nb[0] * bx.nb[1])};
+	// staged cells k = lx + 4 ly + 16 lz; this lane's: 2 lane and 2 lane + 1
+	double t0, t1;
+	const int gy = staged_coord(bx, 1, bc[1], (lane >> 1) & 3, t0, t1);
+	const int gz = staged_coord(bx, 2, bc[2], lane >> 3, t0, t1);
+	const int row0 = bx.coff + (gz * g.nc[1] + gy) * g.nc[0];
+	const int ca = row0 + staged_coord(bx, 0, bc[0], 2 * (lane & 1), t0, t1);
+	const int cb = row0 + staged_coord(bx, 0, bc[0], 2 * (lane & 1) + 1, t0, t1);
+	const int sa = cstart[ca], ea = cstart[ca + 1], sb = cstart[cb], eb = cstart[cb + 1];
+	const int na = max(0, ea - sa), nb = max(0, eb - sb);
+	int inc = na + nb;
+	for (int o = 1; o < 32; o <<= 1) {
+		const int y = __shfl_up_sync(kFull, inc, o);
+		if (lane >= o) inc += y;
+	}
+	const int slot_a = inc - (na + nb);
+	const int total = __shfl_sync(kFull, inc, 31);
+	const bool staged = total <= p.s_cap;
+	if (warp == 0) {
+		S.cs[2 * lane] = slot_a;
+		S.cs[2 * lane + 1] = slot_a + na;
+		if (lane == 31) S.cs[64] = total;
+		S.gst[2 * lane] = sa;
+		S.gst[2 * lane + 1] = sb;
+		S.cnt[2 * lane] = na;
+		S.cnt[2 * lane + 1] = nb;
+	} else if (warp == 1) {
+		own_prefix(bx, brick, na, nb, s_own, s_ocell);
+	}
+	// lane 4 d + l holds the shift and the frame offset (of the brick's centre) of staged coordinate l of
+	// dimension d
+	double sh_l = 0.0, k_l = 0.0;
+	if (lane < 12) {
+		staged_coord(bx, lane >> 2, bc[lane >> 2], lane & 3, sh_l, k_l);
+		k_l -= (double) bx.frame_c[lane >> 2];
+	}
+	if (staged) {
+		for (int rr = 0; rr < 2; rr++) {
+			// row `row`: its four cells' prefix counts, and the offset from a molecule's place in the row
+			// to its index in the sorted arrays, per cell
+			const int row = 2 * warp + rr;
+			const int slot0 = __shfl_sync(kFull, slot_a, 2 * row);
+			const int p1 = __shfl_sync(kFull, na, 2 * row);
+			const int p2 = p1 + __shfl_sync(kFull, nb, 2 * row);
+			const int p3 = p2 + __shfl_sync(kFull, na, 2 * row + 1);
+			const int len = p3 + __shfl_sync(kFull, nb, 2 * row + 1);
+			const int o0 = __shfl_sync(kFull, sa, 2 * row), o1 = __shfl_sync(kFull, sb, 2 * row) - p1;
+			const int o2 = __shfl_sync(kFull, sa, 2 * row + 1) - p2, o3 = __shfl_sync(kFull, sb, 2 * row + 1) - p3;
+			const double ky = __shfl_sync(kFull, k_l, 4 + (row & 3)), kz = __shfl_sync(kFull, k_l, 8 + (row >> 2));
+			const double shy = __shfl_sync(kFull, sh_l, 4 + (row & 3)), shz = __shfl_sync(kFull, sh_l, 8 + (row >> 2));
+			for (int e0 = 0; e0 < len; e0 += 64) {
+				double x[2], y[2], z[2];
+				int q[2], l[2];
+#pragma unroll
+				for (int u = 0; u < 2; u++) {
+					const int e = e0 + 32 * u + lane;
+					l[u] = (e >= p1 ? 1 : 0) + (e >= p2 ? 1 : 0) + (e >= p3 ? 1 : 0);
+					const int gi = e + (e >= p2 ? (e >= p3 ? o3 : o2) : (e >= p1 ? o1 : o0));
+					x[u] = y[u] = z[u] = 0.0;
+					q[u] = 0;
+					if (e < len) {
+						x[u] = rx[gi];
+						y[u] = ry[gi];
+						z[u] = rz[gi];
+						q[u] = cid[gi];
+					}
+				}
+#pragma unroll
+				for (int u = 0; u < 2; u++) {
+					const double kx = __shfl_sync(kFull, k_l, l[u]), shx = __shfl_sync(kFull, sh_l, l[u]);
+					const int e = e0 + 32 * u + lane;
+					if (e < len)
+						stage_at<kStageTraverse>(bx, S, slot0 + e, x[u], y[u], z[u], q[u], kx, ky, kz, shx, shy, shz);
 				}
 			}
 		}
@@ -397,72 +521,66 @@ static __device__ __noinline__ bool exact_cut(const Smem& S, double rc2, int j, 
 	return dd < rc2;
 }
 
-// One list entry j of molecule i in FP32 with FP64-ready accumulators (branch-free: an invalid
-// entry, v = false, or a pair outside the cutoff contributes zeros; the rare pairs within a few ulp
-// of rc are decided in double from the same hi/lo parts).
-template <bool kSingle, bool kLjIsRc>
-__device__ __forceinline__ void lj32(const Const& p, bool v, const float4& hi_i, const float3& lo_i, int ti, int ns,
-                                     const float4 hj, const Box& bx, const float* pf, float eps24_1, float sig2_1,
-                                     float shift6_1, float& ax, float& ay, float& az, float& au, float& aw, int& anp,
-                                     bool& same, const Smem& S, int j, int gi, const double* rx, const double* ry,
-                                     const double* rz) {
-	const float3 lj = unpack_lo(__float_as_uint(hj.w), bx);
-	const float h0 = hi_i.x - hj.x, h1 = hi_i.y - hj.y, h2 = hi_i.z - hj.z;  // exact
-	const float e0 = h0 + (lo_i.x - lj.x), e1 = h1 + (lo_i.y - lj.y), e2 = h2 + (lo_i.z - lj.z);
-	const float d2f = fmaf(e0, e0, fmaf(e1, e1, e2 * e2));
-	bool in = v && d2f < p.rc2f;
-	const bool amb = v && fabsf(d2f - p.rc2f) <= p.band;
-	if (amb) in = exact_cut(S, p.rc2, j, gi, rx, ry, rz);
-	anp += in ? 1 : 0;
-	same |= in && d2f == 0.f;
-	const bool lj_in = kLjIsRc ? in : (in && d2f < p.rclj2f);
-	float eps24, sig2, shift6;
-	if (kSingle) {
-		eps24 = eps24_1;
-		sig2 = sig2_1;
-		shift6 = shift6_1;
-	} else {
-		const int pk = ti * ns + unpack_cid(__float_as_uint(hj.w));
-		eps24 = pf[pk];
-		sig2 = pf[KK + pk];
-		shift6 = pf[2 * KK + pk];
-	}
-	const float inv = rcp_approx(lj_in ? d2f : 1.0f);
-	const float s2 = sig2 * inv;
-	const float s6 = s2 * s2 * s2;
-	const float s12 = s6 * s6;
-	const float m = s12 - s6;
-	const float fac = lj_in ? eps24 * (s12 + m) * inv : 0.f;
-	ax = fmaf(fac, e0, ax);
-	ay = fmaf(fac, e1, ay);
-	az = fmaf(fac, e2, az);
-	au += lj_in ? fmaf(eps24, m, shift6) : 0.f;
-	aw = fmaf(fac, d2f, aw);
+// 1/x for a positive normal x: the hardware's approximation y (rcp.approx.ftz.f64, about 20 bits) and
+// one step of Chebyshev's third-order iteration, y + y (e + e^2) with e = 1 - x y: e^3 is below 2^-58,
+// so what is left is the last rounding. Three FP64 instructions and no branch; the correctly rounded
+// intrinsic, with its branch for special operands, made the whole FP64 evaluation a fifth slower.
+__device__ __forceinline__ double rcp64(double x) {
+	double y;
+	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+	const double e = fma(-x, y, 1.0);
+	return fma(y, fma(e, e, e), y);
 }
 
-// One list entry j (staged slot) of molecule i at the double image position (xi, yi, zi), in FP64
-// with the reference's operation order.
-template <bool kSingle>
-__device__ __forceinline__ void lj64(const Const& p, double xi, double yi, double zi, int ti, int ns, int j,
-                                     const Smem& S, double& ax, double& ay, double& az, double& au, double& aw,
-                                     int& anp, bool& same) {
-	const double d0 = __dsub_rn(xi, S.img[j]);
-	const double d1 = __dsub_rn(yi, S.img[p.s_cap + j]);
-	const double d2 = __dsub_rn(zi, S.img[2 * p.s_cap + j]);
+// FP64 sums of one molecule's pairs: force, energy and virial before the pair parameters that the
+// single-species form applies once per molecule (sums64_finish).
+struct Sums64 {
+	double x, y, z, u, w;
+	int np, nlj;   // pairs within rc; pairs within rcLJ (where that is another radius)
+};
+
+// One candidate pair in FP64: d = r_i - r_j, branch-free (a pair outside the cutoffs, or v = false,
+// adds zeros). The squared distance and both cutoff tests keep the reference's operations and
+// roundings (no contraction), so the pairs within rc are the reference's; the force law is
+// PotForceLJ's (molecules/potforce.h:41-53), contracted: with s6 = (sig2/r^2)^3, m = s6^2 - s6 and
+// e = s6^2 + m the sums are F += (e/r^2) d, U += m, W += e (the virial term d.f is e, as f = (e/r^2) d):
+// 22 FP64 instructions against 38 and a division in the reference's order. A zero distance (its high
+// word is zero) sets `same` and leaves non-finite sums.
+template <bool kSingle, bool kLjIsRc>
+__device__ __forceinline__ void lj64(double d0, double d1, double d2, bool v, double rc2, double rclj2, double eps24,
+                                     double sig2, double shift6, Sums64& s, bool& same) {
 	const double dd = __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
-	if (!(dd < p.rc2)) return;
-	anp++;
-	if (dd == 0.0) same = true;
-	if (!(dd < p.rclj2)) return;
-	int pk = 0;
-	if (!kSingle) pk = ti * ns + unpack_cid(__float_as_uint(S.hi[j].w));
-	double f0, f1, f2, u, w;
-	lj_pair_fp64(d0, d1, d2, dd, S.pd[pk], S.pd[KK + pk], S.pd[2 * KK + pk], f0, f1, f2, u, w);
-	ax += f0;
-	ay += f1;
-	az += f2;
-	au += u;
-	aw = __dadd_rn(aw, w);
+	const bool in = v && dd < rc2;
+	const bool lj = kLjIsRc ? in : (in && dd < rclj2);
+	s.np += in ? 1 : 0;
+	if (!kLjIsRc) s.nlj += lj ? 1 : 0;
+	same |= in && __double2hiint(dd) == 0;
+	const double inv = lj ? rcp64(dd) : 0.0;
+	const double s2 = sig2 * inv;
+	const double s6 = s2 * s2 * s2;
+	const double m = fma(s6, s6, -s6);
+	double e = fma(s6, s6, m);
+	if (kSingle) {
+		s.u += m;
+	} else {
+		e *= eps24;
+		s.u = fma(eps24, m, s.u) + (lj ? shift6 : 0.0);
+	}
+	const double fac = e * inv;
+	s.x = fma(fac, d0, s.x);
+	s.y = fma(fac, d1, s.y);
+	s.z = fma(fac, d2, s.z);
+	s.w += e;
+}
+
+// The pair parameters of a single-species molecule's sums.
+template <bool kLjIsRc>
+__device__ __forceinline__ void sums64_finish(Sums64& s, double eps24, double shift6) {
+	s.x *= eps24;
+	s.y *= eps24;
+	s.z *= eps24;
+	s.w *= eps24;
+	s.u = fma(eps24, s.u, shift6 * (double) (kLjIsRc ? s.np : s.nlj));
 }
 
 // Neighbour lists of the Verlet-skin mode: entry k of molecule i (sorted slot) is a staged slot of
@@ -488,162 +606,198 @@ struct Lists {
 constexpr int kSparseCap = 128;
 constexpr unsigned short kListOverflow = 0xffff;
 
+// Rows of the traversal's lanes: the 27 cells around a cell are 9 rows of 3 (row r: y offset r % 3 - 1,
+// z offset r / 3 - 1), and the lanes of a molecule share its rows so that their hits are about equal
+// (the middle row holds about 22 % of them, an edge row 12 %, a corner row 7 %). Entry lpm - 1 + sub:
+// the rows of lane `sub` of lpm, one per 4 bits, 15 past the last.
+static __constant__ unsigned long long kRowsOf[15] = {
+    0xff876543210ull,                                                                // 1 lane
+    0xf86204ull, 0xf7531ull,                                                         // 2 lanes
+    0xfff04ull, 0xfff31ull, 0xfff75ull, 0xf862ull,                                   // 4 lanes
+    0xff4ull, 0xff1ull, 0xff3ull, 0xff5ull, 0xff7ull, 0xf80ull, 0xf62ull, 0xffffull  // 8 lanes
+};
+__host__ __device__ constexpr int rows_per_lane(int lpm) { return lpm == 1 ? 9 : lpm == 2 ? 5 : lpm == 4 ? 3 : 2; }
+
+// Hit words a lane collects before it evaluates them.
+constexpr int kHitWords = 24;
+
 // Forces on the molecules of brick `brick` (index within its box) of box `bx`; U, W and the pair
 // count go to partials[slot]. The pair table must already be in shared memory (load_params).
 // Ends with a CTA-wide barrier after which no thread reads the staged data.
-template <bool kFP64, bool kSingle, bool kLjIsRc, int kCap, bool kWide = true>
+//
+// One evaluation, in FP64, serves both precision modes: what the FP32 form would save in the force law
+// it spends on unpacking its split positions, here and in the staging (250,047 molecules at rc = 2.5:
+// 121 us in FP64, 136 with an FP32 evaluation in the same structure).
+//
+// The brick's own molecules, of all its cells in one sequence, are spread over the CTA's lanes, lpm
+// lanes per molecule: the largest of 1, 2, 4, 8 that the CTA's 256 lanes allow, so the warps that
+// work are full whatever the cells hold (at rc = 2.5 a cell of a liquid holds 11-13 molecules: with
+// one warp per cell, 60 % of every warp stood idle). A lane's filter walks its rows of three staged
+// cells in blocks of 16 slots; lanes of other cells read other addresses in the same step. Hits stay
+// a bit mask: one word per block (16 hit bits, the block's first slot above them), and the evaluation
+// takes the bits of its words one by one, so the lanes of a warp wait for each other only at the end
+// of a batch of words, not in every block.
+//
+// Bound by instruction issue (of 250,047 molecules at rc = 2.5: staging 25 %, filter 30 %, evaluation
+// 45 %); three CTAs per SM. Measured, us per traversal, against one warp per cell with per-lane index
+// lists and the reference's operation order: 250,047 molecules at rc = 2.5 121 (328), at rc = 3.0 190
+// (381); a 786,432-molecule two-species slab 530 (1339); 16,384 molecules 24 (34).
+template <bool kSingle, bool kLjIsRc, int kWords>
 __device__ __forceinline__ void pairs(const Const& p, const Box& bx, int brick, int64_t slot, unsigned char* smem,
                                       const double* rx, const double* ry, const double* rz, const int32_t* cid,
                                       const int32_t* cstart, double* fx, double* fy, double* fz, double* partials,
                                       int* status) {
-	const SmemLayout L = layout(p.s_cap, kFP64, kCap);
+	const SmemLayout L = layout(p.s_cap, true, kWords);
 	const Smem S = views(smem, L);
-	float4* s_hi = S.hi;
-	double* s_img = S.img;
-	HalfPair* s_h16 = S.h16;
-	int* s_cs = S.cs;
-	unsigned short* s_list = S.list;
-	int* s_cnt = S.cnt;
-	int* s_gst = S.gst;
-	double* s_pd = S.pd;
-	float* s_pf = S.pf;
-	const Grid& g = bx.g;
+	__shared__ int s_own[kWarps + 1], s_ocell[kWarps];
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int ns = p.ns;
-	const bool staged = stage<kFP64, true, kWide>(p, bx, brick, S, rx, ry, rz, cid, cstart);
-
-	// ---- pairs: warp w owns brick cell (1 + (w&1), 1 + ((w>>1)&1), 1 + (w>>2)) -----------------
+	const bool staged = stage_rows(p, bx, brick, S, rx, ry, rz, cid, cstart, s_own, s_ocell);
+	const int n_own = s_own[kWarps];
 	double U = 0.0, W = 0.0, NP = 0.0;
 	bool same = false;
-	const int il[3] = {1 + (warp & 1), 1 + ((warp >> 1) & 1), 1 + (warp >> 2)};
-	int icell;
-	const bool cell_ok = own_cell(bx, brick, warp, icell);
-	if (cell_ok && !staged) {
+	if (!staged) {
 		// over capacity: gather from global memory
-		const int st = s_gst[icell], cnt = s_cnt[icell];
-		for (int e = lane; e < cnt; e += 32) {
-			PairSums s = gather_pairs<!kFP64>(st + e, rx, ry, rz, cid, cstart, g, s_pd, ns, p.rc2, p.rclj2, bx.coff);
-			fx[st + e] = s.F[0];
-			fy[st + e] = s.F[1];
-			fz[st + e] = s.F[2];
+		for (int t = tid; t < n_own; t += kThreads) {
+			int w = 0;
+			while (w < kWarps - 1 && s_own[w + 1] <= t) w++;
+			const int gi = S.gst[s_ocell[w]] + (t - s_own[w]);
+			PairSums s = gather_pairs<false>(gi, rx, ry, rz, cid, cstart, bx.g, S.pd, ns, p.rc2, p.rclj2, bx.coff);
+			fx[gi] = s.F[0];
+			fy[gi] = s.F[1];
+			fz[gi] = s.F[2];
 			U += s.U;
 			W += s.W;
 			NP += s.np;
 			same |= s.same;
 		}
-	} else if (cell_ok) {
-		const int i0 = s_cs[icell], ni = s_cs[icell + 1] - i0;
-		unsigned short* mylist = s_list + warp * kCap * 32 + lane;
-		for (int b0 = 0; b0 < ni; b0 += 32) {
-			const bool act = b0 + lane < ni;
-			const int slot_i = i0 + (act ? b0 + lane : 0);
-			const float4 hi_i = s_hi[slot_i];
-			const float3 lo_i = unpack_lo(__float_as_uint(hi_i.w), bx);
-			double xi = 0, yi = 0, zi = 0;
-			if (kFP64) {
-				xi = s_img[slot_i];
-				yi = s_img[p.s_cap + slot_i];
-				zi = s_img[2 * p.s_cap + slot_i];
-			}
-			const int ti = unpack_cid(__float_as_uint(hi_i.w));
-			const int gi = s_gst[icell] + (slot_i - i0);
-			int cnt = 0;
-			double Fx = 0.0, Fy = 0.0, Fz = 0.0;
-			const float eps24_1 = s_pf[0], sig2_1 = s_pf[KK], shift6_1 = s_pf[2 * KK];
+	} else {
+		const int lpm = n_own > kThreads / 2 ? 1 : n_own > kThreads / 4 ? 2 : n_own > kThreads / 8 ? 4 : 8;
+		const int lg = lpm == 1 ? 0 : lpm == 2 ? 1 : lpm == 4 ? 2 : 3;
+		const int nrows = rows_per_lane(lpm);
+		const int sub = lane & (lpm - 1);
+		const unsigned long long rows = kRowsOf[lpm - 1 + sub];
+		unsigned* const words = S.words + tid;
+		const double eps24_d = S.pd[0], sig2_d = S.pd[KK], shift6_d = S.pd[2 * KK];
+		for (int base0 = 0; base0 < n_own; base0 += kThreads >> lg) {
+			const int t0 = base0 + ((warp * 32) >> lg);
+			if (t0 >= n_own) break;   // this warp has no molecule (in this round or a later one)
+			const int t = t0 + (lane >> lg);
+			const bool act = t < n_own;
+			int w = 0;
+			if (act)
+				while (w < kWarps - 1 && s_own[w + 1] <= t) w++;
+			const int il0 = 1 + (w & 1), il1 = 1 + ((w >> 1) & 1), il2 = 1 + (w >> 2);
+			const int oc = s_ocell[w];
+			const int slot_i = S.cs[oc] + (act ? t - s_own[w] : 0);
+			const int gi = S.gst[oc] + (act ? t - s_own[w] : 0);
+			const double xi = S.img[3 * slot_i], yi = S.img[3 * slot_i + 1], zi = S.img[3 * slot_i + 2];
+			const int ti = kSingle ? 0 : S.comp[slot_i];
+			Sums64 s64{0.0, 0.0, 0.0, 0.0, 0.0, 0, 0};
+			int cnt = 0, hits = 0;   // words and hits collected
 
-			// one list entry in FP32 (branch-free: lanes past their list length or outside the
-			// cutoff contribute zeros; the rare pairs within a few ulp of rc are decided in double)
-			auto pair_fp32 = [&](int tt, float& ax, float& ay, float& az, float& au, float& aw, int& anp) {
-				const bool v = tt < cnt;
-				const int j = v ? (int) mylist[tt * 32] : slot_i;
-				lj32<kSingle, kLjIsRc>(p, v, hi_i, lo_i, ti, ns, s_hi[j], bx, s_pf, eps24_1, sig2_1, shift6_1, ax, ay, az,
-				                       au, aw, anp, same, S, j, gi, rx, ry, rz);
-			};
-			auto pair_fp64 = [&](int tt, double& ax, double& ay, double& az, double& au, double& aw, int& anp) {
-				if (tt >= cnt) return;
-				lj64<kSingle>(p, xi, yi, zi, ti, ns, mylist[tt * 32], S, ax, ay, az, au, aw, anp, same);
-			};
-			auto flush = [&]() {
-				const int mx = __reduce_max_sync(kFull, cnt);
-				int anp = 0;
-				if (kFP64) {
-					double ax[2] = {0, 0}, ay[2] = {0, 0}, az[2] = {0, 0}, au[2] = {0, 0}, aw[2] = {0, 0};
-					for (int t = 0; t < mx; t += 2) {
-#pragma unroll
-						for (int u = 0; u < 2; u++) pair_fp64(t + u, ax[u], ay[u], az[u], au[u], aw[u], anp);
+			// evaluates the collected words
+			auto evaluate = [&]() {
+				const int mx = __reduce_max_sync(kFull, hits);
+				const unsigned* next = words;
+				unsigned wd = 0u, nx = *next;   // this word's bits left; the next word
+#pragma unroll 2
+				for (int h = 0; h < mx; h++) {
+					bool v = h < hits;
+					if (v && (wd & 0xffffu) == 0u) {
+						wd = nx;
+						next += kThreads;   // (the word past the last one is never used)
 					}
-					Fx += ax[0] + ax[1];
-					Fy += ay[0] + ay[1];
-					Fz += az[0] + az[1];
-					U += au[0] + au[1];
-					W = __dadd_rn(W, __dadd_rn(aw[0], aw[1]));
-				} else {
-					// four independent accumulator sets: four pair chains in flight per lane
-					float ax[4] = {0.f, 0.f, 0.f, 0.f}, ay[4] = {0.f, 0.f, 0.f, 0.f}, az[4] = {0.f, 0.f, 0.f, 0.f};
-					float au[4] = {0.f, 0.f, 0.f, 0.f}, aw[4] = {0.f, 0.f, 0.f, 0.f};
-					for (int t = 0; t < mx; t += 4) {
-#pragma unroll
-						for (int u = 0; u < 4; u++) pair_fp32(t + u, ax[u], ay[u], az[u], au[u], aw[u], anp);
+					nx = *next;
+					const int bit = __ffs(wd) - 1;
+					const int j = v ? (int) (wd >> 16) + ((bit & 7) << 1) + (bit >> 3) : slot_i;
+					wd &= wd - 1u;
+					v = v && j != slot_i;
+					double e24 = 0.0, sg2 = sig2_d, sh6 = 0.0;
+					if (!kSingle) {
+						const int pk = ti * ns + S.comp[j];
+						e24 = S.pd[pk];
+						sg2 = S.pd[KK + pk];
+						sh6 = S.pd[2 * KK + pk];
 					}
-					Fx += ((double) ax[0] + (double) ax[1]) + ((double) ax[2] + (double) ax[3]);
-					Fy += ((double) ay[0] + (double) ay[1]) + ((double) ay[2] + (double) ay[3]);
-					Fz += ((double) az[0] + (double) az[1]) + ((double) az[2] + (double) az[3]);
-					U += ((double) au[0] + (double) au[1]) + ((double) au[2] + (double) au[3]);
-					W += ((double) aw[0] + (double) aw[1]) + ((double) aw[2] + (double) aw[3]);
+					lj64<kSingle, kLjIsRc>(__dsub_rn(xi, S.img[3 * j]), __dsub_rn(yi, S.img[3 * j + 1]),
+					                       __dsub_rn(zi, S.img[3 * j + 2]), v, p.rc2, p.rclj2, e24, sg2, sh6, s64, same);
 				}
-				NP += (double) anp;
-				cnt = 0;
+				cnt = hits = 0;
 			};
 
-			// filter: the 9 rows of 3 staged cells around the i cell; every pair of consecutive
-			// staged molecules is broadcast to all lanes and tested with packed half arithmetic
-			const __half2 xi2 = __float2half2_rn(act ? hi_i.x - bx.frame_c[0] : 60000.f);
-			const __half2 yi2 = __float2half2_rn(hi_i.y - bx.frame_c[1]);
-			const __half2 zi2 = __float2half2_rn(hi_i.z - bx.frame_c[2]);
+			// filter: packed half-precision test against rc^2 plus a margin covering its rounding
+			const __half* hh = S.h + 8 * (slot_i >> 1) + (slot_i & 1);
+			const __half2 xi2 = __half2half2(hh[0]), yi2 = __half2half2(hh[2]), zi2 = __half2half2(hh[4]);
 			const __half2 rc2h = __float2half2_rn(bx.rc2_h);
-			// one 32-slot block [base, base + 32): per-lane hit mask, bit b = slot base + b
-			auto block_mask = [&](int mb) -> unsigned {
-				unsigned mask = 0u;
+			int q = 0, base = 0, left = 0;   // next row; this lane's next slot and what is left of its row
+			unsigned first = 0u;             // the slot before an odd first slot belongs to another row
+			for (bool more = true; more;) {
+				// fill: blocks until a lane's words are full or the rows are done
+				for (;;) {
+					const int nblk = (__reduce_max_sync(kFull, left) + 15) >> 4;
+					if (nblk <= 0) {
+						if (q == nrows) {
+							more = false;
+							break;
+						}
+						const int r = (int) (rows >> (4 * q)) & 15;
+						q++;
+						left = 0;
+						if (act && r < 9) {
+							const int k0 = (il0 - 1) + 4 * (il1 + (r % 3) - 1) + 16 * (il2 + (r / 3) - 1);
+							const int a = S.cs[k0];
+							base = a & ~1;
+							left = S.cs[k0 + 3] - base;
+							first = (unsigned) (a & 1);
+						}
+						continue;
+					}
+					const int room = kWords - __reduce_max_sync(kFull, cnt);
+					if (room == 0) break;
+					const HalfPair* H = S.h16 + (base >> 1);
+					for (int ib = min(nblk, room); ib > 0; ib--) {
+						// bit k: slot base + 2k, bit 16 + k: slot base + 2k + 1
+						unsigned m = 0u;
+						if (left > 0) {
 #pragma unroll
-				for (int k = 0; k < 16; k++) {
-					const HalfPair H = s_h16[mb + k];
-					const __half2 dx = __hsub2(xi2, H.x), dy = __hsub2(yi2, H.y), dz = __hsub2(zi2, H.z);
-					const __half2 d2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
-					const unsigned hm = __hlt2_mask(d2, rc2h);
-					mask |= ((hm & 1u) | ((hm >> 15) & 2u)) << (2 * k);
-				}
-				return mask;
-			};
-			for (int r = 0; r < 9; r++) {
-				const int ky = il[1] + (r % 3) - 1, kz = il[2] + (r / 3) - 1;
-				const int k0 = (il[0] - 1) + 4 * ky + 16 * kz;
-				const int a = s_cs[k0], b = s_cs[k0 + 3];
-				for (int base = a & ~1; base < b; base += 32) {
-					unsigned mask = block_mask(base >> 1);
-					// keep slots in [a, b) and drop i itself
-					const int lo = a - base, hi = b - base;
-					unsigned valid = hi >= 32 ? 0xffffffffu : ((1u << hi) - 1u);
-					if (lo > 0) valid &= ~((1u << lo) - 1u);
-					const int self = slot_i - base;
-					if (self >= 0 && self < 32) valid &= ~(1u << self);
-					mask &= valid;
-					if (!act) mask = 0u;
-					if (__reduce_max_sync(kFull, cnt + __popc(mask)) > kCap) flush();
-					while (mask) {
-						const int bit = __ffs(mask) - 1;
-						mask &= mask - 1u;
-						mylist[cnt * 32] = (unsigned short) (base + bit);
-						cnt++;
+							for (int k = 0; k < 8; k++) {
+								const HalfPair P = H[k];
+								const __half2 dx = __hsub2(xi2, P.x), dy = __hsub2(yi2, P.y), dz = __hsub2(zi2, P.z);
+								const __half2 d2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
+								m |= __hlt2_mask(d2, rc2h) & ((1u << k) | (1u << (16 + k)));
+							}
+							// keep slots in [a, b)
+							if (left < 16) m &= ((1u << ((left + 1) >> 1)) - 1u) | (((1u << (left >> 1)) - 1u) << 16);
+							m &= ~first;
+						}
+						first = 0u;
+						// even slots' bits in byte 0, odd slots' in byte 1, the block's first slot above
+						words[cnt * kThreads] = __byte_perm(m, (unsigned) base, 0x5420);
+						cnt += m != 0u ? 1 : 0;
+						hits += __popc(m);
+						base += 16;
+						left -= 16;
+						H += 8;
 					}
 				}
+				evaluate();
 			}
-			flush();
-			if (act) {
-				fx[gi] = Fx;
-				fy[gi] = Fy;
-				fz[gi] = Fz;
-				if (!(Fx == Fx && Fy == Fy && Fz == Fz) || isinf(Fx) || isinf(Fy) || isinf(Fz))
-					atomicOr(status, kStatusNonFinite);
+			if (kSingle) sums64_finish<kLjIsRc>(s64, eps24_d, shift6_d);
+			U += s64.u;
+			W += s64.w;
+			NP += (double) s64.np;
+			// the molecule's force: its lanes' sums in a fixed order
+			for (int o = 1; o < lpm; o <<= 1) {
+				s64.x += __shfl_xor_sync(kFull, s64.x, o);
+				s64.y += __shfl_xor_sync(kFull, s64.y, o);
+				s64.z += __shfl_xor_sync(kFull, s64.z, o);
+			}
+			if (act && sub == 0) {
+				fx[gi] = s64.x;
+				fy[gi] = s64.y;
+				fz[gi] = s64.z;
+				if (!(isfinite(s64.x) && isfinite(s64.y) && isfinite(s64.z))) atomicOr(status, kStatusNonFinite);
 			}
 		}
 	}
@@ -986,9 +1140,9 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 	const float3 lo_i = unpack_lo(__float_as_uint(hi_i.w), bx);
 	double xi = 0, yi = 0, zi = 0;
 	if (kFP64) {
-		xi = S.img[slot_i];
-		yi = S.img[p.s_cap + slot_i];
-		zi = S.img[2 * p.s_cap + slot_i];
+		xi = S.img[3 * slot_i];
+		yi = S.img[3 * slot_i + 1];
+		zi = S.img[3 * slot_i + 2];
 	}
 	const int ti = unpack_cid(__float_as_uint(hi_i.w));
 	const int gi = act ? S.gst[s_ocell[w]] + (t - s_own[w]) : S.gst[s_ocell[0]];
@@ -1033,7 +1187,7 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 	};
 	uint4 nxt = sub < nb8 ? my8[(int64_t) sub * lists.n] : make_uint4(0u, 0u, 0u, 0u);
 	if (kFP64) {
-		double ax[2] = {0, 0}, ay[2] = {0, 0}, az[2] = {0, 0}, au[2] = {0, 0}, aw[2] = {0, 0};
+		Sums64 s64{0.0, 0.0, 0.0, 0.0, 0.0, 0, 0};
 		for (int k = 0; k < nk; k++) {
 			const int b = sub + k * lpm;
 			const uint4 cur = nxt;
@@ -1045,8 +1199,16 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 				const unsigned raw = (e[u >> 1] >> (16 * (u & 1))) & 0xffffu;
 				const int j = min((int) raw, p.s_cap - 1);
 				// (a pruned list may hold sentinel slots before its end)
-				if (kk < cnt && raw < (unsigned) p.s_cap) lj64<kSingle>(p, xi, yi, zi, ti, ns, j, S, ax[u & 1], ay[u & 1], az[u & 1], au[u & 1],
-				                            aw[u & 1], anp, same);
+				const bool v = kk < cnt && raw < (unsigned) p.s_cap;
+				double e24 = 0.0, sg2 = S.pd[KK], sh6 = 0.0;
+				if (!kSingle) {
+					const int pk = ti * ns + unpack_cid(__float_as_uint(S.hi[j].w));
+					e24 = S.pd[pk];
+					sg2 = S.pd[KK + pk];
+					sh6 = S.pd[2 * KK + pk];
+				}
+				lj64<kSingle, kLjIsRc>(__dsub_rn(xi, S.img[3 * j]), __dsub_rn(yi, S.img[3 * j + 1]),
+				              __dsub_rn(zi, S.img[3 * j + 2]), v, p.rc2, p.rclj2, e24, sg2, sh6, s64, same);
 				if (kPrune) {
 					// the prune test on the staged hi parts (rp2f covers the lo parts)
 					const float4 hj = S.hi[j];
@@ -1056,11 +1218,13 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 			}
 			if (kPrune && kept - done >= 8) flush();
 		}
-		Fx += ax[0] + ax[1];
-		Fy += ay[0] + ay[1];
-		Fz += az[0] + az[1];
-		U += au[0] + au[1];
-		W = __dadd_rn(W, __dadd_rn(aw[0], aw[1]));
+		if (kSingle) sums64_finish<kLjIsRc>(s64, S.pd[0], S.pd[2 * KK]);
+		Fx = s64.x;
+		Fy = s64.y;
+		Fz = s64.z;
+		U += s64.u;
+		W += s64.w;
+		anp = s64.np;
 	} else {
 		// FP32, branch-free. Per coordinate e = fma(m_i - m_j, step, hi_i - hi_j) with m = 2^23 +
 		// the 9-bit lo field (exact integer difference, one rounding). Single-species runs sum
@@ -1238,27 +1402,15 @@ __device__ __forceinline__ void list_pairs(const Const& p, const Box& bx, int br
                                            const int32_t* cid, const int32_t* cstart, double* fx, double* fy,
                                            double* fz, double* partials, int* status, const Lists lists,
                                            const Kick& kick, const PruneOut& po = PruneOut{}) {
-	const SmemLayout L = layout(p.s_cap, kFP64, 0, false);
+	const SmemLayout L = layout(p.s_cap, kFP64);
 	const Smem S = views(smem, L);
 	const int tid = threadIdx.x, warp = tid >> 5;
 	const int ns = p.ns;
-	const bool staged = stage<kFP64, false, kWide>(p, bx, brick, S, rx, ry, rz, cid, cstart);
-	__shared__ int s_own[9], s_ocell[8];
-	if (tid == 0) {
-		// sentinel slot: far from every molecule (entries past a list's end point to it)
-		S.hi[p.s_cap] = make_float4(1e15f, 1e15f, 1e15f, __uint_as_float((256u << 18) | (256u << 9) | 256u));
-		int acc = 0;
-		for (int w = 0; w < 8; w++) {
-			int ic;
-			const bool ok = own_cell(bx, brick, w, ic);
-			s_own[w] = acc;
-			s_ocell[w] = ic;
-			acc += ok ? S.cnt[ic] : 0;
-		}
-		s_own[8] = acc;
-	}
-	__syncthreads();
-	const int n_own = s_own[8];
+	__shared__ int s_own[kWarps + 1], s_ocell[kWarps];
+	// sentinel slot: far from every molecule (entries past a list's end point to it)
+	if (tid == 0) S.hi[p.s_cap] = make_float4(1e15f, 1e15f, 1e15f, __uint_as_float((256u << 18) | (256u << 9) | 256u));
+	const bool staged = stage_cells<kFP64, kWide>(p, bx, brick, S, rx, ry, rz, cid, cstart, s_own, s_ocell);
+	const int n_own = s_own[kWarps];
 	double U = 0.0, W = 0.0, NP = 0.0, MV = 0.0;
 	bool same = false;
 	if (!staged) {
@@ -1295,11 +1447,11 @@ __device__ __forceinline__ void list_pairs(const Const& p, const Box& bx, int br
 }
 
 // A sparse brick (see kSparseCap) by one warp, in its own shared-memory area laid out as
-// layout(kSparseCap, kFP64, 0, false) plus 17 ints (own-cell prefix and cells): staging of the 4x4x4
+// layout(kSparseCap, kFP64) plus 17 ints (own-cell prefix and cells): staging of the 4x4x4
 // region flattened over its molecules (cell found by bisection of the staged-cell starts), then
 // list_chunk; U, W, pair count to partials[brick]. Warp-level synchronisation only.
 __host__ __device__ inline size_t sparse_warp_bytes(bool fp64) {
-	return align16(layout(kSparseCap, fp64, 0, false).total + sizeof(int) * 17);
+	return align16(layout(kSparseCap, fp64).total + sizeof(int) * 17);
 }
 
 template <bool kFP64, bool kSingle, bool kLjIsRc>
@@ -1308,7 +1460,7 @@ __device__ __forceinline__ void list_pairs_warp(const Const& p, const Box& bx, i
                                                 const int32_t* cid, const int32_t* cstart, double* fx, double* fy,
                                                 double* fz, double* partials, int* status, const Lists& lists,
                                                 const Kick& kick) {
-	const SmemLayout L = layout(kSparseCap, kFP64, 0, false);
+	const SmemLayout L = layout(kSparseCap, kFP64);
 	const Smem S = views(ws, L);
 	int* own = reinterpret_cast<int*>(ws + L.total);
 	const int lane = threadIdx.x & 31;
@@ -1317,21 +1469,7 @@ __device__ __forceinline__ void list_pairs_warp(const Const& p, const Box& bx, i
 	for (int c = lane; c < 64; c += 32) {
 		const int l[3] = {c & 3, (c >> 2) & 3, c >> 4};
 		int gc[3];
-		for (int d = 0; d < 3; d++) {
-			int gcd = 2 * bc[d] - 1 + l[d];
-			double sh = 0.0;
-			if (gcd < 0) {
-				gcd += g.nc[d];
-				sh = -g.L[d];
-			} else if (gcd >= g.nc[d]) {
-				gcd -= g.nc[d];
-				sh = g.L[d];
-			}
-			gc[d] = gcd;
-			S.csh[3 * c + d] = sh;
-			const double cbr = (2 * bc[d] + 1) * g.cell_length[d];
-			S.ck[3 * c + d] = (sh - cbr) + (double) bx.frame_c[d];
-		}
+		for (int d = 0; d < 3; d++) gc[d] = staged_coord(bx, d, bc[d], l[d], S.csh[3 * c + d], S.ck[3 * c + d]);
 		const int gcell = bx.coff + (gc[2] * g.nc[1] + gc[1]) * g.nc[0] + gc[0];
 		const int st = cstart[gcell];
 		S.gst[c] = st;
@@ -1364,18 +1502,9 @@ __device__ __forceinline__ void list_pairs_warp(const Const& p, const Box& bx, i
 					hi = mid - 1;
 			}
 			const int gi = S.gst[lo] + (t - S.cs[lo]);
-			const double x = rx[gi], y = ry[gi], z = rz[gi];
-			const double Xd = __dadd_rn(x, S.ck[3 * lo]), Yd = __dadd_rn(y, S.ck[3 * lo + 1]);
-			const double Zd = __dadd_rn(z, S.ck[3 * lo + 2]);
-			const float X = __double2float_rn(Xd), Y = __double2float_rn(Yd), Z = __double2float_rn(Zd);
-			const unsigned w = pack_lo(__double2float_rn(Xd - (double) X), __double2float_rn(Yd - (double) Y),
-			                           __double2float_rn(Zd - (double) Z), cid[gi], bx);
-			S.hi[t] = make_float4(X, Y, Z, __uint_as_float(w));
-			if (kFP64) {
-				S.img[t] = __dadd_rn(x, S.csh[3 * lo]);
-				S.img[kSparseCap + t] = __dadd_rn(y, S.csh[3 * lo + 1]);
-				S.img[2 * kSparseCap + t] = __dadd_rn(z, S.csh[3 * lo + 2]);
-			}
+			stage_at<kFP64 ? kStageList64 : kStageList32>(bx, S, t, rx[gi], ry[gi], rz[gi], cid[gi], S.ck[3 * lo],
+			                                              S.ck[3 * lo + 1], S.ck[3 * lo + 2], S.csh[3 * lo],
+			                                              S.csh[3 * lo + 1], S.csh[3 * lo + 2]);
 		}
 	}
 	if (lane == 0) {

@@ -72,7 +72,7 @@ constexpr NaLayout na_layout() {
 	L.scalars = o;
 	o += na_align(sizeof(double) * 64);
 	L.status = o;
-	o += na_align(sizeof(int));
+	o += na_align(sizeof(int) + 4 * sizeof(unsigned));   // the status word, then the reductions' tickets
 	L.params = o;
 	o += na_align(sizeof(PairParams));
 	L.total = o;
@@ -274,12 +274,13 @@ extern "C" int mdgpu_forces_noalloc(int device, void* stream, int64_t n, const d
 	c.partial_cap = kPartialBlocks;
 	c.scalars = reinterpret_cast<double*>(base + L.scalars);
 	c.status = reinterpret_cast<int*>(base + L.status);
+	c.tickets = reinterpret_cast<unsigned*>(c.status + 1);
 	c.d_pp = reinterpret_cast<PairParams*>(base + L.params);
 	c.pair_kernel = 0;
 
-	// the shared array keeps the previous call's contents: clear the status word (the binning
+	// the shared array keeps the previous call's contents: clear the status word and tickets (the binning
 	// clears the cell counts itself) and upload this call's parameter table
-	e = cudaMemsetAsync(c.status, 0, sizeof(int), c.stream);
+	e = cudaMemsetAsync(c.status, 0, sizeof(int) + 4 * sizeof(unsigned), c.stream);
 	if (e == cudaSuccess) e = cudaMemcpyAsync(c.d_pp, &hp, sizeof(PairParams), cudaMemcpyHostToDevice, c.stream);
 	if (e == cudaSuccess) {
 		k_na_load<<<(unsigned) ((n + 255) / 256), 256, 0, c.stream>>>(n, d_r, d_cid, ncomp, c.p, c.status);

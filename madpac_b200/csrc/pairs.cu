@@ -70,8 +70,7 @@ __global__ void __launch_bounds__(kReduceBlock) k_pairs_gather(int64_t n, const 
 __global__ void k_reduce_partials(int64_t nblocks, const double* __restrict__ partials, double* out, int nval) {
 	__shared__ double sh[4][1024 / 32];
 	double acc[4] = {0, 0, 0, 0};
-	for (int64_t b = threadIdx.x; b < nblocks; b += blockDim.x)
-		for (int k = 0; k < nval; k++) acc[k] += partials[b * 4 + k];
+	add_partials(partials, threadIdx.x, blockDim.x, nblocks, acc);
 	int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	for (int k = 0; k < nval; k++) {
 		double v = warp_sum(acc[k]);

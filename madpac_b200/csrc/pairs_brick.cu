@@ -21,21 +21,25 @@
 namespace mdgpu {
 namespace {
 
-constexpr int kListCap = 64;
+// Resident CTAs per SM of the traversal (registers and the usual shared memory are sized for it). Two,
+// with 128 registers, took 168 us against 144 for 250,047 molecules at rc = 2.5 (and 220 against 235 at
+// rc = 3.0), four, with 64, 213.
+constexpr int kTraverseMinBlocks = 3;
 
-template <bool kFP64, bool kSingle, bool kLjIsRc>
-__global__ void __launch_bounds__(brick::kThreads, 2)
+template <bool kSingle, bool kLjIsRc>
+__global__ void __launch_bounds__(brick::kThreads, kTraverseMinBlocks)
     k_pairs_brick(brick::Const p, brick::Box bx, const double* __restrict__ rx, const double* __restrict__ ry,
                   const double* __restrict__ rz, const int32_t* __restrict__ cid,
                   const int32_t* __restrict__ cstart, const PairParams* __restrict__ pp,
                   double* __restrict__ fx, double* __restrict__ fy, double* __restrict__ fz,
                   double* __restrict__ partials, int* __restrict__ status, const int* __restrict__ gate,
-                  brick::Lists lists) {
+                  brick::Lists lists, unsigned* ticket, double* scalars) {
 	extern __shared__ __align__(16) unsigned char smem[];
-	brick::load_params(smem, brick::layout(p.s_cap, kFP64, kListCap), pp, p.ns);
-	__syncthreads();
-	brick::pairs<kFP64, kSingle, kLjIsRc, kListCap>(p, bx, blockIdx.x, blockIdx.x, smem, rx, ry, rz, cid, cstart, fx,
-	                                                fy, fz, partials, status);
+	brick::load_params(smem, brick::layout(p.s_cap, true, brick::kHitWords), pp, p.ns);
+	brick::pairs<kSingle, kLjIsRc, brick::kHitWords>(p, bx, blockIdx.x, blockIdx.x, smem, rx, ry, rz, cid, cstart, fx,
+	                                                 fy, fz, partials, status);
+	// U6 sum, virial sum and pair count over every brick, by the last CTA (ticket null: by a later launch)
+	if (ticket) last_block_sum(ticket, partials, gridDim.x, 3, scalars);
 }
 
 // Verlet-skin build step (runs only when *gate is this step's id): the lists, no forces.
@@ -89,7 +93,7 @@ __global__ void __launch_bounds__(brick::kThreads, kFP64 ? 2 : kListMinBlocks)
 	}
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ int s_item;
-	brick::load_params(smem, brick::layout(p.s_cap, kFP64, 0, false), pp, p.ns);
+	brick::load_params(smem, brick::layout(p.s_cap, kFP64), pp, p.ns);
 	if (threadIdx.x == 0) brick::drift_slot() = 0u;   // read after the barriers below
 	if (lists.kind == nullptr) {
 		// every brick, one CTA each
@@ -148,7 +152,7 @@ __global__ void __launch_bounds__(brick::kThreads, 2)
 	extern __shared__ __align__(16) unsigned char smem[];
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	unsigned char* ws = smem + warp * brick::sparse_warp_bytes(kFP64);
-	const brick::SmemLayout L = brick::layout(brick::kSparseCap, kFP64, 0, false);
+	const brick::SmemLayout L = brick::layout(brick::kSparseCap, kFP64);
 	double* pd = reinterpret_cast<double*>(ws + L.params);
 	float* pf = reinterpret_cast<float*>(pd + 3 * brick::KK);
 	for (int k = lane; k < p.ns * p.ns; k += 32) {
@@ -212,22 +216,34 @@ struct Plan {
 
 // kind 0: plain traversal, 2: list evaluation of the skin mode (two CTAs per SM).
 Plan plan(Context* c, const Grid& g, double filter_radius, int kind) {
-	const bool fp64 = c->precision == MDGPU_FP64;
+	const bool fp64 = kind == 0 || c->precision == MDGPU_FP64;   // the traversal evaluates both modes in FP64
 	Plan P;
 	brick::init_box(P.bx, g, filter_radius, 0, kind == 0 ? 0.0 : 0.5 * c->skin);
 	const int max_optin = device_max_optin(c->device);
 	size_t budget = 110 * 1024;
+	if (kind == 0) {
+		// three CTAs per SM when a region of 64 cells fits their share with room for its fluctuations
+		const size_t small = (224 / kTraverseMinBlocks - 2) * 1024;
+		const double rho = c->rho_typ > 0.0 ? c->rho_typ : (double) c->n / (g.L[0] * g.L[1] * g.L[2]);
+		const double region = 64.0 * rho * g.cell_length[0] * g.cell_length[1] * g.cell_length[2];
+		if (1.3 * region + 64.0 <= brick::capacity_for(small, fp64, brick::kHitWords)) budget = small;
+	}
 	if (kind == 2 && !fp64) budget = std::min(budget, (size_t) (224 / kListMinBlocks - 2) * 1024);
 	if (kind == 2 && pruning(c)) budget -= brick::kPruneRingBytes;   // the prune variant's ring
 	if (budget > (size_t) max_optin) budget = (size_t) max_optin;
-	const int lcap = kind == 2 ? 0 : kListCap;
-	const bool half = kind != 2;
-	const int s_cap = brick::capacity_for(budget, fp64, lcap, half);
+	const int words = kind == 2 ? 0 : brick::kHitWords;
+	const int s_cap = brick::capacity_for(budget, fp64, words);
 	P.p = brick::make_const(c->sp.n, s_cap, c->rc, c->rc_lj);
-	P.bytes = brick::layout(s_cap, fp64, lcap, half).total;
+	P.bytes = brick::layout(s_cap, fp64, words).total;
 	P.nbricks = P.bx.nb[0] * P.bx.nb[1] * P.bx.nb[2];
 	return P;
 }
+
+// Whether the traversal's last CTA sums the bricks' partials. It costs every CTA a fence and an atomic
+// before it ends, which is cheaper than another launch up to about one resident round of CTAs (16,384
+// molecules: 1 against 3 us), but not where many short CTAs follow one another (24,400 bricks of a slab:
+// 47 against 8 us).
+bool fold_in_traversal(const Context* c, const Plan& P) { return P.nbricks <= kTraverseMinBlocks * c->num_sms; }
 
 template <typename K, typename... Extra>
 cudaError_t go(Context* c, const Plan& P, K kern, const int* gate, const brick::Lists& lists, Extra... extra) {
@@ -252,6 +268,10 @@ cudaError_t dispatch(Context* c, const Plan& P, const int* gate, const brick::Li
 	if (kKind == 2) {
 		unsigned* t = c->tickets;
 		double* out = c->scalars;
+		if (fp64 && ljrc)
+			return single ? go(c, P, k_pairs_list<true, true, true, kPr>, gate, lists, t, out, kick, record, po, half_prune)
+			              : go(c, P, k_pairs_list<true, false, true, kPr>, gate, lists, t, out, kick, record, po,
+			                   half_prune);
 		if (fp64)
 			return single ? go(c, P, k_pairs_list<true, true, false, kPr>, gate, lists, t, out, kick, record, po, half_prune)
 			              : go(c, P, k_pairs_list<true, false, false, kPr>, gate, lists, t, out, kick, record, po,
@@ -264,12 +284,11 @@ cudaError_t dispatch(Context* c, const Plan& P, const int* gate, const brick::Li
 		              : go(c, P, k_pairs_list<false, false, false, kPr>, gate, lists, t, out, kick, record, po,
 		                   half_prune);
 	}
-	if (fp64) return single ? go(c, P, k_pairs_brick<true, true, false>, gate, lists)
-	                        : go(c, P, k_pairs_brick<true, false, false>, gate, lists);
-	if (ljrc) return single ? go(c, P, k_pairs_brick<false, true, true>, gate, lists)
-	                        : go(c, P, k_pairs_brick<false, false, true>, gate, lists);
-	return single ? go(c, P, k_pairs_brick<false, true, false>, gate, lists)
-	              : go(c, P, k_pairs_brick<false, false, false>, gate, lists);
+	unsigned* t = fold_in_traversal(c, P) ? c->tickets + 2 : nullptr;
+	if (ljrc) return single ? go(c, P, k_pairs_brick<true, true>, gate, lists, t, c->scalars)
+	                        : go(c, P, k_pairs_brick<false, true>, gate, lists, t, c->scalars);
+	return single ? go(c, P, k_pairs_brick<true, false>, gate, lists, t, c->scalars)
+	              : go(c, P, k_pairs_brick<false, false>, gate, lists, t, c->scalars);
 }
 
 brick::Lists lists_of(Context* c) {
@@ -297,7 +316,7 @@ cudaError_t launch_pairs_brick(Context* c) {
 	cudaError_t e = dispatch<0>(c, P, nullptr, brick::Lists{});
 	if (e == cudaSuccess) e = cudaGetLastError();
 	prof_end(c, 1, 1);
-	if (e != cudaSuccess) return e;
+	if (e != cudaSuccess || fold_in_traversal(c, P)) return e;
 	return launch_reduce(c, P.nbricks, c->scalars, 3);
 }
 
@@ -376,7 +395,9 @@ cudaError_t launch_pairs_skin(Context* c, int kick_mode, double dt, double* reco
 	if (e == cudaSuccess && sparse) {
 		const bool fp64 = c->precision == MDGPU_FP64;
 		const bool single = c->sp.n == 1, ljrc = c->rc_lj == c->rc;
-		auto ks = fp64 ? (single ? k_pairs_list_sparse<true, true, false> : k_pairs_list_sparse<true, false, false>)
+		auto ks = fp64 ? (single ? (ljrc ? k_pairs_list_sparse<true, true, true> : k_pairs_list_sparse<true, true, false>)
+		                         : (ljrc ? k_pairs_list_sparse<true, false, true>
+		                                 : k_pairs_list_sparse<true, false, false>))
 		               : (single ? (ljrc ? k_pairs_list_sparse<false, true, true> : k_pairs_list_sparse<false, true, false>)
 		                         : (ljrc ? k_pairs_list_sparse<false, false, true>
 		                                 : k_pairs_list_sparse<false, false, false>));

@@ -45,6 +45,21 @@ __device__ __forceinline__ void block_sum3(double a, double b, double c, double*
 	block_sum3_at(a, b, c, partials, blockIdx.x);
 }
 
+// Adds the rows first, first + stride, ... of the partials to acc. The sum of a large grid is bound by
+// the latency of these loads, so eight rows are in flight.
+__device__ __forceinline__ void add_partials(const double* partials, int64_t first, int64_t stride, int64_t nparts,
+                                             double* acc) {
+#pragma unroll 8
+	for (int64_t b = first; b < nparts; b += stride) {
+		const double2 lo = __ldcg(reinterpret_cast<const double2*>(partials + b * 4));
+		const double2 hi = __ldcg(reinterpret_cast<const double2*>(partials + b * 4) + 1);
+		acc[0] += lo.x;
+		acc[1] += lo.y;
+		acc[2] += hi.x;
+		acc[3] += hi.y;
+	}
+}
+
 // Run by every thread of every block after the block's partials (written by its thread 0) are in
 // place: the last block to arrive (ticket counter, reset here) sums the nparts partials in a fixed
 // order into out[0..nval) -- the same sums run to run, without a separate reduction launch.
@@ -53,15 +68,16 @@ __device__ __forceinline__ bool last_block_sum(unsigned* counter, const double* 
                                                double* out) {
 	__shared__ int s_last;
 	__shared__ double sh[4][kReduceBlock / 32];
-	__threadfence();
-	__syncthreads();
-	if (threadIdx.x == 0) s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+	// thread 0 wrote the block's partials: only it has to wait for its stores
+	if (threadIdx.x == 0) {
+		__threadfence();
+		s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+	}
 	__syncthreads();
 	if (!s_last) return false;
 	__threadfence();
 	double acc[4] = {0, 0, 0, 0};
-	for (int64_t b = threadIdx.x; b < nparts; b += blockDim.x)
-		for (int k = 0; k < nval; k++) acc[k] += __ldcg(partials + b * 4 + k);
+	add_partials(partials, threadIdx.x, blockDim.x, nparts, acc);
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	for (int k = 0; k < nval; k++) {
 		const double v = warp_sum(acc[k]);
