@@ -11,8 +11,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmdgpu.so")
 SOURCES = ["api.cu", "binning.cu", "pairs.cu", "pairs_brick.cu", "integrate.cu", "peaks.cu", "noalloc.cu", "adjoint.cu",
            "traj.cu", "coupling.cu",
-           "batch.cu", "phase_space.cu", "rigid.cu"]
-HEADERS = ["md_internal.h", "reduce.cuh", "pair_common.cuh", "brick.cuh"]
+           "batch.cu", "phase_space.cu", "rigid.cu", "transfer.cu"]
+HEADERS = ["md_internal.h", "reduce.cuh", "pair_common.cuh", "brick.cuh", "grid_sync.cuh", "transfer.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

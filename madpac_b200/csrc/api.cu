@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "md_internal.h"
+#include "transfer.h"
 
 using mdgpu::Context;
 
@@ -46,28 +47,41 @@ __global__ void k_store_aos(int64_t n, const double* __restrict__ x, const doubl
 	aos[3 * u + 2] = z[s];
 }
 
-// positions -> caller order with the periodic wrap r<0 -> r+L, r>=L -> r-L
-__global__ void k_store_pos(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
-                            const double* __restrict__ z, const int32_t* __restrict__ uidx, Grid g,
-                            double* __restrict__ aos) {
+// Where a read-back packs the molecules in the caller's order (null: not asked for).
+struct Packed {
+	double *r, *v, *F;
+	uint64_t* id;
+	int32_t* cid;
+};
+
+// Every field that a read-back asks for in one pass; positions with the periodic wrap r<0 -> r+L, r>=L -> r-L.
+__global__ void k_pack(int64_t n, Particles p, Grid g, Packed o) {
 	int64_t s = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
 	if (s >= n) return;
-	int64_t u = uidx[s];
-	const double r[3] = {x[s], y[s], z[s]};
-	for (int d = 0; d < 3; d++) {
-		double w = r[d];
-		if (w < 0.0)
-			w = __dadd_rn(w, g.L[d]);
-		else if (w >= g.L[d])
-			w = __dsub_rn(w, g.L[d]);
-		aos[3 * u + d] = w;
+	const int64_t u = p.uidx[s];
+	if (o.r) {
+		const double r[3] = {p.rx[s], p.ry[s], p.rz[s]};
+		for (int d = 0; d < 3; d++) {
+			double w = r[d];
+			if (w < 0.0)
+				w = __dadd_rn(w, g.L[d]);
+			else if (w >= g.L[d])
+				w = __dsub_rn(w, g.L[d]);
+			o.r[3 * u + d] = w;
+		}
 	}
-}
-
-template <typename T>
-__global__ void k_store_scalar(int64_t n, const T* __restrict__ x, const int32_t* __restrict__ uidx, T* __restrict__ out) {
-	int64_t s = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-	if (s < n) out[uidx[s]] = x[s];
+	if (o.v) {
+		o.v[3 * u + 0] = p.vx[s];
+		o.v[3 * u + 1] = p.vy[s];
+		o.v[3 * u + 2] = p.vz[s];
+	}
+	if (o.F) {
+		o.F[3 * u + 0] = p.fx[s];
+		o.F[3 * u + 1] = p.fy[s];
+		o.F[3 * u + 2] = p.fz[s];
+	}
+	if (o.id) o.id[u] = p.id[s];
+	if (o.cid) o.cid[u] = p.cid[s];
 }
 
 // inner cell -> reference halo-inclusive cell index, caller order
@@ -437,6 +451,7 @@ int mdgpu_create(mdgpu_ctx** out, const double length[3], double cutoff, double 
 	if (!full) return MDGPU_ERR_ARG;
 	Context* c = &full->pub.c;
 	*out = &full->pub;
+	transfer_retain();
 	if (ncomp < 1 || ncomp > kMaxSpecies) return fail(c, MDGPU_ERR_ARG, "ncomp must be in 1..8");
 	if (!(cutoff > 0)) return fail(c, MDGPU_ERR_ARG, "cutoff must be positive");
 	if (!(lj_cutoff >= 0)) return fail(c, MDGPU_ERR_ARG, "lj_cutoff must be 0 (= cutoff) or positive");
@@ -534,6 +549,7 @@ int mdgpu_destroy(mdgpu_ctx* ctx) {
 	for (auto ev : full->x.pool) cudaEventDestroy(ev);
 	if (c->stream) cudaStreamDestroy(c->stream);
 	delete full;
+	transfer_release();
 	return MDGPU_OK;
 }
 
@@ -625,22 +641,24 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 	}
 	c->n = n;
 	void* st;
-	MD_CUDA(staging(c, x->stage, sizeof(double) * 3 * n, &st));
+	MD_CUDA(staging(c, x->stage, sizeof(double) * (F ? 9 : 6) * n, &st));
 	double* aos = (double*) st;
-	MD_CUDA(cudaMemcpyAsync(aos, r, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
+	const size_t b3 = sizeof(double) * 3 * n;
+	const CopySpan in[5] = {{(void*) r, aos, b3},
+	                        {(void*) v, aos + 3 * n, b3},
+	                        {(void*) F, aos + 6 * n, b3},
+	                        {(void*) id, c->p.id, sizeof(uint64_t) * n},
+	                        {(void*) cid, c->p.cid, sizeof(int32_t) * n}};
+	MD_CUDA(copy_to_device(c->device, c->stream, in, 5));
 	k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, nullptr, c->p.rx, c->p.ry, c->p.rz);
-	MD_CUDA(cudaMemcpyAsync(aos, v, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-	k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, nullptr, c->p.vx, c->p.vy, c->p.vz);
+	k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 3 * n, nullptr, c->p.vx, c->p.vy, c->p.vz);
 	if (F) {
-		MD_CUDA(cudaMemcpyAsync(aos, F, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-		k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, nullptr, c->p.fx, c->p.fy, c->p.fz);
+		k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 6 * n, nullptr, c->p.fx, c->p.fy, c->p.fz);
 	} else {
 		MD_CUDA(cudaMemsetAsync(c->p.fx, 0, sizeof(double) * n, c->stream));
 		MD_CUDA(cudaMemsetAsync(c->p.fy, 0, sizeof(double) * n, c->stream));
 		MD_CUDA(cudaMemsetAsync(c->p.fz, 0, sizeof(double) * n, c->stream));
 	}
-	MD_CUDA(cudaMemcpyAsync(c->p.id, id, sizeof(uint64_t) * n, cudaMemcpyHostToDevice, c->stream));
-	MD_CUDA(cudaMemcpyAsync(c->p.cid, cid, sizeof(int32_t) * n, cudaMemcpyHostToDevice, c->stream));
 	k_iota<<<blocks_for(n), kThreads, 0, c->stream>>>(n, c->p.uidx);
 	MD_CUDA(cudaGetLastError());
 	MD_CUDA(cudaStreamSynchronize(c->stream));
@@ -657,15 +675,13 @@ int mdgpu_set_state(mdgpu_ctx* ctx, int64_t n, const double* r, const double* v)
 	void* st;
 	MD_CUDA(staging(c, extra(c)->stage, sizeof(double) * 6 * n, &st));
 	double* aos = (double*) st;
+	const CopySpan in[2] = {{(void*) r, aos, sizeof(double) * 3 * n}, {(void*) v, aos + 3 * n, sizeof(double) * 3 * n}};
+	MD_CUDA(copy_to_device(c->device, c->stream, in, 2));
 	if (r) {
-		MD_CUDA(cudaMemcpyAsync(aos, r, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
 		k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, c->p.uidx, c->p.rx, c->p.ry, c->p.rz);
 		c->cells_valid = false;
 	}
-	if (v) {
-		MD_CUDA(cudaMemcpyAsync(aos + 3 * n, v, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-		k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 3 * n, c->p.uidx, c->p.vx, c->p.vy, c->p.vz);
-	}
+	if (v) k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 3 * n, c->p.uidx, c->p.vx, c->p.vy, c->p.vz);
 	count_launches(c, (r ? 1 : 0) + (v ? 1 : 0));
 	MD_CUDA(cudaGetLastError());
 	return MDGPU_OK;
@@ -676,33 +692,30 @@ int mdgpu_get_particles(mdgpu_ctx* ctx, int64_t n, uint64_t* id, int32_t* cid, d
 	Context* c = &ctx->c;
 	if (n != c->n) return fail(c, MDGPU_ERR_ARG, "n does not match the loaded molecules");
 	MD_CUDA(cudaSetDevice(c->device));
+	// the fields asked for one after another in the staging buffer, packed by one kernel
 	void* st;
-	MD_CUDA(staging(c, extra(c)->stage, sizeof(double) * 3 * n, &st));
-	double* aos = (double*) st;
-	struct {
-		double* out;
-		double *x, *y, *z;
-	} sets[3] = {{r, c->p.rx, c->p.ry, c->p.rz}, {v, c->p.vx, c->p.vy, c->p.vz}, {F, c->p.fx, c->p.fy, c->p.fz}};
-	for (auto& s : sets) {
-		if (!s.out) continue;
-		if (s.out == r)   // positions in [0, L) as after LinkedCells::update (the skin mode defers the wrap)
-			k_store_pos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, s.x, s.y, s.z, c->p.uidx, c->g, aos);
-		else
-			k_store_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, s.x, s.y, s.z, c->p.uidx, aos);
-		MD_CUDA(cudaMemcpyAsync(s.out, aos, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->stream));
-		MD_CUDA(cudaStreamSynchronize(c->stream));
-	}
-	if (id) {
-		k_store_scalar<uint64_t><<<blocks_for(n), kThreads, 0, c->stream>>>(n, c->p.id, c->p.uidx, (uint64_t*) aos);
-		MD_CUDA(cudaMemcpyAsync(id, aos, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, c->stream));
-		MD_CUDA(cudaStreamSynchronize(c->stream));
-	}
-	if (cid) {
-		k_store_scalar<int32_t><<<blocks_for(n), kThreads, 0, c->stream>>>(n, c->p.cid, c->p.uidx, (int32_t*) aos);
-		MD_CUDA(cudaMemcpyAsync(cid, aos, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c->stream));
-		MD_CUDA(cudaStreamSynchronize(c->stream));
-	}
+	const size_t b3 = sizeof(double) * 3 * n;
+	MD_CUDA(staging(c, extra(c)->stage, ((r ? 3 : 0) + (v ? 3 : 0) + (F ? 3 : 0) + 2) * sizeof(double) * n, &st));
+	Packed o{};
+	CopySpan out[5];
+	int k = 0;
+	unsigned char* at = (unsigned char*) st;
+	auto place = [&](void* host, size_t bytes) -> void* {
+		if (!host) return nullptr;
+		void* dev = at;
+		out[k++] = CopySpan{host, dev, bytes};
+		at += bytes;
+		return dev;
+	};
+	o.r = (double*) place(r, b3);
+	o.v = (double*) place(v, b3);
+	o.F = (double*) place(F, b3);
+	o.id = (uint64_t*) place(id, sizeof(uint64_t) * n);
+	o.cid = (int32_t*) place(cid, sizeof(int32_t) * n);
+	if (k == 0) return MDGPU_OK;
+	k_pack<<<blocks_for(n), kThreads, 0, c->stream>>>(n, c->p, c->g, o);
 	MD_CUDA(cudaGetLastError());
+	MD_CUDA(copy_to_host(c->device, c->stream, out, k));
 	return MDGPU_OK;
 }
 
@@ -743,8 +756,9 @@ int mdgpu_get_cell_index(mdgpu_ctx* ctx, int64_t n, int64_t* cell) {
 	void* st;
 	MD_CUDA(staging(c, extra(c)->stage, sizeof(int64_t) * n, &st));
 	k_store_refcell<<<blocks_for(n), kThreads, 0, c->stream>>>(n, c->cell, c->p.uidx, c->g, (int64_t*) st);
-	MD_CUDA(cudaMemcpyAsync(cell, st, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, c->stream));
-	MD_CUDA(cudaStreamSynchronize(c->stream));
+	MD_CUDA(cudaGetLastError());
+	const CopySpan out{cell, st, sizeof(int64_t) * n};
+	MD_CUDA(copy_to_host(c->device, c->stream, &out, 1));
 	return MDGPU_OK;
 }
 
@@ -1110,13 +1124,15 @@ int mdgpu_adjoint(mdgpu_ctx* ctx, const double* gF, double gU, double* dL_dr, do
 	void* st;
 	MD_CUDA(staging(c, extra(c)->stage, sizeof(double) * 3 * n, &st));
 	double* aos = (double*) st;
-	MD_CUDA(cudaMemcpyAsync(aos, gF, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
+	const CopySpan in{(void*) gF, aos, sizeof(double) * 3 * n};
+	MD_CUDA(copy_to_device(c->device, c->stream, &in, 1));
 	k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, c->p.uidx, gx, gy, gz);
 	count_launches(c, 1);
 	MD_CUDA(launch_adjoint(c, gx, gy, gz, gU, ox, oy, oz, pgrad, pout));
 	k_store_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, ox, oy, oz, c->p.uidx, aos);
 	count_launches(c, 1);
-	MD_CUDA(cudaMemcpyAsync(dL_dr, aos, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->stream));
+	const CopySpan out{dL_dr, aos, sizeof(double) * 3 * n};
+	MD_CUDA(copy_to_host(c->device, c->stream, &out, 1));
 	double par[2 * KK];
 	MD_CUDA(cudaMemcpyAsync(par, pout, sizeof(par), cudaMemcpyDeviceToHost, c->stream));
 	int sts = check_status(c);

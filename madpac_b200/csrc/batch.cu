@@ -34,6 +34,7 @@
 #include "grid_sync.cuh"
 #include "md_internal.h"
 #include "reduce.cuh"
+#include "transfer.h"
 
 namespace mdgpu {
 namespace {
@@ -879,6 +880,7 @@ int mdgpu_batch_create(mdgpu_batch** out, int32_t nboxes, const double* lengths,
 	mdgpu_batch* h = new (std::nothrow) mdgpu_batch();
 	if (!h) return MDGPU_ERR_ARG;
 	*out = h;
+	transfer_retain();
 	Batch* b = &h->b;
 	if (nboxes < 1) return bfail(b, MDGPU_ERR_ARG, "nboxes must be >= 1");
 	if (ncomp < 1 || ncomp > kMaxSpecies) return bfail(b, MDGPU_ERR_ARG, "ncomp must be in 1..8");
@@ -957,6 +959,7 @@ int mdgpu_batch_destroy(mdgpu_batch* h) {
 	if (b->ev1) cudaEventDestroy(b->ev1);
 	if (b->stream) cudaStreamDestroy(b->stream);
 	delete h;
+	transfer_release();
 	return MDGPU_OK;
 }
 
@@ -971,7 +974,7 @@ int mdgpu_batch_set_particles(mdgpu_batch* h, int64_t ntotal, const uint64_t* id
 	for (int64_t i = 0; i < ntotal; i++)
 		if (cid[i] < 0 || cid[i] >= b->sp.n) return bfail(b, MDGPU_ERR_ARG, "component id out of range");
 	B_CUDA(cudaSetDevice(b->device));
-	const size_t need = sizeof(double) * 3 * ntotal;
+	const size_t need = sizeof(double) * 11 * ntotal;   // a read-back's r, v, F, id and cid
 	if (b->stage_bytes < need) {
 		cudaFree(b->stage);
 		b->stage = nullptr;
@@ -981,15 +984,17 @@ int mdgpu_batch_set_particles(mdgpu_batch* h, int64_t ntotal, const uint64_t* id
 	}
 	b->cur = 0;
 	Particles& p = b->buf[0];
-	B_CUDA(cudaMemcpyAsync(b->stage, r, need, cudaMemcpyHostToDevice, b->stream));
+	const size_t b3 = sizeof(double) * 3 * ntotal;
+	const CopySpan in[4] = {{(void*) r, b->stage, b3},
+	                        {(void*) v, b->stage + 3 * ntotal, b3},
+	                        {(void*) id, p.id, sizeof(uint64_t) * ntotal},
+	                        {(void*) cid, p.cid, sizeof(int32_t) * ntotal}};
+	B_CUDA(copy_to_device(b->device, b->stream, in, 4));
 	k_load3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, b->stage, p.rx, p.ry, p.rz);
-	B_CUDA(cudaMemcpyAsync(b->stage, v, need, cudaMemcpyHostToDevice, b->stream));
-	k_load3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, b->stage, p.vx, p.vy, p.vz);
+	k_load3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, b->stage + 3 * ntotal, p.vx, p.vy, p.vz);
 	B_CUDA(cudaMemsetAsync(p.fx, 0, sizeof(double) * ntotal, b->stream));
 	B_CUDA(cudaMemsetAsync(p.fy, 0, sizeof(double) * ntotal, b->stream));
 	B_CUDA(cudaMemsetAsync(p.fz, 0, sizeof(double) * ntotal, b->stream));
-	B_CUDA(cudaMemcpyAsync(p.id, id, sizeof(uint64_t) * ntotal, cudaMemcpyHostToDevice, b->stream));
-	B_CUDA(cudaMemcpyAsync(p.cid, cid, sizeof(int32_t) * ntotal, cudaMemcpyHostToDevice, b->stream));
 	k_iota32<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, p.uidx);
 	if (b->valid) B_CUDA(cudaMemsetAsync(b->valid, 0, sizeof(int), b->stream));
 	B_CUDA(cudaGetLastError());
@@ -1007,31 +1012,31 @@ int mdgpu_batch_get_particles(mdgpu_batch* h, int64_t ntotal, uint64_t* id, int3
 	if (!b->loaded) return bfail(b, MDGPU_ERR_STATE, "no molecules loaded");
 	B_CUDA(cudaSetDevice(b->device));
 	const Particles& p = b->buf[b->cur];
-	struct {
-		double* out;
-		double *x, *y, *z;
-	} sets[3] = {{r, p.rx, p.ry, p.rz}, {v, p.vx, p.vy, p.vz}, {F, p.fx, p.fy, p.fz}};
-	for (auto& s : sets) {
-		if (!s.out) continue;
-		if (s.out == r)
-			k_store3_wrap<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, s.x, s.y, s.z, p.uidx, b->d_bid, b->d_len,
-			                                                          b->stage);
-		else
-			k_store3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, s.x, s.y, s.z, p.uidx, b->stage);
-		B_CUDA(cudaMemcpyAsync(s.out, b->stage, sizeof(double) * 3 * ntotal, cudaMemcpyDeviceToHost, b->stream));
-		B_CUDA(cudaStreamSynchronize(b->stream));
-	}
-	if (id) {
-		k_store1<uint64_t><<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, p.id, p.uidx, (uint64_t*) b->stage);
-		B_CUDA(cudaMemcpyAsync(id, b->stage, sizeof(uint64_t) * ntotal, cudaMemcpyDeviceToHost, b->stream));
-		B_CUDA(cudaStreamSynchronize(b->stream));
-	}
-	if (cid) {
-		k_store1<int32_t><<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, p.cid, p.uidx, (int32_t*) b->stage);
-		B_CUDA(cudaMemcpyAsync(cid, b->stage, sizeof(int32_t) * ntotal, cudaMemcpyDeviceToHost, b->stream));
-		B_CUDA(cudaStreamSynchronize(b->stream));
-	}
+	CopySpan out[5];
+	int k = 0;
+	unsigned char* at = (unsigned char*) b->stage;
+	auto place = [&](void* host, size_t bytes) -> void* {
+		void* dev = at;
+		out[k++] = CopySpan{host, dev, bytes};
+		at += bytes;
+		return dev;
+	};
+	const size_t b3 = sizeof(double) * 3 * ntotal;
+	if (r)
+		k_store3_wrap<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, p.rx, p.ry, p.rz, p.uidx, b->d_bid, b->d_len,
+		                                                          (double*) place(r, b3));
+	if (v)
+		k_store3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, p.vx, p.vy, p.vz, p.uidx, (double*) place(v, b3));
+	if (F)
+		k_store3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, p.fx, p.fy, p.fz, p.uidx, (double*) place(F, b3));
+	if (id)
+		k_store1<uint64_t><<<blocks(ntotal), kThreads, 0, b->stream>>>(
+		    ntotal, p.id, p.uidx, (uint64_t*) place(id, sizeof(uint64_t) * ntotal));
+	if (cid)
+		k_store1<int32_t><<<blocks(ntotal), kThreads, 0, b->stream>>>(
+		    ntotal, p.cid, p.uidx, (int32_t*) place(cid, sizeof(int32_t) * ntotal));
 	B_CUDA(cudaGetLastError());
+	B_CUDA(copy_to_host(b->device, b->stream, out, k));
 	return MDGPU_OK;
 }
 

@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "md_internal.h"
+#include "transfer.h"
 #include "reduce.cuh"
 
 namespace mdgpu {
@@ -1179,7 +1180,7 @@ struct mdgpu_rigid {
 	std::vector<mdgpu_site> sites_in;
 	std::vector<mdgpu_charge> charges_in;
 	std::vector<double> inertia_in, mix_in;
-	double* stage = nullptr;    // 4 x cap host <-> device staging
+	double* stage = nullptr;    // kRigidPlanes x cap host <-> device staging
 	double* partials = nullptr; // per-block reduction partials (4 doubles per block of the pair kernel)
 	double* scal = nullptr;     // [0..2] pair sums, [3..4] kinetic sums
 	double* steps = nullptr;    // 5 doubles per step of mdgpu_rigid_run
@@ -1540,7 +1541,7 @@ int ensure_capacity(mdgpu_rigid* h, int64_t n) {
 	RG_CUDA(cudaMalloc(&h->es, sizeof(double) * 3 * std::max(1, h->hp.ns_max) * n));
 	RG_CUDA(cudaMalloc(&h->rec, sizeof(float4) * kRecFloat4 * n));
 	RG_CUDA(cudaMalloc(&h->ss, sizeof(double) * 2 * kRigidPlanes * n));
-	RG_CUDA(cudaMalloc(&h->stage, sizeof(double) * 4 * n));
+	RG_CUDA(cudaMalloc(&h->stage, sizeof(double) * kRigidPlanes * n));
 	RG_CUDA(cudaMalloc(&h->partials, sizeof(double) * 4 * nblocks(n * kRigidLanes)));
 	h->cap = n;
 	return MDGPU_OK;
@@ -1822,11 +1823,11 @@ int mdgpu_rigid_set_particles(mdgpu_rigid* h, int64_t n, const uint64_t* id, con
 	st = ensure_capacity(h, n);
 	if (st) return st;
 	const unsigned nb4 = (unsigned) nblocks(4 * n), nb3 = (unsigned) nblocks(3 * n);
-	RG_CUDA(cudaMemcpyAsync(h->stage, q, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, c->stream));
+	const CopySpan in[2] = {{(void*) q, h->stage, sizeof(double) * 4 * n},
+	                        {(void*) D, h->stage + 4 * n, sizeof(double) * 3 * n}};
+	RG_CUDA(copy_to_device(c->device, c->stream, in, 2));
 	k_scatter_soa<double><<<nb4, kRigidThreads, 0, c->stream>>>(n, 4, h->stage, h->q);
-	RG_CUDA(cudaStreamSynchronize(c->stream));
-	RG_CUDA(cudaMemcpyAsync(h->stage, D, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-	k_scatter_soa<double><<<nb3, kRigidThreads, 0, c->stream>>>(n, 3, h->stage, h->D);
+	k_scatter_soa<double><<<nb3, kRigidThreads, 0, c->stream>>>(n, 3, h->stage + 4 * n, h->D);
 	RG_CUDA(cudaMemsetAsync(h->M, 0, sizeof(double) * 3 * n, c->stream));
 	RG_CUDA(cudaGetLastError());
 	RG_CUDA(cudaStreamSynchronize(c->stream));
@@ -1846,13 +1847,17 @@ int mdgpu_rigid_get_particles(mdgpu_rigid* h, int64_t n, uint64_t* id, int32_t* 
 		const double* src;
 		int k;
 	} sets[3] = {{q, h->q, 4}, {D, h->D, 3}, {M, h->M, 3}};
+	CopySpan out[3];
+	int k = 0;
+	double* at = h->stage;
 	for (auto& s : sets) {
 		if (!s.out) continue;
-		k_gather_soa<double><<<(unsigned) nblocks(s.k * n), kRigidThreads, 0, c->stream>>>(n, s.k, s.src, h->stage);
-		RG_CUDA(cudaMemcpyAsync(s.out, h->stage, sizeof(double) * s.k * n, cudaMemcpyDeviceToHost, c->stream));
-		RG_CUDA(cudaStreamSynchronize(c->stream));
+		k_gather_soa<double><<<(unsigned) nblocks(s.k * n), kRigidThreads, 0, c->stream>>>(n, s.k, s.src, at);
+		out[k++] = CopySpan{s.out, at, sizeof(double) * s.k * n};
+		at += s.k * n;
 	}
 	RG_CUDA(cudaGetLastError());
+	RG_CUDA(copy_to_host(c->device, c->stream, out, k));
 	return MDGPU_OK;
 }
 

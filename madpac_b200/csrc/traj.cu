@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "md_internal.h"
+#include "transfer.h"
 
 namespace mdgpu {
 
@@ -259,8 +260,8 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 		cudaFree(t->rbar);
 		cudaFree(t->gs);
 		t->rbar = t->gs = nullptr;
-		// rbar, vbar, Fbar (3n each), cm (n), rows (3n); gs, os (3n each), pgrad, par
-		e = cudaMalloc(&t->rbar, sizeof(double) * 13 * n);
+		// rbar, vbar, Fbar (3n each), cm (n), rows (6n); gs, os (3n each), pgrad, par
+		e = cudaMalloc(&t->rbar, sizeof(double) * 16 * n);
 		if (e == cudaSuccess) e = cudaMalloc(&t->gs, sizeof(double) * (6 * n + nb * 2 * KK + 2 * KK));
 		if (e != cudaSuccess) return set_cuda_error(c, e, "cudaMalloc (trajectory cotangents)");
 		t->cap_n = n;
@@ -305,7 +306,8 @@ int mdgpu_traj_backward(mdgpu_ctx* ctx, const double* gF, double gU, double* dL_
 	const int64_t n = c->n;
 	const double dt = t->dt;
 	// cotangents of the final state: Fbar = gF, rbar = vbar = 0; parameter sums 0
-	e = cudaMemcpyAsync(t->rows, gF, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream);
+	const CopySpan in{(void*) gF, t->rows, sizeof(double) * 3 * n};
+	e = copy_to_device(c->device, c->stream, &in, 1);
 	if (e == cudaSuccess) {
 		k_rows_to_planes<<<nblk(n), kT, 0, c->stream>>>(n, t->rows, t->Fbar);
 		count_launches(c, 1);
@@ -347,13 +349,11 @@ int mdgpu_traj_backward(mdgpu_ctx* ctx, const double* gF, double gU, double* dL_
 	double par[2 * KK];
 	if (e == cudaSuccess) {
 		k_planes_to_rows<<<nblk(n), kT, 0, c->stream>>>(n, t->rbar, t->rows);
-		count_launches(c, 1);
-		e = cudaMemcpyAsync(dL_dr0, t->rows, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->stream);
-	}
-	if (e == cudaSuccess && dL_dv0) {
-		k_planes_to_rows<<<nblk(n), kT, 0, c->stream>>>(n, t->vbar, t->rows + 0);
-		count_launches(c, 1);
-		e = cudaMemcpyAsync(dL_dv0, t->rows, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->stream);
+		if (dL_dv0) k_planes_to_rows<<<nblk(n), kT, 0, c->stream>>>(n, t->vbar, t->rows + 3 * n);
+		count_launches(c, dL_dv0 ? 2 : 1);
+		const CopySpan out[2] = {{dL_dr0, t->rows, sizeof(double) * 3 * n}, {dL_dv0, t->rows + 3 * n, sizeof(double) * 3 * n}};
+		e = cudaGetLastError();
+		if (e == cudaSuccess) e = copy_to_host(c->device, c->stream, out, 2);
 	}
 	if (e == cudaSuccess) e = cudaMemcpyAsync(par, t->par, sizeof(par), cudaMemcpyDeviceToHost, c->stream);
 	if (e != cudaSuccess) return set_cuda_error(c, e, "trajectory backward");

@@ -1,0 +1,216 @@
+// Copies between a caller's pageable arrays and the device.
+//
+// A plain cudaMemcpyAsync to or from pageable memory is staged by the driver in one thread: 12 GB/s
+// measured, and on arrays the caller has just allocated that thread also takes every page fault. Here the
+// arrays are cut into chunks that go through pinned buffers: each host thread copies its chunks between
+// the caller's memory and one of its two buffers while the other one's DMA runs. Large copies use several
+// threads, which live for the call only; small ones the calling thread alone.
+//
+// Measured, state of 1,048,576 molecules on 16 cores: 88 MB out in 4.3 ms (13.4 by plain copies), into
+// arrays just allocated in 7 ms (25), 50 MB in in 1.9 ms (3.8); four threads 9 ms into new arrays.
+#include "transfer.h"
+
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <mutex>
+#include <new>
+#include <thread>
+#include <vector>
+
+namespace mdgpu {
+namespace {
+
+constexpr size_t kChunk = 512 * 1024;       // bytes per DMA: about 10 us on the link
+constexpr size_t kPerThread = 1536 * 1024;  // bytes that pay for another thread (20 us to start one)
+constexpr int kMaxThreads = 8;
+constexpr size_t kMaxIdle = 2 * kMaxThreads;   // lanes kept for later calls: 16 MB of pinned memory
+
+// One thread's pair of pinned chunks.
+struct Lane {
+	unsigned char* buf[2] = {nullptr, nullptr};
+	cudaEvent_t done[2] = {nullptr, nullptr};   // the buffer's DMA
+	int device = -1;                            // whose events these are
+};
+
+std::mutex g_mutex;
+std::vector<Lane> g_idle;
+int g_users = 0;
+
+void free_lane(Lane& l) {
+	for (int b = 0; b < 2; b++) {
+		if (l.done[b]) cudaEventDestroy(l.done[b]);
+		if (l.buf[b]) cudaFreeHost(l.buf[b]);
+	}
+	l = Lane{};
+}
+
+// A lane of the device from the idle ones, or a new one.
+cudaError_t take_lane(int device, Lane& l) {
+	{
+		std::lock_guard<std::mutex> lock(g_mutex);
+		for (size_t k = 0; k < g_idle.size(); k++)
+			if (g_idle[k].device == device) {
+				l = g_idle[k];
+				g_idle.erase(g_idle.begin() + (std::ptrdiff_t) k);
+				return cudaSuccess;
+			}
+	}
+	l = Lane{};
+	l.device = device;
+	cudaError_t e = cudaSuccess;
+	for (int b = 0; b < 2 && e == cudaSuccess; b++) {
+		e = cudaHostAlloc((void**) &l.buf[b], kChunk, cudaHostAllocPortable);
+		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.done[b], cudaEventDisableTiming);
+	}
+	if (e != cudaSuccess) free_lane(l);
+	return e;
+}
+
+// Back to the idle ones; every DMA of the lane has ended.
+void give_lane(Lane& l) {
+	try {
+		std::lock_guard<std::mutex> lock(g_mutex);
+		if (g_users > 0 && g_idle.size() < kMaxIdle) {
+			g_idle.push_back(l);
+			return;
+		}
+	} catch (...) {
+	}
+	free_lane(l);
+}
+
+struct Job {
+	int device;
+	cudaStream_t stream;
+	std::vector<CopySpan> chunks;
+	std::atomic<size_t> next{0};
+	std::atomic<int> err{(int) cudaSuccess};
+
+	bool ok() const { return err.load(std::memory_order_relaxed) == (int) cudaSuccess; }
+	bool check(cudaError_t e) {
+		if (e != cudaSuccess) err.store((int) e, std::memory_order_relaxed);
+		return e == cudaSuccess;
+	}
+	const CopySpan* take() {
+		const size_t k = next.fetch_add(1, std::memory_order_relaxed);
+		return k < chunks.size() && ok() ? &chunks[k] : nullptr;
+	}
+};
+
+// One thread's share of a copy. Never leaves with a DMA of its lane in flight.
+void work(Job& job, Lane& l, bool to_host) {
+	if (!job.check(cudaSetDevice(job.device))) return;
+	const CopySpan* pending[2] = {nullptr, nullptr};   // the chunk in each buffer's DMA
+	for (int b = 0;; b ^= 1) {
+		// buffer b is free once its DMA has ended (and, on the way out, its chunk is copied)
+		if (pending[b]) {
+			if (job.check(cudaEventSynchronize(l.done[b])) && to_host)
+				std::memcpy(pending[b]->host, l.buf[b], pending[b]->bytes);
+			pending[b] = nullptr;
+		}
+		const CopySpan* c = job.take();
+		if (!c) break;
+		if (!to_host) std::memcpy(l.buf[b], c->host, c->bytes);
+		const cudaError_t e = to_host ? cudaMemcpyAsync(l.buf[b], c->dev, c->bytes, cudaMemcpyDeviceToHost, job.stream)
+		                              : cudaMemcpyAsync(c->dev, l.buf[b], c->bytes, cudaMemcpyHostToDevice, job.stream);
+		if (!job.check(e)) break;
+		if (!job.check(cudaEventRecord(l.done[b], job.stream))) {
+			cudaStreamSynchronize(job.stream);
+			break;
+		}
+		pending[b] = c;
+	}
+	for (int b = 0; b < 2; b++)
+		if (pending[b] && job.check(cudaEventSynchronize(l.done[b])) && to_host)
+			std::memcpy(pending[b]->host, l.buf[b], pending[b]->bytes);
+}
+
+bool pinned(const void* host) {
+	cudaPointerAttributes a{};
+	if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+		cudaGetLastError();
+		return false;
+	}
+	return a.type == cudaMemoryTypeHost;
+}
+
+cudaError_t copy(int device, cudaStream_t s, const CopySpan* spans, int n, bool to_host) {
+	try {
+		Job job;
+		job.device = device;
+		job.stream = s;
+		bool direct = false;
+		size_t total = 0;
+		for (int k = 0; k < n; k++) {
+			if (!spans[k].host || spans[k].bytes == 0) continue;
+			if (spans[k].bytes >= kChunk && pinned(spans[k].host)) {
+				// pinned by the caller: the DMA runs at the link's rate by itself
+				const cudaError_t e =
+				    to_host ? cudaMemcpyAsync(spans[k].host, spans[k].dev, spans[k].bytes, cudaMemcpyDeviceToHost, s)
+				            : cudaMemcpyAsync(spans[k].dev, spans[k].host, spans[k].bytes, cudaMemcpyHostToDevice, s);
+				if (e != cudaSuccess) return e;
+				direct = true;
+				continue;
+			}
+			for (size_t o = 0; o < spans[k].bytes; o += kChunk)
+				job.chunks.push_back(CopySpan{(unsigned char*) spans[k].host + o, (unsigned char*) spans[k].dev + o,
+				                              std::min(kChunk, spans[k].bytes - o)});
+			total += spans[k].bytes;
+		}
+		if (!job.chunks.empty()) {
+			const int cores = std::max(1, (int) std::thread::hardware_concurrency() / 2);
+			const int want = std::max(1, std::min({kMaxThreads, cores, (int) (total / kPerThread)}));
+			std::vector<Lane> lanes;
+			lanes.reserve((size_t) want);
+			cudaError_t e = cudaSuccess;
+			for (int t = 0; t < want; t++) {
+				Lane l;
+				e = take_lane(device, l);
+				if (e != cudaSuccess) break;   // fewer lanes do as well
+				lanes.push_back(l);
+			}
+			if (lanes.empty()) return e;
+			std::vector<std::thread> threads;
+			threads.reserve(lanes.size());
+			try {
+				for (size_t t = 1; t < lanes.size(); t++)
+					threads.emplace_back([&job, &lanes, t, to_host] { work(job, lanes[t], to_host); });
+			} catch (...) {   // no more threads: those that run take all chunks
+			}
+			work(job, lanes[0], to_host);
+			for (auto& t : threads) t.join();
+			for (Lane& l : lanes) give_lane(l);
+			if (!job.ok()) return (cudaError_t) job.err.load();
+		}
+		return direct && to_host ? cudaStreamSynchronize(s) : cudaSuccess;
+	} catch (const std::bad_alloc&) {
+		return cudaErrorMemoryAllocation;
+	}
+}
+
+}  // namespace
+
+cudaError_t copy_to_host(int device, cudaStream_t s, const CopySpan* spans, int n) {
+	return copy(device, s, spans, n, true);
+}
+
+cudaError_t copy_to_device(int device, cudaStream_t s, const CopySpan* spans, int n) {
+	return copy(device, s, spans, n, false);
+}
+
+void transfer_retain() {
+	std::lock_guard<std::mutex> lock(g_mutex);
+	g_users++;
+}
+
+void transfer_release() {
+	std::vector<Lane> old;
+	{
+		std::lock_guard<std::mutex> lock(g_mutex);
+		if (--g_users == 0) old.swap(g_idle);
+	}
+	for (Lane& l : old) free_lane(l);
+}
+
+}  // namespace mdgpu

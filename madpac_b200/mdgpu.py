@@ -345,9 +345,9 @@ class Batch:
 
     def getParticles(self) -> Dict[str, np.ndarray]:
         n = self.ntotal
-        ids = np.zeros(n, dtype=np.uint64)
-        cid = np.zeros(n, dtype=np.int32)
-        r, v, F = np.zeros((n, 3)), np.zeros((n, 3)), np.zeros((n, 3))
+        ids = np.empty(n, dtype=np.uint64)
+        cid = np.empty(n, dtype=np.int32)
+        r, v, F = np.empty((n, 3)), np.empty((n, 3)), np.empty((n, 3))
         self._check(self.lib.mdgpu_batch_get_particles(self.h, n, _ptr(ids), _ptr(cid), _ptr(r), _ptr(v), _ptr(F)))
         return dict(id=ids, cid=cid, r=r, v=v, F=F)
 
@@ -513,10 +513,10 @@ class RigidLinkedCells:
 
     def getParticles(self) -> Dict[str, np.ndarray]:
         n = self.n
-        ids = np.zeros(n, dtype=np.uint64)
-        cid = np.zeros(n, dtype=np.int32)
-        r, v, F, D, M = (np.zeros((n, 3)) for _ in range(5))
-        q = np.zeros((n, 4))
+        ids = np.empty(n, dtype=np.uint64)
+        cid = np.empty(n, dtype=np.int32)
+        r, v, F, D, M = (np.empty((n, 3)) for _ in range(5))
+        q = np.empty((n, 4))
         self._check(self.lib.mdgpu_rigid_get_particles(self.h, n, _ptr(ids), _ptr(cid), _ptr(r), _ptr(v), _ptr(F),
                                                        _ptr(q), _ptr(D), _ptr(M)))
         return dict(id=ids, cid=cid, r=r, v=v, F=F, q=q, D=D, M=M)
@@ -657,15 +657,15 @@ class LinkedCells:
         return u.value, w.value, p.value
 
     def getCellIndexOfMolecule(self) -> np.ndarray:
-        out = np.zeros(self.n, dtype=np.int64)
+        out = np.empty(self.n, dtype=np.int64)
         self._check(self.lib.mdgpu_get_cell_index(self.h, self.n, _ptr(out)))
         return out
 
     def getParticles(self) -> Dict[str, np.ndarray]:
         n = self.n
-        ids = np.zeros(n, dtype=np.uint64)
-        cid = np.zeros(n, dtype=np.int32)
-        r, v, F = np.zeros((n, 3)), np.zeros((n, 3)), np.zeros((n, 3))
+        ids = np.empty(n, dtype=np.uint64)
+        cid = np.empty(n, dtype=np.int32)
+        r, v, F = np.empty((n, 3)), np.empty((n, 3)), np.empty((n, 3))
         self._check(self.lib.mdgpu_get_particles(self.h, n, _ptr(ids), _ptr(cid), _ptr(r), _ptr(v), _ptr(F)))
         return dict(id=ids, cid=cid, r=r, v=v, F=F)
 
@@ -742,7 +742,7 @@ class LinkedCells:
         """(dL/dr (n, 3), dL/d eps_ab, dL/d sigma_ab) for cotangents gF = dL/dF, gU = dL/dUpot at the
         current positions (after update)."""
         ns = len(self.components)
-        gr = np.zeros((self.n, 3))
+        gr = np.empty((self.n, 3))
         ge = np.zeros((ns, ns))
         gs = np.zeros((ns, ns))
         self._check(self.lib.mdgpu_adjoint(self.h, _ptr(_c64(gF, shape=(self.n, 3))), float(gU), _ptr(gr), _ptr(ge),
@@ -761,7 +761,7 @@ class LinkedCells:
         trajectory of the last trajForward: (dL/dr0, dL/dv0, dL/d eps_ab, dL/d sigma_ab, recomputed
         steps). The context holds the start state afterwards."""
         ns = len(self.components)
-        gr, gv = np.zeros((self.n, 3)), np.zeros((self.n, 3))
+        gr, gv = np.empty((self.n, 3)), np.empty((self.n, 3))
         ge, gs = np.zeros((ns, ns)), np.zeros((ns, ns))
         rec = ctypes.c_int64()
         self._check(self.lib.mdgpu_traj_backward(self.h, _ptr(_c64(gF, shape=(self.n, 3))), float(gU), _ptr(gr),
