@@ -172,7 +172,7 @@ cudaError_t launch_bin(Context* c, bool permute_forces);
 // once unless *c->rebuild == c->step_id; the sorted arrays end in c->p (buffer roles unchanged)
 // and c->perm[i] holds the index before the sort of the molecule now at i. `extra` (nextra planes of
 // n doubles, `scratch` as large) are sorted with the molecules. With `always` it builds in every
-// launch (the per-step binning of the trajectory adjoint: one launch instead of launch_bin's six).
+// launch (the per-step binning of the trajectory adjoint: one launch instead of launch_bin's five).
 cudaError_t launch_rebuild(Context* c, const Grid& g, double* extra = nullptr, double* scratch = nullptr,
                            int nextra = 0, bool always = false);
 cudaError_t launch_pairs(Context* c);                 // partials -> scalars[0..2] (U6sum, W, npairs)

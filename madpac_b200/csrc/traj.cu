@@ -159,7 +159,7 @@ void free_traj(Context* c) {
 namespace {
 
 // The binning of every step: the cooperative rebuild in its always-build form, one launch (the
-// same (cell, id) order as launch_bin's six kernels).
+// same (cell, id) order as launch_bin's five kernels).
 cudaError_t traj_bin(Context* c) { return launch_rebuild(c, c->g, nullptr, nullptr, 0, true); }
 
 // One reference step (NVE) on the context: pre-kick and drift, binning, forces, closing kick.
