@@ -538,6 +538,8 @@ int mdgpu_destroy(mdgpu_ctx* ctx) {
 	cudaFree(c->rb_look);
 	cudaFree(c->rb_slot);
 	cudaFree(c->tickets);
+	cudaFree(c->trav_list);
+	cudaFree(c->trav_counts);
 	cudaFree(c->brick_kind);
 	cudaFree(full->x.stage.ptr);
 	if (c->h_scalars) cudaFreeHost(c->h_scalars);
@@ -637,6 +639,11 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 		const int64_t blocks = (n + kReduceBlock - 1) / kReduceBlock;
 		c->partial_cap = (blocks > bricks ? blocks : bricks) + 1024;
 		MD_CUDA(cudaMalloc(&c->partials, sizeof(double) * 4 * c->partial_cap));
+		if (!c->trav_list) {
+			MD_CUDA(cudaMalloc(&c->trav_list, sizeof(int32_t) * bricks));
+			MD_CUDA(cudaMalloc(&c->trav_counts, sizeof(unsigned) * 2));
+			c->trav_cap = (int) bricks;
+		}
 		c->cap = n;
 	}
 	c->n = n;

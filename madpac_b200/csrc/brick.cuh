@@ -641,7 +641,7 @@ constexpr int kHitWords = 24;
 // Bound by instruction issue (of 250,047 molecules at rc = 2.5: staging 25 %, filter 30 %, evaluation
 // 45 %); three CTAs per SM. Measured, us per traversal, against one warp per cell with per-lane index
 // lists and the reference's operation order: 250,047 molecules at rc = 2.5 121 (328), at rc = 3.0 190
-// (381); a 786,432-molecule two-species slab 530 (1339); 16,384 molecules 24 (34).
+// (381); 16,384 molecules of two species 26 (34).
 template <bool kSingle, bool kLjIsRc, int kWords>
 __device__ __forceinline__ void pairs(const Const& p, const Box& bx, int brick, int64_t slot, unsigned char* smem,
                                       const double* rx, const double* ry, const double* rz, const int32_t* cid,
@@ -803,6 +803,141 @@ __device__ __forceinline__ void pairs(const Const& p, const Box& bx, int brick, 
 	}
 	if (same) atomicOr(status, kStatusSamePosition);
 	block_sum3_at(U, W, NP, partials, slot);
+}
+
+// Lanes per molecule for g molecules on one warp: the largest power of two with lpm * g <= 32.
+__device__ __forceinline__ int lanes_per_molecule(int g) {
+	int lpm = 1;
+	while (lpm * 2 * g <= 32) lpm *= 2;
+	return lpm;
+}
+
+// The traversal of a sparse brick by one warp, without CTA barriers. Its shared memory: the staged
+// molecules' double images, component ids and staged cells, the cells' first slots and first molecules.
+struct SparseTraverse {
+	double img[3 * kSparseCap];
+	int cs[65], gst[64];
+	unsigned char comp[kSparseCap], cell[kSparseCap];
+};
+
+// Forces on the molecules of brick `brick` if it is sparse (see kSparseCap); false otherwise. Of the staged
+// region each molecule tests all, lpm lanes per molecule: with a few molecules in all, a filter costs more
+// than it saves. Candidates outside the 27 cells around the molecule's own are left out, as in pairs.
+template <bool kSingle, bool kLjIsRc>
+__device__ __forceinline__ bool pairs_sparse(const Const& p, const Box& bx, int brick, SparseTraverse& S,
+                                             const PairParams* __restrict__ pp, const double* rx, const double* ry,
+                                             const double* rz, const int32_t* cid, const int32_t* cstart, double* fx,
+                                             double* fy, double* fz, double* partials, int* status) {
+	const int lane = threadIdx.x & 31;
+	const Grid& g = bx.g;
+	const int bc[3] = {brick % bx.nb[0], (brick / bx.nb[0]) % bx.nb[1], brick / (bx.nb[0] * bx.nb[1])};
+	// staged cells 2 lane and 2 lane + 1, as in stage_rows
+	double t0, t1;
+	const int gy = staged_coord(bx, 1, bc[1], (lane >> 1) & 3, t0, t1);
+	const int gz = staged_coord(bx, 2, bc[2], lane >> 3, t0, t1);
+	const int row0 = bx.coff + (gz * g.nc[1] + gy) * g.nc[0];
+	const int ca = row0 + staged_coord(bx, 0, bc[0], 2 * (lane & 1), t0, t1);
+	const int cb = row0 + staged_coord(bx, 0, bc[0], 2 * (lane & 1) + 1, t0, t1);
+	const int sa = cstart[ca], ea = cstart[ca + 1], sb = cstart[cb], eb = cstart[cb + 1];
+	const int na = max(0, ea - sa), nb = max(0, eb - sb);
+	int inc = na + nb;
+	for (int o = 1; o < 32; o <<= 1) {
+		const int y = __shfl_up_sync(kFull, inc, o);
+		if (lane >= o) inc += y;
+	}
+	const int slot_a = inc - (na + nb);
+	const int total = __shfl_sync(kFull, inc, 31);
+	// the own cells' counts in lanes 0..7, and their sum
+	int ic = 0;
+	const bool ok = lane < kWarps && own_cell(bx, brick, lane, ic);
+	const int ia = __shfl_sync(kFull, na, ic >> 1), ib = __shfl_sync(kFull, nb, ic >> 1);
+	const int c_own = ok ? ((ic & 1) ? ib : ia) : 0;
+	const int n_own = __reduce_add_sync(kFull, c_own);
+	if (total > kSparseCap || n_own > 32) return false;
+	double U = 0.0, W = 0.0, NP = 0.0;
+	if (n_own > 0) {
+		S.cs[2 * lane] = slot_a;
+		S.cs[2 * lane + 1] = slot_a + na;
+		S.gst[2 * lane] = sa;
+		S.gst[2 * lane + 1] = sb;
+		if (lane == 31) S.cs[64] = total;
+		__syncwarp();
+		double sh_l = 0.0, k_l = 0.0;   // lane 4 d + l: the shift of staged coordinate l of dimension d
+		if (lane < 12) staged_coord(bx, lane >> 2, bc[lane >> 2], lane & 3, sh_l, k_l);
+		for (int t = lane; t < ((total + 31) & ~31); t += 32) {
+			int c = 0;
+			for (int step = 32; step; step >>= 1)
+				if (S.cs[c + step] <= t) c += step;
+			const double shx = __shfl_sync(kFull, sh_l, c & 3), shy = __shfl_sync(kFull, sh_l, 4 + ((c >> 2) & 3));
+			const double shz = __shfl_sync(kFull, sh_l, 8 + (c >> 4));
+			if (t < total) {
+				const int gi = S.gst[c] + (t - S.cs[c]);
+				S.img[3 * t] = __dadd_rn(rx[gi], shx);
+				S.img[3 * t + 1] = __dadd_rn(ry[gi], shy);
+				S.img[3 * t + 2] = __dadd_rn(rz[gi], shz);
+				S.comp[t] = (unsigned char) cid[gi];
+				S.cell[t] = (unsigned char) c;
+			}
+		}
+		__syncwarp();
+		int own = c_own;   // inclusive prefix of the own cells' counts in lanes 0..7
+		for (int o = 1; o < kWarps; o <<= 1) {
+			const int y = __shfl_up_sync(kFull, own, o);
+			if (lane >= o) own += y;
+		}
+		const int lpm = lanes_per_molecule(n_own);
+		const int sub = lane & (lpm - 1), t = lane / lpm;
+		const bool act = t < n_own;
+		int w = 0;
+		for (int k = 0; k < kWarps - 1; k++) w += t >= __shfl_sync(kFull, own, k) ? 1 : 0;
+		const int before = w > 0 ? w - 1 : 0;
+		const int prev = __shfl_sync(kFull, own, before);
+		const int oc = __shfl_sync(kFull, ic, w);
+		const int e = act ? t - (w > 0 ? prev : 0) : 0;
+		const int slot_i = min(S.cs[oc] + e, max(0, total - 1)), gi = S.gst[oc] + e;
+		const double xi = S.img[3 * slot_i], yi = S.img[3 * slot_i + 1], zi = S.img[3 * slot_i + 2];
+		const int ti = kSingle ? 0 : S.comp[slot_i];
+		Sums64 s64{0.0, 0.0, 0.0, 0.0, 0.0, 0, 0};
+		bool same = false;
+		for (int j0 = 0; j0 < total; j0 += lpm) {
+			const int j = min(j0 + sub, total - 1);
+			const int cj = S.cell[j];
+			const bool near = abs((cj & 3) - (oc & 3)) <= 1 && abs(((cj >> 2) & 3) - ((oc >> 2) & 3)) <= 1 &&
+			                  abs((cj >> 4) - (oc >> 4)) <= 1;
+			const bool v = act && j0 + sub < total && j != slot_i && near;
+			const int pk = kSingle ? 0 : ti * p.ns + S.comp[j];
+			lj64<kSingle, kLjIsRc>(__dsub_rn(xi, S.img[3 * j]), __dsub_rn(yi, S.img[3 * j + 1]),
+			                       __dsub_rn(zi, S.img[3 * j + 2]), v, p.rc2, p.rclj2, pp->eps24[pk], pp->sig2[pk],
+			                       pp->shift6[pk], s64, same);
+		}
+		if (kSingle) sums64_finish<kLjIsRc>(s64, pp->eps24[0], pp->shift6[0]);
+		U = s64.u;
+		W = s64.w;
+		NP = (double) s64.np;
+		for (int o = 1; o < lpm; o <<= 1) {
+			s64.x += __shfl_xor_sync(kFull, s64.x, o);
+			s64.y += __shfl_xor_sync(kFull, s64.y, o);
+			s64.z += __shfl_xor_sync(kFull, s64.z, o);
+		}
+		if (act && sub == 0) {
+			fx[gi] = s64.x;
+			fy[gi] = s64.y;
+			fz[gi] = s64.z;
+			if (!(isfinite(s64.x) && isfinite(s64.y) && isfinite(s64.z))) atomicOr(status, kStatusNonFinite);
+		}
+		if (same) atomicOr(status, kStatusSamePosition);
+		U = warp_sum(U);
+		W = warp_sum(W);
+		NP = warp_sum(NP);
+		__syncwarp();   // the next brick of this warp stages into the same memory
+	}
+	if (lane == 0) {
+		partials[4 * (int64_t) brick + 0] = U;
+		partials[4 * (int64_t) brick + 1] = W;
+		partials[4 * (int64_t) brick + 2] = NP;
+		partials[4 * (int64_t) brick + 3] = 0.0;
+	}
+	return true;
 }
 
 // Entries of each lane's write-combining ring in build_lists: up to 7 unwritten entries plus the
@@ -1070,13 +1205,6 @@ __device__ __forceinline__ double finish(const Kick& k, int64_t gi, double Fx, d
 // finish; the atomic is skipped when the value there is already as large).
 __device__ __forceinline__ void drift_flush(unsigned* dmax) {
 	if (dmax && threadIdx.x == 0 && drift_slot() > __ldcg(dmax)) atomicMax(dmax, drift_slot());
-}
-
-// Lanes per molecule for g molecules on one warp: the largest power of two with lpm * g <= 32.
-__device__ __forceinline__ int lanes_per_molecule(int g) {
-	int lpm = 1;
-	while (lpm * 2 * g <= 32) lpm *= 2;
-	return lpm;
 }
 
 #ifndef MDGPU_LIST_ACC

@@ -110,6 +110,11 @@ struct Context {
 	int* status = nullptr;          // device status word
 	unsigned* tickets = nullptr;    // last-block counters of the in-kernel reductions (self-resetting)
 	PairParams* d_pp = nullptr;     // device copy of the pair parameters
+	// the traversal's bricks that are not sparse (trav_cap entries; null: no sparse bricks looked for),
+	// their number and the queue over them
+	int32_t* trav_list = nullptr;
+	int trav_cap = 0;
+	unsigned* trav_counts = nullptr;
 	// Verlet-skin mode of mdgpu_step / mdgpu_run (skin > 0): per-molecule candidate lists of radius
 	// rc + skin on a frozen cell structure, rebuilt (with the binning) by device-side gating when a
 	// molecule has moved more than skin/2 since the last build

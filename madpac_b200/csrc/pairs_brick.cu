@@ -35,11 +35,46 @@ __global__ void __launch_bounds__(brick::kThreads, kTraverseMinBlocks)
                   double* __restrict__ partials, int* __restrict__ status, const int* __restrict__ gate,
                   brick::Lists lists, unsigned* ticket, double* scalars) {
 	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ int s_item;
 	brick::load_params(smem, brick::layout(p.s_cap, true, brick::kHitWords), pp, p.ns);
-	brick::pairs<kSingle, kLjIsRc, brick::kHitWords>(p, bx, blockIdx.x, blockIdx.x, smem, rx, ry, rz, cid, cstart, fx,
-	                                                 fy, fz, partials, status);
+	// every brick, one CTA each, or (lists.counts) those that k_pairs_sparse left: a resident grid takes
+	// them from a queue
+	const bool queue = lists.counts != nullptr;
+	const int nwork = queue ? (int) *(volatile unsigned*) lists.counts : 0;
+	int b = (int) blockIdx.x;
+	do {
+		if (queue) {
+			__syncthreads();
+			if (threadIdx.x == 0) s_item = (int) atomicAdd(lists.counts + 1, 1u);
+			__syncthreads();
+			if (s_item >= nwork) break;
+			b = lists.blist[s_item];
+		}
+		brick::pairs<kSingle, kLjIsRc, brick::kHitWords>(p, bx, b, b, smem, rx, ry, rz, cid, cstart, fx, fy, fz,
+		                                                 partials, status);
+	} while (queue);
 	// U6 sum, virial sum and pair count over every brick, by the last CTA (ticket null: by a later launch)
 	if (ticket) last_block_sum(ticket, partials, gridDim.x, 3, scalars);
+}
+
+// The sparse bricks of a traversal (vapour: a few molecules), one warp each; the others go to counts[0],
+// blist. A CTA of the dense kernel spends 9000 cycles on such a brick, most of them waiting for its
+// staging's loads; here as many bricks as warps fit wait at once. Measured, us per traversal: the 786,432-
+// molecule slab 532 -> 394 (its sparse bricks 26), a vapour of 100,000 at density 0.02 987 -> 45.
+template <bool kSingle, bool kLjIsRc>
+__global__ void __launch_bounds__(brick::kThreads, 4)
+    k_pairs_sparse(brick::Const p, brick::Box bx, int nbricks, const double* __restrict__ rx,
+                   const double* __restrict__ ry, const double* __restrict__ rz, const int32_t* __restrict__ cid,
+                   const int32_t* __restrict__ cstart, const PairParams* __restrict__ pp, double* __restrict__ fx,
+                   double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ partials,
+                   int* __restrict__ status, brick::Lists lists) {
+	__shared__ brick::SparseTraverse s_warp[brick::kWarps];
+	const int b = (int) blockIdx.x * brick::kWarps + (int) (threadIdx.x >> 5);
+	if (b >= nbricks) return;
+	if (!brick::pairs_sparse<kSingle, kLjIsRc>(p, bx, b, s_warp[threadIdx.x >> 5], pp, rx, ry, rz, cid, cstart, fx, fy,
+	                                           fz, partials, status) &&
+	    (threadIdx.x & 31) == 0)
+		lists.blist[atomicAdd(lists.counts, 1u)] = b;
 }
 
 // Verlet-skin build step (runs only when *gate is this step's id): the lists, no forces.
@@ -248,9 +283,10 @@ bool fold_in_traversal(const Context* c, const Plan& P) { return P.nbricks <= kT
 template <typename K, typename... Extra>
 cudaError_t go(Context* c, const Plan& P, K kern, const int* gate, const brick::Lists& lists, Extra... extra) {
 	cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) P.bytes);
-	// the list kernel runs as a resident grid over a queue of the dense bricks when the sparse ones
-	// are evaluated apart (lists.kind set); otherwise one CTA per brick
-	const int grid = lists.kind && sizeof...(Extra) > 0 ? resident_grid(c, kern, P.bytes, P.nbricks) : P.nbricks;
+	// the list kernel runs as a resident grid over a queue of the dense bricks when the sparse ones are
+	// evaluated apart (lists.kind set, or lists.counts in the traversal); otherwise one CTA per brick
+	const bool queue = lists.kind || (lists.counts && !lists.nbr);
+	const int grid = queue ? resident_grid(c, kern, P.bytes, P.nbricks) : P.nbricks;
 	if (r == cudaSuccess)
 		kern<<<grid, brick::kThreads, P.bytes, c->stream>>>(P.p, P.bx, c->p.rx, c->p.ry, c->p.rz, c->p.cid,
 		                                                         c->cell_start, c->d_pp, c->p.fx, c->p.fy, c->p.fz,
@@ -310,12 +346,38 @@ brick::Lists lists_of(Context* c) {
 
 }  // namespace
 
+// Whether a traversal looks for sparse bricks first: where there are several rounds of bricks and many
+// are expected to be sparse -- a dilute fluid, or one that leaves much of the box nearly empty (the density
+// around a typical molecule is well above the mean). A homogeneous liquid has none, and skips the launch.
+bool sparse_traversal(const Context* c, const Plan& P) {
+	if (!c->trav_list || P.nbricks > c->trav_cap || P.nbricks < 2 * kTraverseMinBlocks * c->num_sms) return false;
+	const Grid& g = c->g;
+	const double rho = (double) c->n / (g.L[0] * g.L[1] * g.L[2]);
+	const double cell = g.cell_length[0] * g.cell_length[1] * g.cell_length[2];
+	return 64.0 * rho * cell <= 0.75 * brick::kSparseCap || c->rho_typ > 1.5 * rho;
+}
+
 cudaError_t launch_pairs_brick(Context* c) {
 	const Plan P = plan(c, c->g, c->rc, 0);
 	prof_begin(c, 1);
-	cudaError_t e = dispatch<0>(c, P, nullptr, brick::Lists{});
+	brick::Lists l{};
+	cudaError_t e = cudaSuccess;
+	const bool sparse = sparse_traversal(c, P);
+	if (sparse) {
+		l.counts = c->trav_counts;
+		l.blist = c->trav_list;
+		e = cudaMemsetAsync(l.counts, 0, sizeof(unsigned) * 2, c->stream);
+		const bool single = c->sp.n == 1, ljrc = c->rc_lj == c->rc;
+		auto ks = single ? (ljrc ? k_pairs_sparse<true, true> : k_pairs_sparse<true, false>)
+		                 : (ljrc ? k_pairs_sparse<false, true> : k_pairs_sparse<false, false>);
+		if (e == cudaSuccess)
+			ks<<<(P.nbricks + brick::kWarps - 1) / brick::kWarps, brick::kThreads, 0, c->stream>>>(
+			    P.p, P.bx, P.nbricks, c->p.rx, c->p.ry, c->p.rz, c->p.cid, c->cell_start, c->d_pp, c->p.fx, c->p.fy,
+			    c->p.fz, c->partials, c->status, l);
+	}
+	if (e == cudaSuccess) e = dispatch<0>(c, P, nullptr, l);
 	if (e == cudaSuccess) e = cudaGetLastError();
-	prof_end(c, 1, 1);
+	prof_end(c, 1, sparse ? 2 : 1);
 	if (e != cudaSuccess || fold_in_traversal(c, P)) return e;
 	return launch_reduce(c, P.nbricks, c->scalars, 3);
 }

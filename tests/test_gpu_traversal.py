@@ -50,6 +50,33 @@ def test_traversal_equals_the_gather_kernel(n, density, rc, species):
         assert np.max(np.abs(got[1] - ref[1])) <= 1e-12 * max(frms, 1.0)
 
 
+@pytest.mark.parametrize("system", ["vapour", "dilute", "slab"])
+@pytest.mark.parametrize("species", [1, 2])
+def test_sparse_bricks(system, species):
+    """Boxes of several rounds of bricks, most of them with a few molecules, which go one per warp: a vapour,
+    a dilute fluid with bricks on both sides of the limits (128 staged, 32 own molecules), a liquid slab."""
+    if system == "slab":
+        s = W.config_c3(9, 41000)
+        if species == 1:
+            s.components, s.mix, s.cid = [W.Component(1.0, 1.0, 1.0, True)], np.ones((0, 2)), np.zeros_like(s.cid)
+    else:
+        n, density = (3100, 0.01) if system == "vapour" else (40001, 0.13)
+        s = jittered(n, density, 2.5, 11, species)
+    out = []
+    for kind in (0, 1):
+        lc = M.LinkedCells.from_system(s)
+        lc.setPairKernel(kind)
+        lc.update()
+        sums = lc.traversePairs()
+        again = lc.traversePairs()
+        assert sums == again
+        out.append((np.array(sums), lc.getParticles()["F"]))
+        lc.close()
+    assert out[0][0][2] == out[1][0][2]
+    assert np.max(np.abs(out[0][0] - out[1][0])) <= 1e-12 * np.max(np.abs(out[1][0]))
+    assert np.max(np.abs(out[0][1] - out[1][1])) <= 1e-12 * max(np.sqrt(np.mean(out[1][1] ** 2)), 1.0)
+
+
 def test_lj_cutoff_below_the_cutoff():
     """rcLJ < rc: pairs between the two count as pairs and exert no force."""
     s = jittered(1372, 0.8, 2.8, 7, 1)
