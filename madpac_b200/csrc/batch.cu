@@ -5,22 +5,32 @@
 // all boxes' cells in one cell-start array (box b's cells at [coff_b, coff_b + ncells_b)), and all
 // boxes' 2x2x2 bricks numbered globally (box b's at [brick0_b, brick0_b + nbricks_b)).
 //
-// One step = one cooperative launch of k_batch_step, CTAs co-resident, three phases:
+// One step = one cooperative launch of k_batch_step, CTAs co-resident, three phases (binning every step):
 //   A  per box (one CTA per box, boxes dealt largest first in a snake order): Leapfrog pre-kick
 //      and drift (Molecule::upd_preF, molecules/Molecule.cpp:128-135), periodic wrap and cell
 //      index (LinkedCells::update, particleContainer/LinkedCells.cpp:165-180, 535-551; paths
 //      relative to madpac/mardyn/), then a counting sort of the box in shared memory: cell counts by
-//      shared atomics, block scan, arrival scatter of (id, old slot), per-cell insertion sort by id,
-//      gather into the other buffer. The result is the same (cell, id) order as the single-box path.
+//      shared atomics, block scan, arrival scatter of (id, old slot), rank by id within the cell,
+//      move into the other buffer. The result is the same (cell, id) order as the single-box path.
 //   -- grid barrier --
 //   B  all bricks of all boxes (static stride or an atomic queue): brick::pairs, the single-box
 //      pair kernel's per-brick work, so forces match the single-box path bit for bit.
 //   -- grid barrier --
 //   C  per box: Leapfrog post-kick (Molecule::upd_postF, Molecule.cpp:193-205), sum m v^2, and the
 //      box's brick partials in a fixed order -> the step record {Upot, virial, sum m v^2, pairs}.
-// Boxes are independent, so nothing crosses between CTAs except at the two barriers. Each barrier
-// wait is bounded by a time limit; a wait that runs out sets the timeout status, the CTA skips the
-// rest of the step, and every later launch returns at once until the host has read the status.
+// Boxes are independent, so nothing crosses between CTAs except at the two barriers.
+//
+// In the Verlet-skin mode (mdgpu_batch_set_skin) phase A kicks, drifts and checks every box, and flags those
+// whose lists must be rebuilt (in a step of the 512-box ensemble about one in twelve). After the barrier
+// the CTAs first take the flagged boxes from a queue (wrap, binning, sort: one CTA per box), then the
+// bricks of the other boxes, whose lists still hold, and only then those of the flagged boxes, which wait
+// for their box (long since done), build their lists and evaluate them. The list evaluation applies the
+// closing kick. A barrier between rebuilding and evaluating kept the whole device waiting for the largest
+// rebuilt box, 300 of a step's 850 us:
+// 512 boxes of 1.17 M molecules took 852 us per step, now 712.
+//
+// Each wait (barrier or box) is bounded by a time limit; a wait that runs out sets the timeout status, the
+// CTA skips the rest of the step, and every later launch returns at once until the host has read the status.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,7 +71,6 @@ struct Kick {
 struct StepArgs {
 	brick::Const pc;
 	const BatchBox* boxes;
-	const int32_t* brick0;      // nboxes + 1
 	const int32_t* order;       // boxes by decreasing molecule count
 	int nboxes, total_bricks;
 	Particles src, dst;
@@ -72,7 +81,7 @@ struct StepArgs {
 	double* partials;
 	double* record;             // nboxes x 4
 	int* status;
-	unsigned* bar;              // [0] arrivals, [1] generation, [2] brick queue
+	unsigned* bar;              // [0] arrivals, [1] generation, [2] brick queue, [3] rebuild queue, [4] its length
 	int64_t timeout_ns;
 	int integrate;              // 0: wrap, bin and forces only (initial force evaluation)
 	int dynamic;                // 0: bricks by static stride, 1: by atomic queue
@@ -81,8 +90,11 @@ struct StepArgs {
 	int skin;
 	double half_skin2;
 	brick::Lists lists;
-	int* box_flag;              // nboxes: 1 = built in this step
+	int* box_flag;              // nboxes: 0 = lists hold, 1 = to be rebuilt in this step, 2 = rebuilt
+	int32_t* rebuild;           // the flagged boxes of the step
+	const int32_t* brick_box;   // box of each brick
 	int* valid;                 // 0: every box builds (molecules just loaded)
+	brick::Kick close;          // the closing kick, applied by the list evaluation (mode 2)
 	int build_cap;              // staged capacity of the list build
 	brick::Const lc;            // constants of the list evaluation (its staged capacity)
 };
@@ -97,6 +109,49 @@ __host__ __device__ inline size_t bin_bytes(int64_t n, int64_t m) {
 	o += sizeof(uint16_t) * (size_t) n;           // cell of each old slot
 	o += sizeof(uint16_t) * (size_t) n;           // old slot in arrival order
 	return o;
+}
+
+// Molecules from(0..n) to to(0..n) of the other buffer, the CTA's threads side by side. A box's largest CTA
+// is on the critical path of the step, so kMove molecules per thread are in flight and every load comes
+// before the first store (the compiler cannot tell the buffers apart and would wait for each field).
+constexpr int kMove = 2;
+template <typename From, typename To>
+__device__ __forceinline__ void move_all(int n, int tid, From from, To to, const Particles& src, const Particles& dst) {
+	for (int f0 = tid; f0 < n; f0 += kMove * kThreads) {
+		double d[kMove][6];
+		uint64_t id[kMove];
+		int32_t ci[kMove], ui[kMove];
+#pragma unroll
+		for (int u = 0; u < kMove; u++) {
+			const int f = f0 + u * kThreads;
+			if (f >= n) continue;
+			const int64_t i = from(f);
+			d[u][0] = src.rx[i];
+			d[u][1] = src.ry[i];
+			d[u][2] = src.rz[i];
+			d[u][3] = src.vx[i];
+			d[u][4] = src.vy[i];
+			d[u][5] = src.vz[i];
+			id[u] = src.id[i];
+			ci[u] = src.cid[i];
+			ui[u] = src.uidx[i];
+		}
+#pragma unroll
+		for (int u = 0; u < kMove; u++) {
+			const int f = f0 + u * kThreads;
+			if (f >= n) continue;
+			const int64_t i = to(f);
+			dst.rx[i] = d[u][0];
+			dst.ry[i] = d[u][1];
+			dst.rz[i] = d[u][2];
+			dst.vx[i] = d[u][3];
+			dst.vy[i] = d[u][4];
+			dst.vz[i] = d[u][5];
+			dst.id[i] = id[u];
+			dst.cid[i] = ci[u];
+			dst.uidx[i] = ui[u];
+		}
+	}
 }
 
 // Phase A for box b: kick-drift, wrap, bin and sort src -> dst.
@@ -115,43 +170,65 @@ __device__ void bin_box(const StepArgs& a, const BatchBox& B, unsigned char* sme
 	for (int c = tid; c < m; c += kThreads) s_count[c] = 0;
 	__syncthreads();
 	bool bad = false;
-	for (int t = tid; t < n; t += kThreads) {
-		const int64_t i = poff + t;
-		double r[3] = {a.src.rx[i], a.src.ry[i], a.src.rz[i]};
-		if (a.integrate) {
-			// Molecule::upd_preF with vcorr = 1: v = vcorr*v + dtInv2m*F; r += dt*v
-			const double k = a.kick.pre[a.src.cid[i]];
-			double* vp[3] = {a.src.vx, a.src.vy, a.src.vz};
-			const double* fp[3] = {a.src.fx, a.src.fy, a.src.fz};
+	for (int t0 = tid; t0 < n; t0 += kMove * kThreads) {
+		double rr[kMove][3], vv[kMove][3], ff[kMove][3], k[kMove];
+#pragma unroll
+		for (int u = 0; u < kMove; u++) {
+			if (t0 + u * kThreads >= n) continue;
+			const int64_t i = poff + t0 + u * kThreads;
+			rr[u][0] = a.src.rx[i];
+			rr[u][1] = a.src.ry[i];
+			rr[u][2] = a.src.rz[i];
+			if (a.integrate) {
+				k[u] = a.kick.pre[a.src.cid[i]];
+				vv[u][0] = a.src.vx[i];
+				vv[u][1] = a.src.vy[i];
+				vv[u][2] = a.src.vz[i];
+				ff[u][0] = a.src.fx[i];
+				ff[u][1] = a.src.fy[i];
+				ff[u][2] = a.src.fz[i];
+			}
+		}
+#pragma unroll
+		for (int u = 0; u < kMove; u++) {
+			const int t = t0 + u * kThreads;
+			if (t >= n) continue;
+			const int64_t i = poff + t;
+			double* r = rr[u];
+			if (a.integrate) {
+				// Molecule::upd_preF with vcorr = 1: v = vcorr*v + dtInv2m*F; r += dt*v
+				for (int d = 0; d < 3; d++) {
+					vv[u][d] = __dadd_rn(__dmul_rn(1.0, vv[u][d]), __dmul_rn(k[u], ff[u][d]));
+					r[d] = __dadd_rn(r[d], __dmul_rn(a.dt, vv[u][d]));
+				}
+				a.src.vx[i] = vv[u][0];
+				a.src.vy[i] = vv[u][1];
+				a.src.vz[i] = vv[u][2];
+			}
+			int ci[3];
 			for (int d = 0; d < 3; d++) {
-				const double v = __dadd_rn(__dmul_rn(1.0, vp[d][i]), __dmul_rn(k, fp[d][i]));
-				vp[d][i] = v;
-				r[d] = __dadd_rn(r[d], __dmul_rn(a.dt, v));
+				const double x = r[d];
+				double xw = x;
+				if (x < 0.0)
+					xw = __dadd_rn(x, g.L[d]);
+				else if (x >= g.L[d])
+					xw = __dsub_rn(x, g.L[d]);
+				r[d] = xw;
+				int c = (int) floor(__ddiv_rn(__dsub_rn(xw, g.halo_min[d]), g.cell_length[d]));
+				if (c < 1 || c > g.nc[d]) {
+					bad = true;
+					c = c < 1 ? 1 : g.nc[d];
+				}
+				ci[d] = c - 1;
+				if (!(x == x)) bad = true;
 			}
+			a.src.rx[i] = r[0];
+			a.src.ry[i] = r[1];
+			a.src.rz[i] = r[2];
+			const int c = (ci[2] * g.nc[1] + ci[1]) * g.nc[0] + ci[0];
+			s_cell[t] = (uint16_t) c;
+			atomicAdd(&s_count[c], 1);
 		}
-		int ci[3];
-		for (int d = 0; d < 3; d++) {
-			const double x = r[d];
-			double xw = x;
-			if (x < 0.0)
-				xw = __dadd_rn(x, g.L[d]);
-			else if (x >= g.L[d])
-				xw = __dsub_rn(x, g.L[d]);
-			r[d] = xw;
-			int c = (int) floor(__ddiv_rn(__dsub_rn(xw, g.halo_min[d]), g.cell_length[d]));
-			if (c < 1 || c > g.nc[d]) {
-				bad = true;
-				c = c < 1 ? 1 : g.nc[d];
-			}
-			ci[d] = c - 1;
-			if (!(x == x)) bad = true;
-		}
-		a.src.rx[i] = r[0];
-		a.src.ry[i] = r[1];
-		a.src.rz[i] = r[2];
-		const int c = (ci[2] * g.nc[1] + ci[1]) * g.nc[0] + ci[0];
-		s_cell[t] = (uint16_t) c;
-		atomicAdd(&s_count[c], 1);
 	}
 	if (bad) atomicOr(a.status, kStatusOutsideHalo);
 	__syncthreads();
@@ -198,141 +275,164 @@ __device__ void bin_box(const StepArgs& a, const BatchBox& B, unsigned char* sme
 		s_from[pos] = (uint16_t) t;
 	}
 	__syncthreads();
-	// per-cell insertion sort by (id, old slot)
-	for (int c = tid; c < m; c += kThreads) {
-		const int s = s_start[c], e = s_start[c + 1];
-		for (int k = s + 1; k < e; k++) {
-			const uint64_t key = s_key[k];
-			const uint16_t fr = s_from[k];
-			int j = k - 1;
-			while (j >= s && (s_key[j] > key || (s_key[j] == key && s_from[j] > fr))) {
-				s_key[j + 1] = s_key[j];
-				s_from[j + 1] = s_from[j];
-				j--;
-			}
-			s_key[j + 1] = key;
-			s_from[j + 1] = fr;
-		}
-	}
-	__syncthreads();
-	// gather into the new order
-	for (int f = tid; f < n; f += kThreads) {
-		const int64_t from = poff + s_from[f], to = poff + f;
-		a.dst.rx[to] = a.src.rx[from];
-		a.dst.ry[to] = a.src.ry[from];
-		a.dst.rz[to] = a.src.rz[from];
-		a.dst.vx[to] = a.src.vx[from];
-		a.dst.vy[to] = a.src.vy[from];
-		a.dst.vz[to] = a.src.vz[from];
-		a.dst.id[to] = s_key[f];
-		a.dst.cid[to] = a.src.cid[from];
-		a.dst.uidx[to] = a.src.uidx[from];
-	}
+	// each molecule to its rank by (id, old slot) among its cell's, all fields into the other buffer (an
+	// insertion sort per cell, by one thread each, took a third of a large box's time)
+	move_all(
+	    n, tid, [&](int f) { return poff + s_from[f]; },
+	    [&](int f) {
+		    const uint16_t fr = s_from[f];
+		    const int c = s_cell[fr], s = s_start[c], e = s_start[c + 1];
+		    const uint64_t key = s_key[f];
+		    int pos = s;
+#pragma unroll 4
+		    for (int j = s; j < e; j++) pos += (s_key[j] < key || (s_key[j] == key && s_from[j] < fr)) ? 1 : 0;
+		    return poff + pos;
+	    },
+	    a.src, a.dst);
 	__syncthreads();
 }
 
-// Phase C for box b: post-kick, sum m v^2, the box's brick partials -> record.
+// Phase C for box b: post-kick, sum m v^2, the box's brick partials -> record. In the Verlet-skin steps
+// the list evaluation has applied the kick and summed m v^2 into its partials.
 __device__ void finish_box(const StepArgs& a, const BatchBox& B, int b) {
-	__shared__ double s_w[kThreads / 32];
+	__shared__ double s_w[4][kThreads / 32];
 	const int tid = threadIdx.x;
 	const Particles& P = a.skin ? a.src : a.dst;
-	double mv2 = 0.0;
-	bool bad = false;
-	for (int t = tid; t < B.n; t += kThreads) {
-		const int64_t i = B.poff + t;
-		const int ty = P.cid[i];
-		double vx = P.vx[i], vy = P.vy[i], vz = P.vz[i];
-		if (a.integrate) {
-			const double k = a.kick.post[ty];
-			vx = __dadd_rn(vx, __dmul_rn(k, P.fx[i]));
-			vy = __dadd_rn(vy, __dmul_rn(k, P.fy[i]));
-			vz = __dadd_rn(vz, __dmul_rn(k, P.fz[i]));
-			P.vx[i] = vx;
-			P.vy[i] = vy;
-			P.vz[i] = vz;
+	double sum[4] = {0.0, 0.0, 0.0, 0.0};   // U, W, pairs, m v^2
+	add_partials(a.partials, B.brick0 + tid, kThreads, B.brick0 + B.bx.nb[0] * B.bx.nb[1] * B.bx.nb[2], sum);
+	if (a.close.mode == 0) {
+		double mv2 = 0.0;
+		bool bad = false;
+		for (int t = tid; t < B.n; t += kThreads) {
+			const int64_t i = B.poff + t;
+			const int ty = P.cid[i];
+			double vx = P.vx[i], vy = P.vy[i], vz = P.vz[i];
+			if (a.integrate) {
+				const double fx = P.fx[i], fy = P.fy[i], fz = P.fz[i];
+				const double k = a.kick.post[ty];
+				vx = __dadd_rn(vx, __dmul_rn(k, fx));
+				vy = __dadd_rn(vy, __dmul_rn(k, fy));
+				vz = __dadd_rn(vz, __dmul_rn(k, fz));
+				P.vx[i] = vx;
+				P.vy[i] = vy;
+				P.vz[i] = vz;
+			}
+			const double v2 = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
+			mv2 += __dmul_rn(a.kick.mass[ty], v2);
+			if (!(v2 == v2) || isinf(v2)) bad = true;
 		}
-		const double v2 = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
-		mv2 += __dmul_rn(a.kick.mass[ty], v2);
-		if (!(v2 == v2) || isinf(v2)) bad = true;
+		if (bad) atomicOr(a.status, kStatusNonFinite);
+		sum[3] = mv2;
 	}
-	if (bad) atomicOr(a.status, kStatusNonFinite);
-	mv2 = warp_sum(mv2);
-	if ((tid & 31) == 0) s_w[tid >> 5] = mv2;
+	for (int k = 0; k < 4; k++) {
+		const double v = warp_sum(sum[k]);
+		if ((tid & 31) == 0) s_w[k][tid >> 5] = v;
+	}
 	__syncthreads();
 	if (tid == 0) {
-		double s = 0.0;
-		for (int w = 0; w < kThreads / 32; w++) s += s_w[w];
-		double U = 0.0, W = 0.0, NP = 0.0;
-		const int nbr = B.bx.nb[0] * B.bx.nb[1] * B.bx.nb[2];
-		for (int k = 0; k < nbr; k++) {
-			const double* q = a.partials + 4 * (int64_t) (B.brick0 + k);
-			U += q[0];
-			W += q[1];
-			NP += q[2];
+		for (int k = 0; k < 4; k++) {
+			sum[k] = 0.0;
+			for (int w = 0; w < kThreads / 32; w++) sum[k] += s_w[k][w];
 		}
 		double* rec = a.record + 4 * (int64_t) b;
-		rec[0] = U * 0.5 / 6.;
-		rec[1] = W * 0.5;
-		rec[2] = s;
-		rec[3] = NP * 0.5;
+		rec[0] = sum[0] * 0.5 / 6.;
+		rec[1] = sum[1] * 0.5;
+		rec[2] = sum[3];
+		rec[3] = sum[2] * 0.5;
 	}
 	__syncthreads();
 }
 
 // Phase A of the Verlet-skin mode for box b: kick-drift in place (no wrap), displacement against
-// the positions of the box's last build; when one moved more than skin/2 (or the lists are not
-// valid) the box is wrapped, binned and sorted into the scratch buffer and copied back.
-__device__ void skin_box(const StepArgs& a, const BatchBox& B, int b, unsigned char* smem) {
+// the positions of the box's last build; the box is flagged and queued for a rebuild when one moved more
+// than skin/2 (or the lists are not valid).
+__device__ void skin_box(const StepArgs& a, const BatchBox& B, int b) {
 	__shared__ int s_any;
 	const int tid = threadIdx.x;
 	if (tid == 0) s_any = 0;
 	__syncthreads();
 	if (a.integrate) {
 		bool moved = false;
-		for (int t = tid; t < B.n; t += kThreads) {
-			const int64_t i = B.poff + t;
-			const double k = a.kick.pre[a.src.cid[i]];
-			const double vx0 = a.src.vx[i], vy0 = a.src.vy[i], vz0 = a.src.vz[i];
-			const double fx = a.src.fx[i], fy = a.src.fy[i], fz = a.src.fz[i];
-			const double x0 = a.src.rx[i], y0 = a.src.ry[i], z0 = a.src.rz[i];
-			const double vx = __dadd_rn(__dmul_rn(1.0, vx0), __dmul_rn(k, fx));
-			const double vy = __dadd_rn(__dmul_rn(1.0, vy0), __dmul_rn(k, fy));
-			const double vz = __dadd_rn(__dmul_rn(1.0, vz0), __dmul_rn(k, fz));
-			const double x = __dadd_rn(x0, __dmul_rn(a.dt, vx));
-			const double y = __dadd_rn(y0, __dmul_rn(a.dt, vy));
-			const double z = __dadd_rn(z0, __dmul_rn(a.dt, vz));
-			a.src.vx[i] = vx;
-			a.src.vy[i] = vy;
-			a.src.vz[i] = vz;
-			a.src.rx[i] = x;
-			a.src.ry[i] = y;
-			a.src.rz[i] = z;
-			const double dx = x - a.lists.rx_ref[i], dy = y - a.lists.ry_ref[i], dz = z - a.lists.rz_ref[i];
-			if (!(dx * dx + dy * dy + dz * dz <= a.half_skin2)) moved = true;
+		for (int t0 = tid; t0 < B.n; t0 += kMove * kThreads) {
+			double v0[kMove][3], f[kMove][3], r0[kMove][3], ref[kMove][3], k[kMove];
+#pragma unroll
+			for (int u = 0; u < kMove; u++) {
+				if (t0 + u * kThreads >= B.n) continue;
+				const int64_t i = B.poff + t0 + u * kThreads;
+				k[u] = a.kick.pre[a.src.cid[i]];
+				v0[u][0] = a.src.vx[i];
+				v0[u][1] = a.src.vy[i];
+				v0[u][2] = a.src.vz[i];
+				f[u][0] = a.src.fx[i];
+				f[u][1] = a.src.fy[i];
+				f[u][2] = a.src.fz[i];
+				r0[u][0] = a.src.rx[i];
+				r0[u][1] = a.src.ry[i];
+				r0[u][2] = a.src.rz[i];
+				ref[u][0] = a.lists.rx_ref[i];
+				ref[u][1] = a.lists.ry_ref[i];
+				ref[u][2] = a.lists.rz_ref[i];
+			}
+#pragma unroll
+			for (int u = 0; u < kMove; u++) {
+				if (t0 + u * kThreads >= B.n) continue;
+				const int64_t i = B.poff + t0 + u * kThreads;
+				double v[3], r[3];
+				for (int d = 0; d < 3; d++) {
+					v[d] = __dadd_rn(__dmul_rn(1.0, v0[u][d]), __dmul_rn(k[u], f[u][d]));
+					r[d] = __dadd_rn(r0[u][d], __dmul_rn(a.dt, v[d]));
+				}
+				a.src.vx[i] = v[0];
+				a.src.vy[i] = v[1];
+				a.src.vz[i] = v[2];
+				a.src.rx[i] = r[0];
+				a.src.ry[i] = r[1];
+				a.src.rz[i] = r[2];
+				const double dx = r[0] - ref[u][0], dy = r[1] - ref[u][1], dz = r[2] - ref[u][2];
+				if (!(dx * dx + dy * dy + dz * dz <= a.half_skin2)) moved = true;
+			}
 		}
 		if (moved) s_any = 1;
 	}
 	__syncthreads();
-	const bool rebuild = s_any != 0 || *a.valid == 0;
-	if (rebuild) {
-		StepArgs a2 = a;
-		a2.integrate = 0;
-		bin_box(a2, B, smem);
-		for (int t = tid; t < B.n; t += kThreads) {
-			const int64_t i = B.poff + t;
-			a.src.rx[i] = a.dst.rx[i];
-			a.src.ry[i] = a.dst.ry[i];
-			a.src.rz[i] = a.dst.rz[i];
-			a.src.vx[i] = a.dst.vx[i];
-			a.src.vy[i] = a.dst.vy[i];
-			a.src.vz[i] = a.dst.vz[i];
-			a.src.id[i] = a.dst.id[i];
-			a.src.cid[i] = a.dst.cid[i];
-			a.src.uidx[i] = a.dst.uidx[i];
-		}
+	if (tid == 0) {
+		const bool rebuild = s_any != 0 || *a.valid == 0;
+		a.box_flag[b] = rebuild ? 1 : 0;
+		if (rebuild) a.rebuild[atomicAdd(a.bar + 4, 1u)] = b;
 	}
-	if (tid == 0) a.box_flag[b] = rebuild ? 1 : 0;
 	__syncthreads();
+}
+
+// The rebuild of a flagged box: wrapped, binned and sorted into the scratch buffer and copied back; then its
+// bricks may be built and evaluated.
+__device__ void rebuild_box(const StepArgs& a, const BatchBox& B, int b, unsigned char* smem) {
+	const int tid = threadIdx.x;
+	StepArgs a2 = a;
+	a2.integrate = 0;
+	bin_box(a2, B, smem);
+	move_all(B.n, tid, [&](int t) { return B.poff + t; }, [&](int t) { return B.poff + t; }, a.dst, a.src);
+	__threadfence();
+	__syncthreads();
+	if (tid == 0) atomicExch(a.box_flag + b, 2);
+}
+
+// Waits (bounded) until flagged box b is rebuilt; false when the wait ran out. Ends with a CTA barrier.
+__device__ bool await_box(const StepArgs& a, int b, int* s_flag) {
+	if (threadIdx.x == 0) {
+		const unsigned* flag = reinterpret_cast<const unsigned*>(a.box_flag + b);
+		const uint64_t t0 = global_ns();
+		while (load_acquire(flag) != 2u) {
+			__nanosleep(100);
+			if ((int64_t) (global_ns() - t0) > a.timeout_ns) {
+				atomicOr(a.status, kStatusTimeout);
+				*s_flag = 1;
+				break;
+			}
+		}
+		__threadfence();
+	}
+	__syncthreads();
+	return *s_flag == 0;
 }
 
 // Boxes of this CTA: j-th in the snake order over boxes sorted by decreasing size.
@@ -354,39 +454,29 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch_step(StepArgs a) {
 	__syncthreads();
 	if (s_flag) return;   // an earlier launch gave up at a barrier: do nothing until the host resets
 
-	// ---- A: per box kick-drift, wrap, bin, sort ----------------------------------------------
+	// ---- A: per box kick-drift, and wrap, bin, sort (or, with the skin, the displacement check) ------------
 	if (a.skin)
-		for_my_boxes(a, [&](int b) { skin_box(a, a.boxes[b], b, smem); });
+		for_my_boxes(a, [&](int b) { skin_box(a, a.boxes[b], b); });
 	else
 		for_my_boxes(a, [&](int b) { bin_box(a, a.boxes[b], smem); });
 	if (!grid_barrier(a.bar, a.status, a.timeout_ns, &s_flag)) return;
 
-	// brick of a global brick index: box with brick0[box] <= item < brick0[box + 1]
-	auto box_of = [&](int item) {
-		int lo = 0, hi = a.nboxes - 1;
-		while (lo < hi) {
-			const int mid = (lo + hi + 1) >> 1;
-			if (a.brick0[mid] <= item)
-				lo = mid;
-			else
-				hi = mid - 1;
-		}
-		return lo;
-	};
-	// every brick once, by static stride or from the queue bar[q]
-	auto for_bricks = [&](int q, auto&& f) {
+	// every brick once, by static stride or from the queue bar[2] (those that `skip` names are left out)
+	auto next_brick = [&](int& at, auto&& skip) {
 		if (a.dynamic) {
-			for (;;) {
-				if (threadIdx.x == 0) s_item = (int) atomicAdd(a.bar + q, 1u);
-				__syncthreads();
-				const int item = s_item;
-				__syncthreads();
-				if (item >= a.total_bricks) break;
-				f(item);
+			__syncthreads();
+			if (threadIdx.x == 0) {
+				int item = (int) atomicAdd(a.bar + 2, 1u);
+				while (item < a.total_bricks && skip(item)) item = (int) atomicAdd(a.bar + 2, 1u);
+				s_item = item;
 			}
+			__syncthreads();
+			at = s_item;
 		} else {
-			for (int item = blockIdx.x; item < a.total_bricks; item += gridDim.x) f(item);
+			at += at < 0 ? (int) blockIdx.x + 1 : (int) gridDim.x;
+			while (at < a.total_bricks && skip(at)) at += (int) gridDim.x;
 		}
+		return at < a.total_bricks;
 	};
 
 	if (!a.skin) {
@@ -394,38 +484,59 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch_step(StepArgs a) {
 		const brick::SmemLayout L = brick::layout(a.pc.s_cap, true, hit_words(kCap));
 		brick::load_params(smem, L, a.pp, a.pc.ns);
 		__syncthreads();
-		for_bricks(2, [&](int item) {
-			const BatchBox& B = a.boxes[box_of(item)];
+		for (int item = -1; next_brick(item, [](int) { return false; });) {
+			const BatchBox& B = a.boxes[a.brick_box[item]];
 			brick::pairs<kSingle, kLjIsRc, hit_words(kCap)>(a.pc, B.bx, item - B.brick0, item, smem, a.dst.rx, a.dst.ry,
-			                                            a.dst.rz, a.dst.cid, a.cstart, a.dst.fx, a.dst.fy, a.dst.fz,
-			                                            a.partials, a.status);
+			                                                a.dst.rz, a.dst.cid, a.cstart, a.dst.fx, a.dst.fy, a.dst.fz,
+			                                                a.partials, a.status);
 			__syncthreads();
-		});
+		}
 	} else {
-		// ---- B1: candidate lists of the boxes that were re-binned -----------------------------
-		for_bricks(2, [&](int item) {
-			const int b = box_of(item);
-			if (!a.box_flag[b]) return;
-			const BatchBox& B = a.boxes[b];
-			brick::build_lists(B.bx, item - B.brick0, a.build_cap, smem, a.src.rx, a.src.ry, a.src.rz, a.cstart, a.lists,
-			                   item);
+		// ---- B1: the flagged boxes, one CTA each ----------------------------------------------
+		const int nflagged = (int) *(volatile unsigned*) (a.bar + 4);
+		for (;;) {
 			__syncthreads();
-		});
-		if (!grid_barrier(a.bar, a.status, a.timeout_ns, &s_flag)) return;
-		// ---- B2: list evaluation of every brick -----------------------------------------------
+			if (threadIdx.x == 0) s_item = nflagged ? (int) atomicAdd(a.bar + 3, 1u) : 0;
+			__syncthreads();
+			const int job = s_item;
+			if (job >= nflagged) break;
+			const int b = a.rebuild[job];
+			rebuild_box(a, a.boxes[b], b, smem);
+		}
+		// ---- B2: list evaluation: the bricks of the other boxes, then, with their list builds, those of the
+		// flagged ones by static stride
 		const brick::SmemLayout L = brick::layout(a.lc.s_cap, kFP64);
-		brick::load_params(smem, L, a.pp, a.lc.ns);
-		if (threadIdx.x == 0)
-			reinterpret_cast<float4*>(smem + L.hi)[a.lc.s_cap] =
-			    make_float4(1e15f, 1e15f, 1e15f, __uint_as_float((256u << 18) | (256u << 9) | 256u));
 		__syncthreads();
-		for_bricks(3, [&](int item) {
-			const BatchBox& B = a.boxes[box_of(item)];
+		brick::load_params(smem, L, a.pp, a.lc.ns);
+		auto flagged = [&](int item) { return *(volatile int*) (a.box_flag + a.brick_box[item]) != 0; };
+		bool second = false;
+		int item = -1;
+		for (;;) {
+			if (!second && !next_brick(item, flagged)) {
+				if (nflagged == 0) break;
+				second = true;
+				item = -1;
+			}
+			if (second) {
+				do item += item < 0 ? (int) blockIdx.x + 1 : (int) gridDim.x;
+				while (item < a.total_bricks && !flagged(item));
+				if (item >= a.total_bricks) break;
+			}
+			const int b = a.brick_box[item];
+			const BatchBox& B = a.boxes[b];
+			if (second) {
+				__syncthreads();
+				if (!await_box(a, b, &s_flag)) return;
+				brick::build_lists(B.bx, item - B.brick0, a.build_cap, smem, a.src.rx, a.src.ry, a.src.rz, a.cstart, a.lists,
+				                   item);
+				__syncthreads();
+				brick::load_params(smem, L, a.pp, a.lc.ns);   // the build's staging overwrote them
+			}
+			__syncthreads();
 			brick::list_pairs<kFP64, kSingle, kLjIsRc, false>(a.lc, B.bx, item - B.brick0, item, smem, a.src.rx, a.src.ry,
 			                                           a.src.rz, a.src.cid, a.cstart, a.src.fx, a.src.fy, a.src.fz,
-			                                           a.partials, a.status, a.lists, brick::Kick{});
-			__syncthreads();
-		});
+			                                           a.partials, a.status, a.lists, a.close);
+		}
 	}
 	if (!grid_barrier(a.bar, a.status, a.timeout_ns, &s_flag)) return;
 
@@ -433,6 +544,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch_step(StepArgs a) {
 	if (blockIdx.x == 0 && threadIdx.x == 0) {
 		a.bar[2] = 0u;   // queues are idle until the next launch
 		a.bar[3] = 0u;
+		a.bar[4] = 0u;
 		if (a.skin) *a.valid = 1;
 	}
 	for_my_boxes(a, [&](int b) { finish_box(a, a.boxes[b], b); });
@@ -521,7 +633,6 @@ struct Batch {
 	int64_t ntotal = 0;
 	int total_cells = 0, total_bricks = 0;
 	std::vector<BatchBox> h_boxes;
-	std::vector<int32_t> h_brick0;
 	std::vector<int32_t> h_order;
 	std::string err;
 	Particles buf[2]{};
@@ -537,7 +648,7 @@ struct Batch {
 	unsigned* bar = nullptr;
 	PairParams* d_pp = nullptr;
 	BatchBox* d_boxes = nullptr;
-	int32_t* d_brick0 = nullptr;
+	int32_t* d_brick_box = nullptr;   // box of each brick
 	int32_t* d_order = nullptr;
 	double* stage = nullptr;
 	size_t stage_bytes = 0;
@@ -559,6 +670,7 @@ struct Batch {
 	unsigned short* nbr_count = nullptr;
 	double* r_ref = nullptr;
 	int* box_flag = nullptr;
+	int32_t* rebuild = nullptr;   // the boxes to be rebuilt in a step
 	int* valid = nullptr;
 	unsigned char* kind = nullptr;
 	unsigned long long* builds = nullptr;
@@ -622,7 +734,7 @@ int check_status(Batch* b) {
 	B_CUDA(cudaMemsetAsync(b->status, 0, sizeof(int), b->stream));
 	if (st & kStatusTimeout) {
 		// barrier words may be left mid-count: start them again
-		B_CUDA(cudaMemsetAsync(b->bar, 0, sizeof(unsigned) * 4, b->stream));
+		B_CUDA(cudaMemsetAsync(b->bar, 0, sizeof(unsigned) * 8, b->stream));
 		B_CUDA(cudaStreamSynchronize(b->stream));
 		b->prepared = false;
 		return bfail(b, MDGPU_ERR_TIMEOUT, "a grid-barrier wait of the batched step kernel ran out");
@@ -679,7 +791,7 @@ StepArgs args(Batch* b, const Launch& L, int src, int integrate, double dt, doub
 	StepArgs a{};
 	a.pc = L.pc;
 	a.boxes = b->d_boxes;
-	a.brick0 = b->d_brick0;
+	a.brick_box = b->d_brick_box;
 	a.order = b->d_order;
 	a.nboxes = b->nboxes;
 	a.total_bricks = b->total_bricks;
@@ -714,9 +826,21 @@ StepArgs args(Batch* b, const Launch& L, int src, int integrate, double dt, doub
 		a.lists.sentinel = L.lc.s_cap;
 		a.lists.kind = b->kind;
 		a.box_flag = b->box_flag;
+		a.rebuild = b->rebuild;
 		a.valid = b->valid;
 		a.build_cap = L.build_cap;
 		a.lc = L.lc;
+		if (integrate) {
+			a.close.mode = 2;
+			a.close.dt = dt;
+			for (int k = 0; k < b->sp.n; k++) {
+				a.close.post[k] = a.kick.post[k];
+				a.close.mass[k] = a.kick.mass[k];
+			}
+			a.close.vx = a.src.vx;
+			a.close.vy = a.src.vy;
+			a.close.vz = a.src.vz;
+		}
 	}
 	return a;
 }
@@ -797,7 +921,6 @@ int box_table(Batch* b) {
 	const int nboxes = b->nboxes;
 	const double grid_rc = b->rc + b->skin;
 	b->h_boxes.assign(nboxes, BatchBox{});
-	b->h_brick0.assign(nboxes + 1, 0);
 	b->max_bin_bytes = 0;
 	int64_t poff = 0, coff = 0, brick0 = 0;
 	for (int k = 0; k < nboxes; k++) {
@@ -817,7 +940,6 @@ int box_table(Batch* b) {
 		B.poff = poff;
 		B.n = (int32_t) b->h_count[k];
 		B.brick0 = (int32_t) brick0;
-		b->h_brick0[k] = (int32_t) brick0;
 		b->max_bin_bytes = std::max(b->max_bin_bytes, bin_bytes(b->h_count[k], g.ncells));
 		poff += b->h_count[k];
 		coff += g.ncells;
@@ -825,7 +947,6 @@ int box_table(Batch* b) {
 		if (poff >= (1LL << 28) || coff >= (1LL << 30) || brick0 >= (1LL << 30))
 			return bfail(b, MDGPU_ERR_CAPACITY, "the batch exceeds 2^28 molecules or 2^30 cells/bricks");
 	}
-	b->h_brick0[nboxes] = (int32_t) brick0;
 	b->ntotal = poff;
 	b->total_cells = (int) coff;
 	b->total_bricks = (int) brick0;
@@ -838,12 +959,12 @@ int box_table(Batch* b) {
 
 // Device copies of the box table and the buffers sized by it (again after a change of the skin).
 int upload_table(Batch* b) {
-	void* old[] = {b->cstart, b->partials, b->d_boxes, b->d_brick0, b->d_order, b->kind};
+	void* old[] = {b->cstart, b->partials, b->d_boxes, b->d_brick_box, b->d_order, b->kind};
 	for (void* x : old) cudaFree(x);
 	b->cstart = nullptr;
 	b->partials = nullptr;
 	b->d_boxes = nullptr;
-	b->d_brick0 = nullptr;
+	b->d_brick_box = nullptr;
 	b->d_order = nullptr;
 	b->kind = nullptr;
 	for (auto& g : b->graphs) cudaGraphExecDestroy(g.exec);
@@ -854,8 +975,13 @@ int upload_table(Batch* b) {
 	B_CUDA(cudaMalloc(&b->kind, b->total_bricks));
 	B_CUDA(cudaMalloc(&b->d_boxes, sizeof(BatchBox) * nboxes));
 	B_CUDA(cudaMemcpy(b->d_boxes, b->h_boxes.data(), sizeof(BatchBox) * nboxes, cudaMemcpyHostToDevice));
-	B_CUDA(cudaMalloc(&b->d_brick0, sizeof(int32_t) * (nboxes + 1)));
-	B_CUDA(cudaMemcpy(b->d_brick0, b->h_brick0.data(), sizeof(int32_t) * (nboxes + 1), cudaMemcpyHostToDevice));
+	std::vector<int32_t> brick_box((size_t) b->total_bricks);
+	for (int k = 0; k < nboxes; k++) {
+		const BatchBox& B = b->h_boxes[k];
+		std::fill_n(brick_box.begin() + B.brick0, B.bx.nb[0] * B.bx.nb[1] * B.bx.nb[2], k);
+	}
+	B_CUDA(cudaMalloc(&b->d_brick_box, sizeof(int32_t) * b->total_bricks));
+	B_CUDA(cudaMemcpy(b->d_brick_box, brick_box.data(), sizeof(int32_t) * b->total_bricks, cudaMemcpyHostToDevice));
 	B_CUDA(cudaMalloc(&b->d_order, sizeof(int32_t) * nboxes));
 	B_CUDA(cudaMemcpy(b->d_order, b->h_order.data(), sizeof(int32_t) * nboxes, cudaMemcpyHostToDevice));
 	return MDGPU_OK;
@@ -923,8 +1049,8 @@ int mdgpu_batch_create(mdgpu_batch** out, int32_t nboxes, const double* lengths,
 	B_CUDA(cudaMalloc(&b->status, sizeof(int)));
 	B_CUDA(cudaMemset(b->status, 0, sizeof(int)));
 	B_CUDA(cudaMallocHost(&b->h_status, sizeof(int)));
-	B_CUDA(cudaMalloc(&b->bar, sizeof(unsigned) * 4));
-	B_CUDA(cudaMemset(b->bar, 0, sizeof(unsigned) * 4));
+	B_CUDA(cudaMalloc(&b->bar, sizeof(unsigned) * 8));
+	B_CUDA(cudaMemset(b->bar, 0, sizeof(unsigned) * 8));
 	PairParams hp = pair_params(b->sp, b->rc, b->rc_lj);
 	B_CUDA(cudaMalloc(&b->d_pp, sizeof(PairParams)));
 	B_CUDA(cudaMemcpy(b->d_pp, &hp, sizeof(PairParams), cudaMemcpyHostToDevice));
@@ -951,7 +1077,7 @@ int mdgpu_batch_destroy(mdgpu_batch* h) {
 	for (int k = 0; k < 2; k++) free_particles(b->buf[k]);
 	if (b->backup_alloc) free_particles(b->backup);
 	void* bufs[] = {b->cstart, b->partials, b->records, b->prep, b->status, b->bar, b->d_pp, b->d_boxes,
-	                b->d_brick0, b->d_order, b->stage, b->nbr, b->nbr_count, b->r_ref, b->box_flag,
+	                b->d_brick_box, b->d_order, b->stage, b->nbr, b->nbr_count, b->r_ref, b->box_flag, b->rebuild,
 	                b->valid, b->kind, b->builds, b->d_bid, b->d_len};
 	for (void* x : bufs) cudaFree(x);
 	if (b->h_status) cudaFreeHost(b->h_status);
@@ -1189,11 +1315,12 @@ int mdgpu_batch_set_skin(mdgpu_batch* h, double skin) {
 		return st;
 	}
 	if (b->max_bin_bytes > 110 * 1024) b->tiles.ctas = 1;
-	void* lists[] = {b->nbr, b->nbr_count, b->r_ref, b->box_flag, b->valid, b->builds};
+	void* lists[] = {b->nbr, b->nbr_count, b->r_ref, b->box_flag, b->rebuild, b->valid, b->builds};
 	for (void* x : lists) cudaFree(x);
 	b->nbr = b->nbr_count = nullptr;
 	b->r_ref = nullptr;
 	b->box_flag = b->valid = nullptr;
+	b->rebuild = nullptr;
 	b->builds = nullptr;
 	if (skin > 0.0) {
 		// list capacity from the densest box (x 1.5 for local fluctuations)
@@ -1208,6 +1335,7 @@ int mdgpu_batch_set_skin(mdgpu_batch* h, double skin) {
 		B_CUDA(cudaMalloc(&b->nbr_count, sizeof(unsigned short) * b->ntotal));
 		B_CUDA(cudaMalloc(&b->r_ref, sizeof(double) * 3 * b->ntotal));
 		B_CUDA(cudaMalloc(&b->box_flag, sizeof(int) * b->nboxes));
+		B_CUDA(cudaMalloc(&b->rebuild, sizeof(int32_t) * b->nboxes));
 		B_CUDA(cudaMalloc(&b->valid, sizeof(int)));
 		B_CUDA(cudaMemset(b->valid, 0, sizeof(int)));
 		B_CUDA(cudaMalloc(&b->builds, sizeof(unsigned long long)));
