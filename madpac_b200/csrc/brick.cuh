@@ -66,7 +66,6 @@ struct Box {
 	float rc2_h;          // rc^2 + margin covering half-precision rounding (packed filter)
 	float lo_step[3];     // fixed-point step of the lo parts: 2^(k-32) for the binade [2^k, 2^(k+1))
 	float lo_inv[3];      // 1 / lo_step
-	float lo_c[3];        // -(2^23 + 256) * lo_step (decoding constant)
 };
 
 struct SmemLayout {
@@ -81,20 +80,20 @@ struct __align__(16) HalfPair {
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
-// Shared memory of the list kernels (they read their lists from global memory): the hi/lo positions
-// with the far-away sentinel slot past the capacity, and in the FP64 form the double images.
-// With words > 0 that of the traversal (pairs, fp64): the packed half-precision copy for its filter, the
-// double images, the component ids and `words` hit words per lane.
+// Shared memory of the list kernels (they read their lists from global memory): in the FP32 form the hi/lo
+// positions with the far-away sentinel slot past the capacity, in the FP64 form the double images and the
+// component ids. With words > 0 that of the traversal (pairs, fp64), which adds the packed half-precision
+// copy for its filter and `words` hit words per lane.
 __host__ __device__ inline SmemLayout layout(int s_cap, bool fp64, int words = 0) {
 	SmemLayout L;
 	size_t o = 0;
 	const bool traverse = words > 0;
 	L.hi = o;
-	if (!traverse) o = align16(o + sizeof(float4) * (s_cap + 1));
+	if (!fp64) o = align16(o + sizeof(float4) * (s_cap + 1));
 	L.img = o;
 	if (fp64) o = align16(o + sizeof(double) * 3 * s_cap);
 	L.comp = o;
-	if (traverse) o = align16(o + s_cap);
+	if (fp64) o = align16(o + s_cap);
 	L.h16 = o;
 	if (traverse) o = align16(o + sizeof(HalfPair) * (s_cap / 2 + 20));  // 16-slot blocks may read past the end
 	L.cstart = o;
@@ -138,7 +137,6 @@ inline void init_box(Box& b, const Grid& g, double rc, int32_t coff, double drif
 		b.frame_c[d] = (float) (1.5 * pk);
 		b.lo_step[d] = (float) std::ldexp(pk, -32);
 		b.lo_inv[d] = (float) std::ldexp(1.0 / pk, 32);
-		b.lo_c[d] = -8388864.0f * b.lo_step[d];
 	}
 	// half-precision filter: coordinates within +-2 cells of the brick centre; each rounding is at
 	// most half an ulp of the largest coordinate, plus the rounding of the packed r^2 itself
@@ -187,7 +185,7 @@ __device__ __forceinline__ void load_params(unsigned char* smem, const SmemLayou
 struct Smem {
 	float4* hi;
 	double* img;
-	unsigned char* comp;  // component ids (traversal)
+	unsigned char* comp;  // component ids (FP64)
 	HalfPair* h16;
 	__half* h;
 	int* cs;              // staged slot of each staged cell (65)
@@ -242,17 +240,15 @@ __device__ __forceinline__ unsigned pack_lo(float lx, float ly, float lz, int ci
 	return w;
 }
 
-// lo = fma(2^23 + field, step, -(2^23 + 256) * step): exact in one FMA (power-of-two step).
-__device__ __forceinline__ float3 unpack_lo(unsigned w, const Box& bx) {
-	return make_float3(fmaf(__uint_as_float(0x4B000000u | (w & 511u)), bx.lo_step[0], bx.lo_c[0]),
-	                   fmaf(__uint_as_float(0x4B000000u | ((w >> 9) & 511u)), bx.lo_step[1], bx.lo_c[1]),
-	                   fmaf(__uint_as_float(0x4B000000u | ((w >> 18) & 511u)), bx.lo_step[2], bx.lo_c[2]));
-}
-
 __device__ __forceinline__ int unpack_cid(unsigned w) { return (int) ((w >> 27) & 7u); }
 
-// What a staging stores: the list kernels' hi/lo frame positions, with the double images in the FP64
-// form, or the traversal's half-precision copy, double images and component ids.
+// Component of a staged slot (FP64), always within the pair table: idle lanes and the padding of lists also
+// look at slots that nothing was staged to.
+__device__ __forceinline__ int component(const Smem& S, int slot) { return S.comp[slot] & (kMaxSpecies - 1); }
+static_assert((kMaxSpecies & (kMaxSpecies - 1)) == 0, "a power of two");
+
+// What a staging stores: the list kernels' hi/lo frame positions (FP32) or double images and component ids
+// (FP64), or the traversal's half-precision copy, double images and component ids.
 enum Staging { kStageList32, kStageList64, kStageTraverse };
 
 // Stages a molecule at double position (x, y, z), component q, at slot slot_s, with its cell's frame
@@ -261,21 +257,23 @@ enum Staging { kStageList32, kStageList64, kStageTraverse };
 template <Staging kMode>
 __device__ __forceinline__ void stage_at(const Box& bx, const Smem& S, int slot_s, double x, double y, double z, int q,
                                          double kx, double ky, double kz, double shx, double shy, double shz) {
-	const double Xd = __dadd_rn(x, kx), Yd = __dadd_rn(y, ky), Zd = __dadd_rn(z, kz);
-	const float X = __double2float_rn(Xd), Y = __double2float_rn(Yd), Z = __double2float_rn(Zd);
-	if (kMode == kStageTraverse) {
-		// half-precision copy relative to the brick centre (slot pairs share one HalfPair)
-		__half* hp = S.h + 8 * (slot_s >> 1) + (slot_s & 1);
-		hp[0] = __float2half_rn(X);
-		hp[2] = __float2half_rn(Y);
-		hp[4] = __float2half_rn(Z);
-		S.comp[slot_s] = (unsigned char) q;
-	} else {
-		const unsigned w = pack_lo(__double2float_rn(Xd - (double) X), __double2float_rn(Yd - (double) Y),
-		                           __double2float_rn(Zd - (double) Z), q, bx);
-		S.hi[slot_s] = make_float4(X, Y, Z, __uint_as_float(w));
+	if (kMode != kStageList64) {
+		const double Xd = __dadd_rn(x, kx), Yd = __dadd_rn(y, ky), Zd = __dadd_rn(z, kz);
+		const float X = __double2float_rn(Xd), Y = __double2float_rn(Yd), Z = __double2float_rn(Zd);
+		if (kMode == kStageTraverse) {
+			// half-precision copy relative to the brick centre (slot pairs share one HalfPair)
+			__half* hp = S.h + 8 * (slot_s >> 1) + (slot_s & 1);
+			hp[0] = __float2half_rn(X);
+			hp[2] = __float2half_rn(Y);
+			hp[4] = __float2half_rn(Z);
+		} else {
+			const unsigned w = pack_lo(__double2float_rn(Xd - (double) X), __double2float_rn(Yd - (double) Y),
+			                           __double2float_rn(Zd - (double) Z), q, bx);
+			S.hi[slot_s] = make_float4(X, Y, Z, __uint_as_float(w));
+		}
 	}
 	if (kMode != kStageList32) {
+		S.comp[slot_s] = (unsigned char) q;
 		S.img[3 * slot_s] = __dadd_rn(x, shx);
 		S.img[3 * slot_s + 1] = __dadd_rn(y, shy);
 		S.img[3 * slot_s + 2] = __dadd_rn(z, shz);
@@ -545,9 +543,9 @@ struct Sums64 {
 // PotForceLJ's (molecules/potforce.h:41-53), contracted: with s6 = (sig2/r^2)^3, m = s6^2 - s6 and
 // e = s6^2 + m the sums are F += (e/r^2) d, U += m, W += e (the virial term d.f is e, as f = (e/r^2) d):
 // 22 FP64 instructions against 38 and a division in the reference's order. A zero distance (its high
-// word is zero) sets `same` and leaves non-finite sums.
+// word is zero) sets `same` and leaves non-finite sums. Returns the squared distance.
 template <bool kSingle, bool kLjIsRc>
-__device__ __forceinline__ void lj64(double d0, double d1, double d2, bool v, double rc2, double rclj2, double eps24,
+__device__ __forceinline__ double lj64(double d0, double d1, double d2, bool v, double rc2, double rclj2, double eps24,
                                      double sig2, double shift6, Sums64& s, bool& same) {
 	const double dd = __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
 	const bool in = v && dd < rc2;
@@ -571,6 +569,7 @@ __device__ __forceinline__ void lj64(double d0, double d1, double d2, bool v, do
 	s.y = fma(fac, d1, s.y);
 	s.z = fma(fac, d2, s.z);
 	s.w += e;
+	return dd;
 }
 
 // The pair parameters of a single-species molecule's sums.
@@ -692,7 +691,7 @@ __device__ __forceinline__ void pairs(const Const& p, const Box& bx, int brick, 
 			const int slot_i = S.cs[oc] + (act ? t - s_own[w] : 0);
 			const int gi = S.gst[oc] + (act ? t - s_own[w] : 0);
 			const double xi = S.img[3 * slot_i], yi = S.img[3 * slot_i + 1], zi = S.img[3 * slot_i + 2];
-			const int ti = kSingle ? 0 : S.comp[slot_i];
+			const int ti = kSingle ? 0 : component(S, slot_i);
 			Sums64 s64{0.0, 0.0, 0.0, 0.0, 0.0, 0, 0};
 			int cnt = 0, hits = 0;   // words and hits collected
 
@@ -715,7 +714,7 @@ __device__ __forceinline__ void pairs(const Const& p, const Box& bx, int brick, 
 					v = v && j != slot_i;
 					double e24 = 0.0, sg2 = sig2_d, sh6 = 0.0;
 					if (!kSingle) {
-						const int pk = ti * ns + S.comp[j];
+						const int pk = ti * ns + component(S, j);
 						e24 = S.pd[pk];
 						sg2 = S.pd[KK + pk];
 						sh6 = S.pd[2 * KK + pk];
@@ -1264,15 +1263,15 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 	if (act)
 		while (w < 7 && s_own[w + 1] <= t) w++;
 	const int slot_i = act ? S.cs[s_ocell[w]] + (t - s_own[w]) : 0;
-	const float4 hi_i = S.hi[slot_i];
-	const float3 lo_i = unpack_lo(__float_as_uint(hi_i.w), bx);
+	float4 hi_i = make_float4(0.f, 0.f, 0.f, 0.f);
 	double xi = 0, yi = 0, zi = 0;
 	if (kFP64) {
 		xi = S.img[3 * slot_i];
 		yi = S.img[3 * slot_i + 1];
 		zi = S.img[3 * slot_i + 2];
 	}
-	const int ti = unpack_cid(__float_as_uint(hi_i.w));
+	if (!kFP64) hi_i = S.hi[slot_i];
+	const int ti = kSingle ? 0 : kFP64 ? component(S, slot_i) : unpack_cid(__float_as_uint(hi_i.w));
 	const int gi = act ? S.gst[s_ocell[w]] + (t - s_own[w]) : S.gst[s_ocell[0]];
 	int cnt = act ? (int) lists.count[gi] : 0;
 	const bool ovf = cnt == kListOverflow;
@@ -1330,19 +1329,15 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 				const bool v = kk < cnt && raw < (unsigned) p.s_cap;
 				double e24 = 0.0, sg2 = S.pd[KK], sh6 = 0.0;
 				if (!kSingle) {
-					const int pk = ti * ns + unpack_cid(__float_as_uint(S.hi[j].w));
+					const int pk = ti * ns + component(S, j);
 					e24 = S.pd[pk];
 					sg2 = S.pd[KK + pk];
 					sh6 = S.pd[2 * KK + pk];
 				}
-				lj64<kSingle, kLjIsRc>(__dsub_rn(xi, S.img[3 * j]), __dsub_rn(yi, S.img[3 * j + 1]),
-				              __dsub_rn(zi, S.img[3 * j + 2]), v, p.rc2, p.rclj2, e24, sg2, sh6, s64, same);
-				if (kPrune) {
-					// the prune test on the staged hi parts (rp2f covers the lo parts)
-					const float4 hj = S.hi[j];
-					const float d0 = hi_i.x - hj.x, d1 = hi_i.y - hj.y, d2 = hi_i.z - hj.z;
-					keep((unsigned) j, kk < cnt && fmaf(d0, d0, fmaf(d1, d1, d2 * d2)) < po.rp2f);
-				}
+				const double dd =
+				    lj64<kSingle, kLjIsRc>(__dsub_rn(xi, S.img[3 * j]), __dsub_rn(yi, S.img[3 * j + 1]),
+				                           __dsub_rn(zi, S.img[3 * j + 2]), v, p.rc2, p.rclj2, e24, sg2, sh6, s64, same);
+				if (kPrune) keep((unsigned) j, v && dd < (double) po.rp2f);
 			}
 			if (kPrune && kept - done >= 8) flush();
 		}
@@ -1536,7 +1531,7 @@ __device__ __forceinline__ void list_pairs(const Const& p, const Box& bx, int br
 	const int ns = p.ns;
 	__shared__ int s_own[kWarps + 1], s_ocell[kWarps];
 	// sentinel slot: far from every molecule (entries past a list's end point to it)
-	if (tid == 0) S.hi[p.s_cap] = make_float4(1e15f, 1e15f, 1e15f, __uint_as_float((256u << 18) | (256u << 9) | 256u));
+	if (!kFP64 && tid == 0) S.hi[p.s_cap] = make_float4(1e15f, 1e15f, 1e15f, __uint_as_float((256u << 18) | (256u << 9) | 256u));
 	const bool staged = stage_cells<kFP64, kWide>(p, bx, brick, S, rx, ry, rz, cid, cstart, s_own, s_ocell);
 	const int n_own = s_own[kWarps];
 	double U = 0.0, W = 0.0, NP = 0.0, MV = 0.0;

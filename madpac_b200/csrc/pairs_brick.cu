@@ -92,11 +92,11 @@ __global__ void __launch_bounds__(brick::kThreads, 3)
 	}
 }
 
-#ifndef MDGPU_LIST_MINB
-#define MDGPU_LIST_MINB 3
-#endif
-// Resident CTAs per SM of the FP32 list kernel (registers and shared memory are sized for it).
-constexpr int kListMinBlocks = MDGPU_LIST_MINB;
+// Resident CTAs per SM of the list kernels (registers and shared memory are sized for it). The FP64 form
+// stages only images and component ids (25 bytes per molecule, 40 with the FP32 form's split positions), so
+// three CTAs hold its regions too: 400,009 molecules, us per step, one species 190 at the start, 132 with two
+// CTAs, 113 with three; two species 204, 142, 143; 1,048,576 with pruned lists 295 with two, 254 with three.
+constexpr int kListMinBlocks = 3;
 
 // The list evaluation of a step. With pruned lists (lists.pst set) it comes in two variants, launched
 // one after the other in every step: kPrune runs in the steps that prune (the lists were built in
@@ -105,7 +105,7 @@ constexpr int kListMinBlocks = MDGPU_LIST_MINB;
 // steps and reads the inner lists. Both decide from values that no CTA of their launch changes (not
 // from the rebuild flag, which the fused kick of this step may set for the next one).
 template <bool kFP64, bool kSingle, bool kLjIsRc, bool kPrune = false>
-__global__ void __launch_bounds__(brick::kThreads, kFP64 ? 2 : kListMinBlocks)
+__global__ void __launch_bounds__(brick::kThreads, kListMinBlocks)
     k_pairs_list(brick::Const p, brick::Box bx, const double* __restrict__ rx, const double* __restrict__ ry,
                  const double* __restrict__ rz, const int32_t* __restrict__ cid,
                  const int32_t* __restrict__ cstart, const PairParams* __restrict__ pp,
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(brick::kThreads, 2)
 		pf[brick::KK + k] = (float) pp->sig2[k];
 		pf[2 * brick::KK + k] = (float) pp->shift6[k];
 	}
-	if (lane == 0)
+	if (!kFP64 && lane == 0)
 		reinterpret_cast<float4*>(ws + L.hi)[brick::kSparseCap] =
 		    make_float4(1e15f, 1e15f, 1e15f, __uint_as_float((256u << 18) | (256u << 9) | 256u));
 	if (threadIdx.x == 0) brick::drift_slot() = 0u;
@@ -249,7 +249,7 @@ struct Plan {
 	int nbricks;
 };
 
-// kind 0: plain traversal, 2: list evaluation of the skin mode (two CTAs per SM).
+// kind 0: plain traversal, 2: list evaluation of the skin mode.
 Plan plan(Context* c, const Grid& g, double filter_radius, int kind) {
 	const bool fp64 = kind == 0 || c->precision == MDGPU_FP64;   // the traversal evaluates both modes in FP64
 	Plan P;
@@ -263,7 +263,7 @@ Plan plan(Context* c, const Grid& g, double filter_radius, int kind) {
 		const double region = 64.0 * rho * g.cell_length[0] * g.cell_length[1] * g.cell_length[2];
 		if (1.3 * region + 64.0 <= brick::capacity_for(small, fp64, brick::kHitWords)) budget = small;
 	}
-	if (kind == 2 && !fp64) budget = std::min(budget, (size_t) (224 / kListMinBlocks - 2) * 1024);
+	if (kind == 2) budget = std::min(budget, (size_t) (224 / kListMinBlocks - 2) * 1024);
 	if (kind == 2 && pruning(c)) budget -= brick::kPruneRingBytes;   // the prune variant's ring
 	if (budget > (size_t) max_optin) budget = (size_t) max_optin;
 	const int words = kind == 2 ? 0 : brick::kHitWords;
@@ -422,9 +422,9 @@ cudaError_t launch_pairs_skin(Context* c, int kick_mode, double dt, double* reco
 		inner.count = c->nbr_in_count;
 		po.nbr = c->nbr_in;
 		po.count = c->nbr_in_count;
-		// the FP64 form tests the staged hi parts only: the lo parts (at most 256 steps each way
-		// per coordinate, plus half a step of quantisation) move the distance by at most
-		// sqrt(3) * 513 steps; the float arithmetic by a few 1e-7 of it
+		// the FP32 form's split positions: the lo parts (at most 256 steps each way per coordinate, plus
+		// half a step of quantisation) move the distance by at most sqrt(3) * 513 steps; the float
+		// arithmetic by a few 1e-7 of it
 		const double lo = 520.0 * std::max(P.bx.lo_step[0], std::max(P.bx.lo_step[1], P.bx.lo_step[2]));
 		const double rp = c->rc + c->prune + 1.7320508075688772 * lo;
 		const double rp2 = rp * rp * (1.0 + 2e-6);
