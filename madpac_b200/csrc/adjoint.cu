@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "md_internal.h"
+#include "pair_common.cuh"
 #include "reduce.cuh"
 
 namespace mdgpu {
@@ -36,23 +37,31 @@ constexpr int kAdjList = 16;   // accepted partners a lane lists before evaluati
 // kMaxSpecies with the per-pair sums in a KK-entry array (local memory).
 template <bool kMixed, int NP>
 __global__ void __launch_bounds__(kReduceBlock) k_adjoint(int64_t n, Particles p, const int32_t* __restrict__ start,
-                                                         Grid g, const PairParams* __restrict__ pp, double rclj,
+                                                         Grid g, const PairParams* __restrict__ pp,
                                                          const double* __restrict__ gfx, const double* __restrict__ gfy,
                                                          const double* __restrict__ gfz, double gU,
                                                          double* __restrict__ ox, double* __restrict__ oy,
                                                          double* __restrict__ oz, double* __restrict__ pgrad) {
-	__shared__ double s_e24[KK], s_s2[KK], s_sh[KK];
+	// per component pair: eps24, sig2, their reciprocals, and the shift's terms c6 and c6'
+	__shared__ double s_e24[KK], s_s2[KK], s_ie[KK], s_is[KK], s_c6[KK], s_c6s[KK];
 	__shared__ double s_acc[kReduceBlock / 32][2 * KK];   // per-warp partials of the parameter terms
 	__shared__ int32_t s_aj[kAdjList * kReduceBlock];      // each lane's accepted partners (column per lane)
 	__shared__ uint8_t s_ai[kAdjList * kReduceBlock];      // and their periodic images (27 codes)
 	const int ns = pp->ns;
 	for (int k = threadIdx.x; k < KK; k += blockDim.x) {
-		s_e24[k] = k < ns * ns ? pp->eps24[k] : 0.0;
-		s_s2[k] = k < ns * ns ? pp->sig2[k] : 0.0;
-		s_sh[k] = k < ns * ns ? pp->shift6[k] : 0.0;
+		const bool in = k < ns * ns;
+		const double e24 = in ? pp->eps24[k] : 0.0, sg2 = in ? pp->sig2[k] : 0.0;
+		const bool shf = in && pp->shift6[k] != 0.0;
+		const double sr6 = sg2 * sg2 * sg2 / (pp->rclj2 * pp->rclj2 * pp->rclj2);
+		s_e24[k] = e24;
+		s_s2[k] = sg2;
+		s_ie[k] = in ? 1.0 / e24 : 0.0;
+		s_is[k] = in ? 1.0 / sg2 : 0.0;
+		s_c6[k] = shf ? sr6 - sr6 * sr6 : 0.0;
+		s_c6s[k] = shf ? 3.0 * sr6 - 6.0 * sr6 * sr6 : 0.0;
 	}
 	__syncthreads();
-	const double rc2 = pp->rc2, rclj2 = pp->rclj2, rclj6 = rclj2 * rclj2 * rclj2;
+	const double cut2 = fmin(pp->rc2, pp->rclj2), gU6 = gU / 6.0;
 	// kAdjLanes consecutive lanes per molecule, each taking every kAdjLanes-th candidate of a cell
 	const int64_t i = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / kAdjLanes;
 	const int sub = threadIdx.x % kAdjLanes;
@@ -94,17 +103,13 @@ __global__ void __launch_bounds__(kReduceBlock) k_adjoint(int64_t n, Particles p
 			const double d0 = xi - (p.rx[j] + sx), d1 = yi - (p.ry[j] + sy), d2 = zi - (p.rz[j] + sz);
 			const double q = d0 * d0 + d1 * d1 + d2 * d2;
 			const int pk = ti * ns + p.cid[j];
-			const double e24 = s_e24[pk], sg2 = s_s2[pk];
 			const double w0 = wix - gfx[j], w1 = wiy - gfy[j], w2 = wiz - gfz[j];
-			const bool shf = s_sh[pk] != 0.0;
-			const double sr6 = sg2 * sg2 * sg2 / rclj6;
-			const double c6 = shf ? sr6 - sr6 * sr6 : 0.0;
-			const double c6s = shf ? 3.0 * sr6 - 6.0 * sr6 * sr6 : 0.0;
+			const double c6 = s_c6[pk], c6s = s_c6s[pk];
 			if (kMixed) {
 				// FP32 from the FP64 difference vector; FP64 sums
 				const float f0 = (float) d0, f1 = (float) d1, f2 = (float) d2;
 				const float qf = fmaf(f0, f0, fmaf(f1, f1, f2 * f2));
-				const float e24f = (float) e24, sg2f = (float) sg2;
+				const float e24f = (float) s_e24[pk], sg2f = (float) s_s2[pk];
 				const float iq = 1.0f / qf;
 				float s6 = sg2f * iq;
 				s6 = s6 * s6 * s6;
@@ -118,25 +123,27 @@ __global__ void __launch_bounds__(kReduceBlock) k_adjoint(int64_t n, Particles p
 				ax += (double) (fac * v0 + t * f0 - gUf * fac * f0);
 				ay += (double) (fac * v1 + t * f1 - gUf * fac * f1);
 				az += (double) (fac * v2 + t * f2 - gUf * fac * f2);
-				add_param(pk, 0.5 * ((double) (fac * dw / e24f) + gU * ((double) (s12 - s6) + c6) / 6.0),
+				add_param(pk, 0.5 * ((double) (fac * dw / e24f) + gU6 * ((double) (s12 - s6) + c6)),
 				          0.5 * ((double) (e24f * (12.0f * s12 - 3.0f * s6) * iq / sg2f * dw) +
-				                 gU * e24 * ((double) (6.0f * s12 - 3.0f * s6) + c6s) / (6.0 * sg2)));
+				                 gU6 * s_e24[pk] * ((double) (6.0f * s12 - 3.0f * s6) + c6s) * s_is[pk]));
 			} else {
-				const double iq = 1.0 / q;
-				double s6 = sg2 * iq;
+				const double e24 = s_e24[pk];
+				const double iq = rcp64(q);
+				double s6 = s_s2[pk] * iq;
 				s6 = s6 * s6 * s6;
 				const double s12 = s6 * s6;
-				const double fac = e24 * (2.0 * s12 - s6) * iq;
-				const double dfac = e24 * (4.0 * s6 - 14.0 * s12) * iq * iq;
+				const double ei = e24 * iq;
+				const double fac = ei * (2.0 * s12 - s6);
+				const double dfac = ei * iq * (4.0 * s6 - 14.0 * s12);
 				const double dw = d0 * w0 + d1 * w1 + d2 * w2;
 				// J w - gU f
-				ax += fac * w0 + 2.0 * dfac * dw * d0 - gU * fac * d0;
-				ay += fac * w1 + 2.0 * dfac * dw * d1 - gU * fac * d1;
-				az += fac * w2 + 2.0 * dfac * dw * d2 - gU * fac * d2;
+				const double t = 2.0 * dfac * dw - gU * fac;
+				ax += fac * w0 + t * d0;
+				ay += fac * w1 + t * d1;
+				az += fac * w2 + t * d2;
 				// parameter terms (half: the pair is seen from both sides)
-				add_param(pk, 0.5 * (fac * dw / e24 + gU * (s12 - s6 + c6) / 6.0),
-				          0.5 * (e24 * (12.0 * s12 - 3.0 * s6) * iq / sg2 * dw +
-				                 gU * e24 * (6.0 * s12 - 3.0 * s6 + c6s) / (6.0 * sg2)));
+				add_param(pk, 0.5 * (fac * dw * s_ie[pk] + gU6 * (s12 - s6 + c6)),
+				          0.5 * s_is[pk] * (ei * (12.0 * s12 - 3.0 * s6) * dw + gU6 * e24 * (6.0 * s12 - 3.0 * s6 + c6s)));
 			}
 		};
 		auto flush = [&]() {
@@ -182,11 +189,12 @@ __global__ void __launch_bounds__(kReduceBlock) k_adjoint(int64_t n, Particles p
 					const bool shifted = (sx != 0.0) || (sy != 0.0) || (sz != 0.0);
 					const uint8_t img = (uint8_t) ((sx < 0.0 ? 0 : sx > 0.0 ? 2 : 1) + 3 * (sy < 0.0 ? 0 : sy > 0.0 ? 2 : 1) +
 					                               9 * (sz < 0.0 ? 0 : sz > 0.0 ? 2 : 1));
-					for (int j = start[nb] + sub; j < start[nb + 1]; j += kAdjLanes) {
+					const double xs = xi - sx, ys = yi - sy, zs = zi - sz;
+					const int j1 = start[nb + 1];
+					for (int j = start[nb] + sub; j < j1; j += kAdjLanes) {
 						if (j == i && !shifted) continue;
-						const double d0 = xi - (p.rx[j] + sx), d1 = yi - (p.ry[j] + sy), d2 = zi - (p.rz[j] + sz);
-						const double q = d0 * d0 + d1 * d1 + d2 * d2;
-						if (!(q < rc2) || !(q < rclj2)) continue;
+						const double d0 = xs - p.rx[j], d1 = ys - p.ry[j], d2 = zs - p.rz[j];
+						if (!(d0 * d0 + d1 * d1 + d2 * d2 < cut2)) continue;
 						aj[acnt * kReduceBlock] = j;
 						ai[acnt * kReduceBlock] = img;
 						if (++acnt == kAdjList) flush();
@@ -257,7 +265,7 @@ cudaError_t launch_adjoint(Context* c, const double* gfx, const double* gfy, con
 	const int np = c->sp.n * c->sp.n;
 #define MD_ADJ(MX, NPV)                                                                                           \
 	k_adjoint<MX, NPV><<<(unsigned) nb, kReduceBlock, 0, c->stream>>>(c->n, c->p, c->cell_start, c->g, c->d_pp,   \
-	                                                                   c->rc_lj, gfx, gfy, gfz, gU, ox, oy, oz, pgrad)
+	                                                                   gfx, gfy, gfz, gU, ox, oy, oz, pgrad)
 	const bool mixed = c->precision == MDGPU_MIXED;
 	if (np == 1)
 		mixed ? MD_ADJ(true, 1) : MD_ADJ(false, 1);

@@ -519,17 +519,6 @@ static __device__ __noinline__ bool exact_cut(const Smem& S, double rc2, int j, 
 	return dd < rc2;
 }
 
-// 1/x for a positive normal x: the hardware's approximation y (rcp.approx.ftz.f64, about 20 bits) and
-// one step of Chebyshev's third-order iteration, y + y (e + e^2) with e = 1 - x y: e^3 is below 2^-58,
-// so what is left is the last rounding. Three FP64 instructions and no branch; the correctly rounded
-// intrinsic, with its branch for special operands, made the whole FP64 evaluation a fifth slower.
-__device__ __forceinline__ double rcp64(double x) {
-	double y;
-	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-	const double e = fma(-x, y, 1.0);
-	return fma(y, fma(e, e, e), y);
-}
-
 // FP64 sums of one molecule's pairs: force, energy and virial before the pair parameters that the
 // single-species form applies once per molecule (sums64_finish).
 struct Sums64 {
