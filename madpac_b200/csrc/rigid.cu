@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "md_internal.h"
+#include "pair_common.cuh"
 #include "transfer.h"
 #include "reduce.cuh"
 
@@ -228,7 +229,7 @@ __device__ __forceinline__ void cross3(const double a[3], const double b[3], dou
 // torque on the oriented site ejj.
 __device__ void charge_oriented(bool quad, const double dr[3], double dr2, const double ejj[3], double par,
                                 double f[3], double m2[3], double& u) {
-	const double invdr2 = __ddiv_rn(1.0, dr2);
+	const double invdr2 = rcp64(dr2);
 	const double invdr = __dsqrt_rn(invdr2);
 	const double costj = dm_(dot3(ejj, dr), invdr);
 	double pT, fac;
@@ -255,7 +256,7 @@ __device__ void charge_oriented(bool quad, const double dr[3], double dr2, const
 __device__ void two_oriented(int kind, const double dr[3], double dr2, const double eii[3], const double ejj[3],
                              double par, double rffac, double f[3], double m1[3], double m2[3], double& u,
                              double& rf) {
-	const double invdr2 = __ddiv_rn(1., dr2);
+	const double invdr2 = rcp64(dr2);
 	const double invdr1 = __dsqrt_rn(invdr2);
 	const double costi = dm_(dot3(eii, dr), invdr1);
 	const double costj = dm_(dot3(ejj, dr), invdr1);
@@ -351,12 +352,8 @@ struct RigidOut {
 #ifndef MDGPU_RIGID_LIST
 #define MDGPU_RIGID_LIST 32
 #endif
-#ifndef MDGPU_RIGID_DIRECT
-#define MDGPU_RIGID_DIRECT 0
-#endif
-// list entries evaluated as they are accepted instead of through the lane's shared-memory list
-constexpr bool kDirect = MDGPU_RIGID_DIRECT != 0;
 constexpr int kRigidLanes = MDGPU_RIGID_LANES;
+constexpr int kScan = 4;   // list entries of a lane tested at a time
 constexpr int kRigidList = MDGPU_RIGID_LIST;
 static_assert(kRigidLanes == 1 || kRigidLanes == 2 || kRigidLanes == 4 || kRigidLanes == 8, "lanes per molecule");
 
@@ -550,7 +547,7 @@ __global__ void __launch_bounds__(kRigidThreads,
 							const double s2 = __dsub_rn(__dadd_rn(m2, di[si][2]), dj2);
 							const double dr2 =
 							    __dadd_rn(__dadd_rn(__dmul_rn(s0, s0), __dmul_rn(s1, s1)), __dmul_rn(s2, s2));
-							const double invdr2 = __ddiv_rn(1.0, dr2);
+							const double invdr2 = rcp64(dr2);
 							double fac;
 							if (lj_j) {
 								const int pk = (bi + si) * kMaxSiteTotal + bj + sj;
@@ -706,8 +703,7 @@ __global__ void __launch_bounds__(kRigidThreads,
 
 		// candidate j in image img (shift sx, sy, sz): the exact cutoff test of the reference; the
 		// accepted ones go to the lane's list
-		auto consider = [&](int j, uint32_t img, double sx, double sy, double sz) {
-			double xj, yj, zj;
+		auto position = [&](int j, double& xj, double& yj, double& zj) {
 			if constexpr (kRec) {
 				const float4* r4 = rec + (int64_t) kRecFloat4 * j;
 				const float4 A = r4[0], B = r4[1];
@@ -719,6 +715,8 @@ __global__ void __launch_bounds__(kRigidThreads,
 				yj = ry[j];
 				zj = rz[j];
 			}
+		};
+		auto consider = [&](int j, uint32_t img, double sx, double sy, double sz, double xj, double yj, double zj) {
 			// the halo image of j (DomainDecompDummy.cpp:64-70, 93-99); adding 0 is exact
 			const double m0 = __dsub_rn(xi, __dadd_rn(xj, sx));
 			const double m1 = __dsub_rn(yi, __dadd_rn(yj, sy));
@@ -728,21 +726,33 @@ __global__ void __launch_bounds__(kRigidThreads,
 			np += 1.0;
 			if (dd == 0.0) same = true;
 			if (!kQ && !(dd < rclj2)) return;
-			const uint32_t code = ((uint32_t) j << 5) | img;
-			if (kDirect && vl.list) {
-				eval_pair(code);   // from a list: evaluated at once
-				return;
-			}
-			list[cnt * kRigidThreads] = code;
-			if (++cnt == kRigidList) evaluate();
+			list[cnt++ * kRigidThreads] = ((uint32_t) j << 5) | img;
 		};
 		const int32_t nlist = vl.list ? vl.count[i] : -1;
 		if (nlist >= 0) {
-			for (int e = sub; e < nlist; e += kRigidLanes) {
-				const uint32_t code = vl.list[(int64_t) e * n + i];
-				const uint32_t img = code & 31u;
-				consider((int) (code >> 5), img, (double) ((int) (img % 3u) - 1) * g.L[0],
-				         (double) ((int) ((img / 3u) % 3u) - 1) * g.L[1], (double) ((int) (img / 9u) - 1) * g.L[2]);
+			// kScan entries at a time: their codes, then their positions are in flight together (one after
+			// another, each entry waited for two dependent loads: 256,000 two-centre molecules 233 us per step,
+			// 203 now, in FP64 350 and 293; loading the next partner ahead in the evaluation as well spilled
+			// and took 215)
+			for (int e0 = sub; e0 < nlist; e0 += kScan * kRigidLanes) {
+				if (cnt + kScan > kRigidList) evaluate();
+				uint32_t code[kScan];
+				double x[kScan], y[kScan], z[kScan];
+#pragma unroll
+				for (int u = 0; u < kScan; u++) {
+					const int e = e0 + u * kRigidLanes;
+					code[u] = e < nlist ? vl.list[(int64_t) e * n + i] : 0u;
+				}
+#pragma unroll
+				for (int u = 0; u < kScan; u++) position((int) (code[u] >> 5), x[u], y[u], z[u]);
+#pragma unroll
+				for (int u = 0; u < kScan; u++) {
+					if (e0 + u * kRigidLanes >= nlist) break;
+					const uint32_t img = code[u] & 31u;
+					consider((int) (code[u] >> 5), img, (double) ((int) (img % 3u) - 1) * g.L[0],
+					         (double) ((int) ((img / 3u) % 3u) - 1) * g.L[1], (double) ((int) (img / 9u) - 1) * g.L[2], x[u],
+					         y[u], z[u]);
+				}
 			}
 		} else {
 			int cc[3];
@@ -787,7 +797,10 @@ __global__ void __launch_bounds__(kRigidThreads,
 						const int j0 = start[nb], j1 = start[nb + 1];
 						for (int j = j0 + sub; j < j1; j += kRigidLanes) {
 							if (j == i && !shifted) continue;
-							consider(j, img, sx, sy, sz);
+							double xj, yj, zj;
+							position(j, xj, yj, zj);
+							consider(j, img, sx, sy, sz, xj, yj, zj);
+							if (cnt == kRigidList) evaluate();
 						}
 					}
 				}
