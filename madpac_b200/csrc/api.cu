@@ -490,8 +490,9 @@ int mdgpu_create(mdgpu_ctx** out, const double length[3], double cutoff, double 
 	MD_CUDA(cudaMemset(c->scalars, 0, sizeof(double) * 64));
 	MD_CUDA(cudaMalloc(&c->status, sizeof(int)));
 	MD_CUDA(cudaMemset(c->status, 0, sizeof(int)));
-	MD_CUDA(cudaMalloc(&c->tickets, sizeof(unsigned) * 4));
-	MD_CUDA(cudaMemset(c->tickets, 0, sizeof(unsigned) * 4));
+	MD_CUDA(cudaMalloc(&c->tickets, sizeof(unsigned) * 8));
+	MD_CUDA(cudaMemset(c->tickets, 0, sizeof(unsigned) * 8));
+	c->trav_counts = c->tickets + 4;
 	MD_CUDA(cudaMallocHost(&c->h_scalars, sizeof(double) * 64));
 	MD_CUDA(cudaMallocHost(&c->h_status, sizeof(int)));
 	PairParams hp = pair_params(c->sp, c->rc, c->rc_lj);
@@ -539,7 +540,6 @@ int mdgpu_destroy(mdgpu_ctx* ctx) {
 	cudaFree(c->rb_slot);
 	cudaFree(c->tickets);
 	cudaFree(c->trav_list);
-	cudaFree(c->trav_counts);
 	cudaFree(c->brick_kind);
 	cudaFree(full->x.stage.ptr);
 	if (c->h_scalars) cudaFreeHost(c->h_scalars);
@@ -639,16 +639,15 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 		const int64_t blocks = (n + kReduceBlock - 1) / kReduceBlock;
 		c->partial_cap = (blocks > bricks ? blocks : bricks) + 1024;
 		MD_CUDA(cudaMalloc(&c->partials, sizeof(double) * 4 * c->partial_cap));
-		if (!c->trav_list) {
+		if (!c->trav_list && bricks >= sparse_min_bricks(c)) {
 			MD_CUDA(cudaMalloc(&c->trav_list, sizeof(int32_t) * bricks));
-			MD_CUDA(cudaMalloc(&c->trav_counts, sizeof(unsigned) * 2));
 			c->trav_cap = (int) bricks;
 		}
 		c->cap = n;
 	}
 	c->n = n;
 	void* st;
-	MD_CUDA(staging(c, x->stage, sizeof(double) * (F ? 9 : 6) * n, &st));
+	MD_CUDA(staging(c, x->stage, sizeof(double) * 11 * n, &st));   // as much as a read-back of every field takes
 	double* aos = (double*) st;
 	const size_t b3 = sizeof(double) * 3 * n;
 	const CopySpan in[5] = {{(void*) r, aos, b3},

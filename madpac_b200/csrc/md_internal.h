@@ -111,7 +111,7 @@ struct Context {
 	unsigned* tickets = nullptr;    // last-block counters of the in-kernel reductions (self-resetting)
 	PairParams* d_pp = nullptr;     // device copy of the pair parameters
 	// the traversal's bricks that are not sparse (trav_cap entries; null: no sparse bricks looked for),
-	// their number and the queue over them
+	// their number and the queue over them (two words beside the tickets)
 	int32_t* trav_list = nullptr;
 	int trav_cap = 0;
 	unsigned* trav_counts = nullptr;
@@ -168,6 +168,8 @@ struct Context {
 };
 
 // Whether the Verlet-skin steps evaluate pruned lists (an inner radius between rc and rc + skin).
+// Fewest bricks of a traversal that looks for sparse ones first: two rounds of resident CTAs (three per SM).
+inline int64_t sparse_min_bricks(const Context* c) { return 6 * (int64_t) c->num_sms; }
 inline bool pruning(const Context* c) { return c->skin > 0.0 && c->prune > 0.0 && c->prune < c->skin; }
 
 // ---- launch helpers implemented in the .cu files -------------------------------------------

@@ -350,7 +350,7 @@ brick::Lists lists_of(Context* c) {
 // are expected to be sparse -- a dilute fluid, or one that leaves much of the box nearly empty (the density
 // around a typical molecule is well above the mean). A homogeneous liquid has none, and skips the launch.
 bool sparse_traversal(const Context* c, const Plan& P) {
-	if (!c->trav_list || P.nbricks > c->trav_cap || P.nbricks < 2 * kTraverseMinBlocks * c->num_sms) return false;
+	if (!c->trav_list || P.nbricks > c->trav_cap || P.nbricks < sparse_min_bricks(c)) return false;
 	const Grid& g = c->g;
 	const double rho = (double) c->n / (g.L[0] * g.L[1] * g.L[2]);
 	const double cell = g.cell_length[0] * g.cell_length[1] * g.cell_length[2];
