@@ -144,32 +144,35 @@ int check_status(Context* c) {
 	return fail(c, MDGPU_ERR_CUDA, "unknown device status");
 }
 
-void free_particles(Particles& p) {
-	cudaFree(p.rx);
-	cudaFree(p.ry);
-	cudaFree(p.rz);
-	cudaFree(p.vx);
-	cudaFree(p.vy);
-	cudaFree(p.vz);
-	cudaFree(p.fx);
-	cudaFree(p.fy);
-	cudaFree(p.fz);
-	cudaFree(p.id);
-	cudaFree(p.cid);
-	cudaFree(p.uidx);
-	p = Particles{};
+// Both particle sets of the context in one allocation (24 small ones made a quarter of the time to set up a
+// box of some ten thousand molecules), every array on a 256-byte boundary.
+cudaError_t alloc_particles(Context* c, int64_t n) {
+	const auto pad = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+	const size_t d = pad(sizeof(double) * n), i = pad(sizeof(int32_t) * n), set = 10 * d + 2 * i;
+	static_assert(sizeof(uint64_t) == sizeof(double), "ids take a double's place");
+	const cudaError_t e = cudaMalloc(&c->particle_block, 2 * set);
+	if (e != cudaSuccess) return e;
+	Particles* sets[2] = {&c->p, &c->q};
+	for (int k = 0; k < 2; k++) {
+		unsigned char* at = static_cast<unsigned char*>(c->particle_block) + k * set;
+		Particles& p = *sets[k];
+		double** arrays[] = {&p.rx, &p.ry, &p.rz, &p.vx, &p.vy, &p.vz, &p.fx, &p.fy, &p.fz};
+		for (double** a : arrays) {
+			*a = reinterpret_cast<double*>(at);
+			at += d;
+		}
+		p.id = reinterpret_cast<uint64_t*>(at);
+		p.cid = reinterpret_cast<int32_t*>(at + d);
+		p.uidx = reinterpret_cast<int32_t*>(at + d + i);
+	}
+	return cudaSuccess;
 }
 
-cudaError_t alloc_particles(Particles& p, int64_t n) {
-	double** d[] = {&p.rx, &p.ry, &p.rz, &p.vx, &p.vy, &p.vz, &p.fx, &p.fy, &p.fz};
-	for (double** a : d) {
-		cudaError_t e = cudaMalloc(a, sizeof(double) * n);
-		if (e != cudaSuccess) return e;
-	}
-	cudaError_t e = cudaMalloc(&p.id, sizeof(uint64_t) * n);
-	if (e == cudaSuccess) e = cudaMalloc(&p.cid, sizeof(int32_t) * n);
-	if (e == cudaSuccess) e = cudaMalloc(&p.uidx, sizeof(int32_t) * n);
-	return e;
+void free_particles(Context* c) {
+	cudaFree(c->particle_block);
+	c->particle_block = nullptr;
+	c->p = Particles{};
+	c->q = Particles{};
 }
 
 // Staging buffer for AoS transfers (n x 3 doubles), reused between calls.
@@ -508,8 +511,7 @@ int mdgpu_destroy(mdgpu_ctx* ctx) {
 	Context* c = &ctx->c;
 	cudaSetDevice(c->device);
 	if (c->stream) cudaStreamSynchronize(c->stream);
-	free_particles(c->p);
-	free_particles(c->q);
+	free_particles(c);
 	cudaFree(c->cell);
 	cudaFree(c->rank);
 	cudaFree(c->perm);
@@ -621,16 +623,15 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 	MD_CUDA(cudaSetDevice(c->device));
 	MD_CUDA(cudaStreamSynchronize(c->stream));
 	if (n > c->cap) {
-		free_particles(c->p);
-		free_particles(c->q);
+		free_particles(c);
 		cudaFree(c->cell);
 		cudaFree(c->rank);
 		cudaFree(c->perm);
 		cudaFree(c->partials);
 		c->cell = c->rank = c->perm = nullptr;
 		c->partials = nullptr;
-		MD_CUDA(alloc_particles(c->p, n));
-		MD_CUDA(alloc_particles(c->q, n));
+		c->cap = 0;
+		MD_CUDA(alloc_particles(c, n));
 		MD_CUDA(cudaMalloc(&c->cell, sizeof(int32_t) * n));
 		MD_CUDA(cudaMalloc(&c->rank, sizeof(int32_t) * n));
 		MD_CUDA(cudaMalloc(&c->perm, sizeof(int32_t) * n));

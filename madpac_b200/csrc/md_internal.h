@@ -92,6 +92,7 @@ struct Context {
 	bool cells_valid = false;
 	std::string err;
 
+	void* particle_block = nullptr;   // the allocation behind p and q
 	Particles p{};      // current (sorted) arrays
 	Particles q{};      // permutation target
 	int32_t* cell = nullptr;        // inner cell of each particle (sorted order after update)
