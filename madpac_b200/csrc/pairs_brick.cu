@@ -78,7 +78,8 @@ __global__ void __launch_bounds__(brick::kThreads, 4)
 }
 
 // Verlet-skin build step (runs only when *gate is this step's id): the lists, no forces.
-__global__ void __launch_bounds__(brick::kThreads, 3)
+constexpr int kBuildMinBlocks = 3;
+__global__ void __launch_bounds__(brick::kThreads, kBuildMinBlocks)
     k_build_lists(brick::Box bx, int nbricks, int s_cap, const double* __restrict__ rx,
                   const double* __restrict__ ry, const double* __restrict__ rz, const int32_t* __restrict__ cstart,
                   const int* __restrict__ gate, int step, brick::Lists lists) {
@@ -249,25 +250,41 @@ struct Plan {
 	int nbricks;
 };
 
+// Shared memory per CTA with `ctas` of them per SM: the SM's 228 KB, less 1 KB reserved per CTA and a margin.
+size_t share(const Context* c, int ctas) {
+	return std::min((size_t) (224 / ctas - 2) * 1024, (size_t) device_max_optin(c->device));
+}
+
+// Whether a capacity of s_cap staged molecules, that of `ctas` CTAs per SM, holds a region of 64 cells with
+// room for its fluctuations. The kernels take the most CTAs per SM for which it does: a region above the
+// capacity gathers its candidates from global memory, ten times as slow. The cells of a small box can be much
+// larger than the radius asks for (3 or 4 along an edge, two or three times the molecules), so the last step
+// is the whole SM for one CTA. A grid of one CTA per SM or less loses nothing by it and asks for the most
+// room (with 3 cells along an edge a region holds some of them twice); a larger one asks for little before
+// that last step (a liquid's regions differ by a percent or two). 20 steps of FP64 runs with skin 0.3, at a
+// density of 0.7 and a cutoff of 2.5, in ms, with one fixed capacity and with this rule: 1,500 molecules
+// 11.2 and 1.5, 3,300 10.0 and 1.3, 5,000 23.7 and 1.8 (FP32 25.3 and 1.5), 8,000 4.8 and 1.3.
+bool region_fits(const Context* c, const Grid& g, int kind, int ctas, int s_cap) {
+	const double rho = c->rho_typ > 0.0 ? c->rho_typ : (double) c->n / (g.L[0] * g.L[1] * g.L[2]);
+	const double region = 64.0 * rho * g.cell_length[0] * g.cell_length[1] * g.cell_length[2];
+	const int64_t nbricks = (int64_t) ((g.nc[0] + 1) / 2) * ((g.nc[1] + 1) / 2) * ((g.nc[2] + 1) / 2);
+	const double room = nbricks <= c->num_sms || (kind == 0 && ctas > 2) ? 1.3 : ctas > 2 ? 1.15 : 1.05;
+	return room * region + 64.0 <= s_cap;
+}
+
 // kind 0: plain traversal, 2: list evaluation of the skin mode.
 Plan plan(Context* c, const Grid& g, double filter_radius, int kind) {
 	const bool fp64 = kind == 0 || c->precision == MDGPU_FP64;   // the traversal evaluates both modes in FP64
 	Plan P;
 	brick::init_box(P.bx, g, filter_radius, 0, kind == 0 ? 0.0 : 0.5 * c->skin);
-	const int max_optin = device_max_optin(c->device);
-	size_t budget = 110 * 1024;
-	if (kind == 0) {
-		// three CTAs per SM when a region of 64 cells fits their share with room for its fluctuations
-		const size_t small = (224 / kTraverseMinBlocks - 2) * 1024;
-		const double rho = c->rho_typ > 0.0 ? c->rho_typ : (double) c->n / (g.L[0] * g.L[1] * g.L[2]);
-		const double region = 64.0 * rho * g.cell_length[0] * g.cell_length[1] * g.cell_length[2];
-		if (1.3 * region + 64.0 <= brick::capacity_for(small, fp64, brick::kHitWords)) budget = small;
-	}
-	if (kind == 2) budget = std::min(budget, (size_t) (224 / kListMinBlocks - 2) * 1024);
-	if (kind == 2 && pruning(c)) budget -= brick::kPruneRingBytes;   // the prune variant's ring
-	if (budget > (size_t) max_optin) budget = (size_t) max_optin;
 	const int words = kind == 2 ? 0 : brick::kHitWords;
-	const int s_cap = brick::capacity_for(budget, fp64, words);
+	// The prune variant's ring takes its part of each share.
+	const size_t ring = kind == 2 && pruning(c) ? brick::kPruneRingBytes : 0;
+	int s_cap = 0;
+	for (int ctas = kind == 2 ? kListMinBlocks : kTraverseMinBlocks; ctas > 0; ctas--) {
+		s_cap = brick::capacity_for(share(c, ctas) - ring, fp64, words);
+		if (region_fits(c, g, kind, ctas, s_cap)) break;
+	}
 	P.p = brick::make_const(c->sp.n, s_cap, c->rc, c->rc_lj);
 	P.bytes = brick::layout(s_cap, fp64, words).total;
 	P.nbricks = P.bx.nb[0] * P.bx.nb[1] * P.bx.nb[2];
@@ -436,15 +453,19 @@ cudaError_t launch_pairs_skin(Context* c, int kick_mode, double dt, double* reco
 		launches++;
 	}
 	prof_begin(c, 1);
-	// build (gated): half-precision staging only, three CTAs per SM
+	// build (gated): half-precision staging only
 	brick::Box bb{};
 	brick::init_box(bb, c->gs, c->rc + c->skin, 0, 0.5 * c->skin);
-	int s_cap = 256;
-	while (brick::build_bytes(s_cap + 64) <= 72 * 1024) s_cap += 64;
+	int s_cap = 0, ctas = kBuildMinBlocks;
+	for (;; ctas--) {
+		s_cap = 256;
+		while (brick::build_bytes(s_cap + 64) <= share(c, ctas)) s_cap += 64;
+		if (ctas == 1 || region_fits(c, c->gs, 2, ctas, s_cap)) break;
+	}
 	const size_t bbytes = brick::build_bytes(s_cap);
 	const int nbricks = bb.nb[0] * bb.nb[1] * bb.nb[2];
 	cudaError_t e = cudaFuncSetAttribute(k_build_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bbytes);
-	const int grid = std::min(nbricks, 3 * c->num_sms);   // three CTAs per SM (launch bounds, 72 KB each)
+	const int grid = std::min(nbricks, ctas * c->num_sms);
 	if (e == cudaSuccess)
 		k_build_lists<<<grid, brick::kThreads, bbytes, c->stream>>>(bb, nbricks, s_cap, c->p.rx, c->p.ry, c->p.rz,
 		                                                           c->cell_start, c->rebuild, c->step_id, l);
