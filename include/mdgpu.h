@@ -35,7 +35,8 @@ extern "C" {
 
 /* ---- precision modes ---------------------------------------------------------------------- */
 #define MDGPU_FP64 0   /* every pair in double precision, same operation order as PotForceLJ */
-#define MDGPU_MIXED 1  /* pair arithmetic in FP32, forces/energy/virial accumulated in FP64 */
+#define MDGPU_MIXED 1  /* pair arithmetic in FP32, forces/energy/virial accumulated in FP64 (the traversal of
+                        * the per-step binning, where FP32 gains nothing, evaluates in FP64 in both modes) */
 
 /* One single-site LJ component: one LJ centre at the molecule origin.
  * Mirrors Component::addLJcenter (molecules/Component.cpp:44-72) with do_shift the

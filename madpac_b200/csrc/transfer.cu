@@ -126,13 +126,15 @@ void work(Job& job, Lane& l, bool to_host) {
 			std::memcpy(pending[b]->host, l.buf[b], pending[b]->bytes);
 }
 
-bool pinned(const void* host) {
+// Whether a span goes to the driver as it is: arrays that the caller pinned (the DMA runs at the link's rate by
+// itself), and what is not host memory, which the driver judges.
+bool plain_copy(const CopySpan& span) {
 	cudaPointerAttributes a{};
-	if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+	if (cudaPointerGetAttributes(&a, span.host) != cudaSuccess) {
 		cudaGetLastError();
 		return false;
 	}
-	return a.type == cudaMemoryTypeHost;
+	return a.type == cudaMemoryTypeDevice || (a.type == cudaMemoryTypeHost && span.bytes >= kChunk);
 }
 
 cudaError_t copy(int device, cudaStream_t s, const CopySpan* spans, int n, bool to_host) {
@@ -144,8 +146,7 @@ cudaError_t copy(int device, cudaStream_t s, const CopySpan* spans, int n, bool 
 		size_t total = 0;
 		for (int k = 0; k < n; k++) {
 			if (!spans[k].host || spans[k].bytes == 0) continue;
-			if (spans[k].bytes >= kChunk && pinned(spans[k].host)) {
-				// pinned by the caller: the DMA runs at the link's rate by itself
+			if (plain_copy(spans[k])) {
 				const cudaError_t e =
 				    to_host ? cudaMemcpyAsync(spans[k].host, spans[k].dev, spans[k].bytes, cudaMemcpyDeviceToHost, s)
 				            : cudaMemcpyAsync(spans[k].dev, spans[k].host, spans[k].bytes, cudaMemcpyHostToDevice, s);
