@@ -257,9 +257,9 @@ size_t share(const Context* c, int ctas) {
 
 // Whether a capacity of s_cap staged molecules, that of `ctas` CTAs per SM, holds a region of 64 cells with
 // room for its fluctuations. The kernels take the most CTAs per SM for which it does: a region above the
-// capacity gathers its candidates from global memory, ten times as slow. The cells of a small box can be much
-// larger than the radius asks for (3 or 4 along an edge, two or three times the molecules), so the last step
-// is the whole SM for one CTA. A grid of one CTA per SM or less loses nothing by it and asks for the most
+// capacity gathers its candidates from global memory, ten times as slow. The skin cells of a small box can be
+// much larger than the radius asks for (3 or 4 along an edge, two or three times the molecules), so the lists'
+// last step is the whole SM for one CTA. A grid of one CTA per SM or less loses nothing by it and asks for the most
 // room (with 3 cells along an edge a region holds some of them twice); a larger one asks for little before
 // that last step (a liquid's regions differ by a percent or two). 20 steps of FP64 runs with skin 0.3, at a
 // density of 0.7 and a cutoff of 2.5, in ms, with one fixed capacity and with this rule: 1,500 molecules
@@ -281,7 +281,9 @@ Plan plan(Context* c, const Grid& g, double filter_radius, int kind) {
 	// The prune variant's ring takes its part of each share.
 	const size_t ring = kind == 2 && pruning(c) ? brick::kPruneRingBytes : 0;
 	int s_cap = 0;
-	for (int ctas = kind == 2 ? kListMinBlocks : kTraverseMinBlocks; ctas > 0; ctas--) {
+	// the traversal stops at two CTAs, the batched ensemble's capacity: both then gather the same bricks, and a
+	// box steps bit for bit as it does alone
+	for (int ctas = kind == 2 ? kListMinBlocks : kTraverseMinBlocks; ctas >= (kind == 2 ? 1 : 2); ctas--) {
 		s_cap = brick::capacity_for(share(c, ctas) - ring, fp64, words);
 		if (region_fits(c, g, kind, ctas, s_cap)) break;
 	}
