@@ -242,8 +242,8 @@ __device__ __forceinline__ unsigned pack_lo(float lx, float ly, float lz, int ci
 
 __device__ __forceinline__ int unpack_cid(unsigned w) { return (int) ((w >> 27) & 7u); }
 
-// Component of a staged slot (FP64), always within the pair table: idle lanes and the padding of lists also
-// look at slots that nothing was staged to.
+// Component of a staged slot (FP64). The mask is a bounds guard only: no lane looks at a slot that nothing was
+// staged to (idle lanes and the padding of lists look at a molecule of their own brick).
 __device__ __forceinline__ int component(const Smem& S, int slot) { return S.comp[slot] & (kMaxSpecies - 1); }
 static_assert((kMaxSpecies & (kMaxSpecies - 1)) == 0, "a power of two");
 
@@ -527,7 +527,8 @@ struct Sums64 {
 };
 
 // One candidate pair in FP64: d = r_i - r_j, branch-free (a pair outside the cutoffs, or v = false,
-// adds zeros). The squared distance and both cutoff tests keep the reference's operations and
+// adds zeros, provided that d and the pair parameters are finite: a caller without a partner passes a
+// staged one). The squared distance and both cutoff tests keep the reference's operations and
 // roundings (no contraction), so the pairs within rc are the reference's; the force law is
 // PotForceLJ's (molecules/potforce.h:41-53), contracted: with s6 = (sig2/r^2)^3, m = s6^2 - s6 and
 // e = s6^2 + m the sums are F += (e/r^2) d, U += m, W += e (the virial term d.f is e, as f = (e/r^2) d):
@@ -1313,9 +1314,10 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 			for (int u = 0; u < 8; u++) {
 				const int kk = 8 * b + u;
 				const unsigned raw = (e[u >> 1] >> (16 * (u & 1))) & 0xffffu;
-				const int j = min((int) raw, p.s_cap - 1);
-				// (a pruned list may hold sentinel slots before its end)
+				// (a pruned list may hold sentinel slots before its end); what is no entry looks at the
+				// molecule itself: nothing was staged to the sentinel's slot, whose bytes may be a NaN
 				const bool v = kk < cnt && raw < (unsigned) p.s_cap;
+				const int j = v ? (int) raw : slot_i;
 				double e24 = 0.0, sg2 = S.pd[KK], sh6 = 0.0;
 				if (!kSingle) {
 					const int pk = ti * ns + component(S, j);
