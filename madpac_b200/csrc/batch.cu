@@ -14,7 +14,8 @@
 //      move into the other buffer. The result is the same (cell, id) order as the single-box path.
 //   -- grid barrier --
 //   B  all bricks of all boxes (static stride or an atomic queue): brick::pairs, the single-box
-//      pair kernel's per-brick work, so forces match the single-box path bit for bit.
+//      pair kernel's per-brick work, so forces match the single-box path bit for bit (where both have the
+//      same staged capacity, two CTAs per SM, or the brick fits in both).
 //   -- grid barrier --
 //   C  per box: Leapfrog post-kick (Molecule::upd_postF, Molecule.cpp:193-205), sum m v^2, and the
 //      box's brick partials in a fixed order -> the step record {Upot, virial, sum m v^2, pairs}.
@@ -446,7 +447,7 @@ __device__ __forceinline__ void for_my_boxes(const StepArgs& a, F&& f) {
 }
 
 template <bool kFP64, bool kSingle, bool kLjIsRc, int kCap>
-__global__ void __launch_bounds__(kThreads, 2) k_batch_step(StepArgs a) {
+__global__ void __launch_bounds__(kThreads, 2) k_batch_step(const __grid_constant__ StepArgs a) {
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ int s_flag;
 	__shared__ int s_item;

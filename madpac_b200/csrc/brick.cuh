@@ -21,11 +21,13 @@
 // absolute, one 16-byte shared load per candidate.
 // The exact cutoff test is dd < rc^2, strict as BlockTraverse.cpp:155, decided in FP64 as the reference
 // decides it; the force law is PotForceLJ's (molecules/potforce.h:41-53). A brick whose region holds more
-// molecules than the shared-memory capacity gathers straight from global memory instead.
+// molecules than the shared-memory capacity is evaluated in parts by the traversal (pairs_in_parts); the list
+// kernels, whose capacity follows the density, gather its candidates straight from global memory.
 //
 // Each unordered pair is evaluated from both sides; energy and virial are halved on readout.
 // Orders of staging, enumeration and accumulation are fixed: results are deterministic and do not
-// depend on which CTA evaluates a brick.
+// depend on which CTA evaluates a brick. (Between launches of different capacity, one of which evaluates a
+// brick whole and the other in parts, the order of a molecule's pairs and the last bits differ.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -296,12 +298,24 @@ __device__ __forceinline__ int staged_coord(const Box& bx, int d, int b, int l, 
 	return gc;
 }
 
-// Prefix sums (9) of the counts of a brick's own cells (cells beyond the grid count as empty) and their
-// staged cells (8), by one warp; the counts of staged cells 2 l and 2 l + 1 are in lane l's na and nb.
-__device__ __forceinline__ void own_prefix(const Box& bx, int brick, int na, int nb, int* s_own, int* s_ocell) {
+// Part of a brick: node 1 is the brick, nodes 2 n and 2 n + 1 are the halves of node n, which split z, then y,
+// then x. The own cells of a part are w (in binary zyx) with w >> (3 - level) == node - 2^level; it needs the
+// cells next to those, 48, 36 or 27 of the 64. True for coordinate l of the staged cells in dimension d.
+__device__ __forceinline__ int part_level(int node) { return 31 - __clz(node); }
+__device__ __forceinline__ bool in_part(int node, int d, int l) {
+	const int level = part_level(node);
+	if (level < 3 - d) return true;
+	return (unsigned) (l - ((node >> (level - 3 + d)) & 1)) <= 2u;
+}
+
+// Prefix sums (9) of the counts of a part's own cells (the other own cells, and cells beyond the grid, count as
+// empty) and their staged cells (8), by one warp; the counts of staged cells 2 l and 2 l + 1 are in lane l's
+// na and nb.
+__device__ __forceinline__ void own_prefix(const Box& bx, int brick, int node, int na, int nb, int* s_own,
+                                           int* s_ocell) {
 	const int lane = threadIdx.x & 31;
 	int ic = 0;
-	const bool ok = lane < kWarps && own_cell(bx, brick, lane, ic);
+	const bool ok = lane < kWarps && own_cell(bx, brick, lane, ic) && ((8 + lane) >> (3 - part_level(node))) == node;
 	const int a = __shfl_sync(kFull, na, ic >> 1), b = __shfl_sync(kFull, nb, ic >> 1);
 	const int c = ok ? ((ic & 1) ? b : a) : 0;
 	int own = c;
@@ -353,7 +367,7 @@ __device__ __forceinline__ bool stage_cells(const Const& p, const Box& bx, int b
 			S.cs[2 * lane + 1] = excl + a;
 			if (lane == 31) S.cs[64] = inc;
 		} else {
-			own_prefix(bx, brick, a, b, s_own, s_ocell);
+			own_prefix(bx, brick, 1, a, b, s_own, s_ocell);
 		}
 	}
 	__syncthreads();
@@ -410,9 +424,10 @@ __device__ __forceinline__ bool stage_cells(const Const& p, const Box& bx, int b
 // Staging of the traversal, whose cells hold few molecules (12 of a warp's 32 lanes at rc = 2.5 in a
 // liquid): the 16 rows of four cells, which are contiguous slots, two rows per warp. Return value and
 // arguments as stage_cells. Its CTA barrier at the end is its only one: every warp loads all cell starts
-// and scans the counts itself (two cells per lane) instead of waiting for one warp's scan.
-__device__ __forceinline__ bool stage_rows(const Const& p, const Box& bx, int brick, const Smem& S, const double* rx,
-                                           const double* ry, const double* rz, const int32_t* cid,
+// and scans the counts itself (two cells per lane) instead of waiting for one warp's scan. Of a part (node > 1)
+// only the cells that it needs are staged; the others count as empty.
+__device__ __forceinline__ bool stage_rows(const Const& p, const Box& bx, int brick, int node, const Smem& S,
+                                           const double* rx, const double* ry, const double* rz, const int32_t* cid,
                                            const int32_t* cstart, int* s_own, int* s_ocell) {
 	const Grid& g = bx.g;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -425,7 +440,12 @@ __device__ __forceinline__ bool stage_rows(const Const& p, const Box& bx, int br
 	const int ca = row0 + staged_coord(bx, 0, bc[0], 2 * (lane & 1), t0, t1);
 	const int cb = row0 + staged_coord(bx, 0, bc[0], 2 * (lane & 1) + 1, t0, t1);
 	const int sa = cstart[ca], ea = cstart[ca + 1], sb = cstart[cb], eb = cstart[cb + 1];
-	const int na = max(0, ea - sa), nb = max(0, eb - sb);
+	int na = max(0, ea - sa), nb = max(0, eb - sb);
+	if (node > 1) {
+		const bool yz = in_part(node, 1, (lane >> 1) & 3) && in_part(node, 2, lane >> 3);
+		if (!yz || !in_part(node, 0, 2 * (lane & 1))) na = 0;
+		if (!yz || !in_part(node, 0, 2 * (lane & 1) + 1)) nb = 0;
+	}
 	int inc = na + nb;
 	for (int o = 1; o < 32; o <<= 1) {
 		const int y = __shfl_up_sync(kFull, inc, o);
@@ -443,7 +463,7 @@ __device__ __forceinline__ bool stage_rows(const Const& p, const Box& bx, int br
 		S.cnt[2 * lane] = na;
 		S.cnt[2 * lane + 1] = nb;
 	} else if (warp == 1) {
-		own_prefix(bx, brick, na, nb, s_own, s_ocell);
+		own_prefix(bx, brick, node, na, nb, s_own, s_ocell);
 	}
 	// lane 4 d + l holds the shift and the frame offset (of the brick's centre) of staged coordinate l of
 	// dimension d
@@ -610,6 +630,192 @@ __host__ __device__ constexpr int rows_per_lane(int lpm) { return lpm == 1 ? 9 :
 // Hit words a lane collects before it evaluates them.
 constexpr int kHitWords = 24;
 
+// The molecules s_own, s_ocell of a staged region: forces to fx, fy, fz, sums to U, W, NP.
+template <bool kSingle, bool kLjIsRc, int kWords>
+__device__ __forceinline__ void pairs_staged(const Const& p, const Box& bx, const Smem& S, const int* s_own,
+                                             const int* s_ocell, double* fx, double* fy, double* fz, int* status,
+                                             double& U, double& W, double& NP, bool& same) {
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const int ns = p.ns;
+	const int n_own = s_own[kWarps];
+	const int lpm = n_own > kThreads / 2 ? 1 : n_own > kThreads / 4 ? 2 : n_own > kThreads / 8 ? 4 : 8;
+	const int lg = lpm == 1 ? 0 : lpm == 2 ? 1 : lpm == 4 ? 2 : 3;
+	const int nrows = rows_per_lane(lpm);
+	const int sub = lane & (lpm - 1);
+	const unsigned long long rows = kRowsOf[lpm - 1 + sub];
+	unsigned* const words = S.words + tid;
+	const double eps24_d = S.pd[0], sig2_d = S.pd[KK], shift6_d = S.pd[2 * KK];
+	for (int base0 = 0; base0 < n_own; base0 += kThreads >> lg) {
+		const int t0 = base0 + ((warp * 32) >> lg);
+		if (t0 >= n_own) break;   // this warp has no molecule (in this round or a later one)
+		const int t = t0 + (lane >> lg);
+		const bool act = t < n_own;
+		int w = 0;
+		if (act)
+			while (w < kWarps - 1 && s_own[w + 1] <= t) w++;
+		const int il0 = 1 + (w & 1), il1 = 1 + ((w >> 1) & 1), il2 = 1 + (w >> 2);
+		const int oc = s_ocell[w];
+		const int slot_i = S.cs[oc] + (act ? t - s_own[w] : 0);
+		const int gi = S.gst[oc] + (act ? t - s_own[w] : 0);
+		const double xi = S.img[3 * slot_i], yi = S.img[3 * slot_i + 1], zi = S.img[3 * slot_i + 2];
+		const int ti = kSingle ? 0 : component(S, slot_i);
+		Sums64 s64{0.0, 0.0, 0.0, 0.0, 0.0, 0, 0};
+		int cnt = 0, hits = 0;   // words and hits collected
+
+		// evaluates the collected words
+		auto evaluate = [&]() {
+			const int mx = __reduce_max_sync(kFull, hits);
+			const unsigned* next = words;
+			unsigned wd = 0u, nx = *next;   // this word's bits left; the next word
+#pragma unroll 2
+			for (int h = 0; h < mx; h++) {
+				bool v = h < hits;
+				if (v && (wd & 0xffffu) == 0u) {
+					wd = nx;
+					next += kThreads;   // (the word past the last one is never used)
+				}
+				nx = *next;
+				const int bit = __ffs(wd) - 1;
+				const int j = v ? (int) (wd >> 16) + ((bit & 7) << 1) + (bit >> 3) : slot_i;
+				wd &= wd - 1u;
+				v = v && j != slot_i;
+				double e24 = 0.0, sg2 = sig2_d, sh6 = 0.0;
+				if (!kSingle) {
+					const int pk = ti * ns + component(S, j);
+					e24 = S.pd[pk];
+					sg2 = S.pd[KK + pk];
+					sh6 = S.pd[2 * KK + pk];
+				}
+				lj64<kSingle, kLjIsRc>(__dsub_rn(xi, S.img[3 * j]), __dsub_rn(yi, S.img[3 * j + 1]),
+				                       __dsub_rn(zi, S.img[3 * j + 2]), v, p.rc2, p.rclj2, e24, sg2, sh6, s64, same);
+			}
+			cnt = hits = 0;
+		};
+
+		// filter: packed half-precision test against rc^2 plus a margin covering its rounding
+		const __half* hh = S.h + 8 * (slot_i >> 1) + (slot_i & 1);
+		const __half2 xi2 = __half2half2(hh[0]), yi2 = __half2half2(hh[2]), zi2 = __half2half2(hh[4]);
+		const __half2 rc2h = __float2half2_rn(bx.rc2_h);
+		int q = 0, base = 0, left = 0;   // next row; this lane's next slot and what is left of its row
+		unsigned first = 0u;             // the slot before an odd first slot belongs to another row
+		for (bool more = true; more;) {
+			// fill: blocks until a lane's words are full or the rows are done
+			for (;;) {
+				const int nblk = (__reduce_max_sync(kFull, left) + 15) >> 4;
+				if (nblk <= 0) {
+					if (q == nrows) {
+						more = false;
+						break;
+					}
+					const int r = (int) (rows >> (4 * q)) & 15;
+					q++;
+					left = 0;
+					if (act && r < 9) {
+						const int k0 = (il0 - 1) + 4 * (il1 + (r % 3) - 1) + 16 * (il2 + (r / 3) - 1);
+						const int a = S.cs[k0];
+						base = a & ~1;
+						left = S.cs[k0 + 3] - base;
+						first = (unsigned) (a & 1);
+					}
+					continue;
+				}
+				const int room = kWords - __reduce_max_sync(kFull, cnt);
+				if (room == 0) break;
+				const HalfPair* H = S.h16 + (base >> 1);
+				for (int ib = min(nblk, room); ib > 0; ib--) {
+					// bit k: slot base + 2k, bit 16 + k: slot base + 2k + 1
+					unsigned m = 0u;
+					if (left > 0) {
+#pragma unroll
+						for (int k = 0; k < 8; k++) {
+							const HalfPair P = H[k];
+							const __half2 dx = __hsub2(xi2, P.x), dy = __hsub2(yi2, P.y), dz = __hsub2(zi2, P.z);
+							const __half2 d2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
+							m |= __hlt2_mask(d2, rc2h) & ((1u << k) | (1u << (16 + k)));
+						}
+						// keep slots in [a, b)
+						if (left < 16) m &= ((1u << ((left + 1) >> 1)) - 1u) | (((1u << (left >> 1)) - 1u) << 16);
+						m &= ~first;
+					}
+					first = 0u;
+					// even slots' bits in byte 0, odd slots' in byte 1, the block's first slot above
+					words[cnt * kThreads] = __byte_perm(m, (unsigned) base, 0x5420);
+					cnt += m != 0u ? 1 : 0;
+					hits += __popc(m);
+					base += 16;
+					left -= 16;
+					H += 8;
+				}
+			}
+			evaluate();
+		}
+		if (kSingle) sums64_finish<kLjIsRc>(s64, eps24_d, shift6_d);
+		U += s64.u;
+		W += s64.w;
+		NP += (double) s64.np;
+		// the molecule's force: its lanes' sums in a fixed order
+		for (int o = 1; o < lpm; o <<= 1) {
+			s64.x += __shfl_xor_sync(kFull, s64.x, o);
+			s64.y += __shfl_xor_sync(kFull, s64.y, o);
+			s64.z += __shfl_xor_sync(kFull, s64.z, o);
+		}
+		if (act && sub == 0) {
+			fx[gi] = s64.x;
+			fy[gi] = s64.y;
+			fz[gi] = s64.z;
+			if (!(isfinite(s64.x) && isfinite(s64.y) && isfinite(s64.z))) atomicOr(status, kStatusNonFinite);
+		}
+	}
+}
+
+// A brick whose region exceeds the staged capacity: in the largest parts that fit, one after the other (kept out
+// of the way of the ordinary bricks' code). Only a part of one own cell whose 27 cells do not fit gathers from
+// global memory. 200,000 molecules at a density of 0.85, us per step: cutoff 3.7 (regions of 3,100; 2,500 fit)
+// 1614 by gathering, 518 in parts; cutoff 4.4 3100 and 1311.
+template <bool kSingle, bool kLjIsRc, int kWords>
+__device__ __noinline__ void pairs_in_parts(const Const& p, const Box& bx, int brick, unsigned char* smem,
+                                            const double* rx, const double* ry, const double* rz, const int32_t* cid,
+                                            const int32_t* cstart, double* fx, double* fy, double* fz, int* s_own,
+                                            int* s_ocell, int* status, double* sums) {
+	const Smem S = views(smem, layout(p.s_cap, true, kWords));
+	double U = 0.0, W = 0.0, NP = 0.0;
+	bool same = false;
+	int node = 2;
+	do {
+		const int level = part_level(node);
+		int icell;
+		if (own_cell(bx, brick, (node << (3 - level)) & 7, icell)) {   // (the first cell: the others lie beyond it)
+			__syncthreads();   // before the next staging
+			const bool staged = stage_rows(p, bx, brick, node, S, rx, ry, rz, cid, cstart, s_own, s_ocell);
+			if (staged) {
+				pairs_staged<kSingle, kLjIsRc, kWords>(p, bx, S, s_own, s_ocell, fx, fy, fz, status, U, W, NP, same);
+			} else if (level < 3) {
+				node *= 2;
+				continue;
+			} else {
+				const int w = node & 7, gi0 = S.gst[s_ocell[w]];
+				for (int t = threadIdx.x; t < s_own[kWarps]; t += kThreads) {
+					const int gi = gi0 + t;
+					PairSums s = gather_pairs<false>(gi, rx, ry, rz, cid, cstart, bx.g, S.pd, p.ns, p.rc2, p.rclj2, bx.coff);
+					fx[gi] = s.F[0];
+					fy[gi] = s.F[1];
+					fz[gi] = s.F[2];
+					U += s.U;
+					W += s.W;
+					NP += s.np;
+					same |= s.same;
+				}
+			}
+		}
+		node++;
+		while (!(node & 1)) node >>= 1;   // both halves done: the next of the level above
+	} while (node > 1);
+	if (same) atomicOr(status, kStatusSamePosition);
+	sums[0] = U;
+	sums[1] = W;
+	sums[2] = NP;
+}
+
 // Forces on the molecules of brick `brick` (index within its box) of box `bx`; U, W and the pair
 // count go to partials[slot]. The pair table must already be in shared memory (load_params).
 // Ends with a CTA-wide barrier after which no thread reads the staged data.
@@ -636,161 +842,21 @@ __device__ __forceinline__ void pairs(const Const& p, const Box& bx, int brick, 
                                       const double* rx, const double* ry, const double* rz, const int32_t* cid,
                                       const int32_t* cstart, double* fx, double* fy, double* fz, double* partials,
                                       int* status) {
-	const SmemLayout L = layout(p.s_cap, true, kWords);
-	const Smem S = views(smem, L);
+	const Smem S = views(smem, layout(p.s_cap, true, kWords));
 	__shared__ int s_own[kWarps + 1], s_ocell[kWarps];
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const int ns = p.ns;
-	const bool staged = stage_rows(p, bx, brick, S, rx, ry, rz, cid, cstart, s_own, s_ocell);
-	const int n_own = s_own[kWarps];
 	double U = 0.0, W = 0.0, NP = 0.0;
-	bool same = false;
-	if (!staged) {
-		// over capacity: gather from global memory
-		for (int t = tid; t < n_own; t += kThreads) {
-			int w = 0;
-			while (w < kWarps - 1 && s_own[w + 1] <= t) w++;
-			const int gi = S.gst[s_ocell[w]] + (t - s_own[w]);
-			PairSums s = gather_pairs<false>(gi, rx, ry, rz, cid, cstart, bx.g, S.pd, ns, p.rc2, p.rclj2, bx.coff);
-			fx[gi] = s.F[0];
-			fy[gi] = s.F[1];
-			fz[gi] = s.F[2];
-			U += s.U;
-			W += s.W;
-			NP += s.np;
-			same |= s.same;
-		}
+	if (stage_rows(p, bx, brick, 1, S, rx, ry, rz, cid, cstart, s_own, s_ocell)) {
+		bool same = false;
+		pairs_staged<kSingle, kLjIsRc, kWords>(p, bx, S, s_own, s_ocell, fx, fy, fz, status, U, W, NP, same);
+		if (same) atomicOr(status, kStatusSamePosition);
 	} else {
-		const int lpm = n_own > kThreads / 2 ? 1 : n_own > kThreads / 4 ? 2 : n_own > kThreads / 8 ? 4 : 8;
-		const int lg = lpm == 1 ? 0 : lpm == 2 ? 1 : lpm == 4 ? 2 : 3;
-		const int nrows = rows_per_lane(lpm);
-		const int sub = lane & (lpm - 1);
-		const unsigned long long rows = kRowsOf[lpm - 1 + sub];
-		unsigned* const words = S.words + tid;
-		const double eps24_d = S.pd[0], sig2_d = S.pd[KK], shift6_d = S.pd[2 * KK];
-		for (int base0 = 0; base0 < n_own; base0 += kThreads >> lg) {
-			const int t0 = base0 + ((warp * 32) >> lg);
-			if (t0 >= n_own) break;   // this warp has no molecule (in this round or a later one)
-			const int t = t0 + (lane >> lg);
-			const bool act = t < n_own;
-			int w = 0;
-			if (act)
-				while (w < kWarps - 1 && s_own[w + 1] <= t) w++;
-			const int il0 = 1 + (w & 1), il1 = 1 + ((w >> 1) & 1), il2 = 1 + (w >> 2);
-			const int oc = s_ocell[w];
-			const int slot_i = S.cs[oc] + (act ? t - s_own[w] : 0);
-			const int gi = S.gst[oc] + (act ? t - s_own[w] : 0);
-			const double xi = S.img[3 * slot_i], yi = S.img[3 * slot_i + 1], zi = S.img[3 * slot_i + 2];
-			const int ti = kSingle ? 0 : component(S, slot_i);
-			Sums64 s64{0.0, 0.0, 0.0, 0.0, 0.0, 0, 0};
-			int cnt = 0, hits = 0;   // words and hits collected
-
-			// evaluates the collected words
-			auto evaluate = [&]() {
-				const int mx = __reduce_max_sync(kFull, hits);
-				const unsigned* next = words;
-				unsigned wd = 0u, nx = *next;   // this word's bits left; the next word
-#pragma unroll 2
-				for (int h = 0; h < mx; h++) {
-					bool v = h < hits;
-					if (v && (wd & 0xffffu) == 0u) {
-						wd = nx;
-						next += kThreads;   // (the word past the last one is never used)
-					}
-					nx = *next;
-					const int bit = __ffs(wd) - 1;
-					const int j = v ? (int) (wd >> 16) + ((bit & 7) << 1) + (bit >> 3) : slot_i;
-					wd &= wd - 1u;
-					v = v && j != slot_i;
-					double e24 = 0.0, sg2 = sig2_d, sh6 = 0.0;
-					if (!kSingle) {
-						const int pk = ti * ns + component(S, j);
-						e24 = S.pd[pk];
-						sg2 = S.pd[KK + pk];
-						sh6 = S.pd[2 * KK + pk];
-					}
-					lj64<kSingle, kLjIsRc>(__dsub_rn(xi, S.img[3 * j]), __dsub_rn(yi, S.img[3 * j + 1]),
-					                       __dsub_rn(zi, S.img[3 * j + 2]), v, p.rc2, p.rclj2, e24, sg2, sh6, s64, same);
-				}
-				cnt = hits = 0;
-			};
-
-			// filter: packed half-precision test against rc^2 plus a margin covering its rounding
-			const __half* hh = S.h + 8 * (slot_i >> 1) + (slot_i & 1);
-			const __half2 xi2 = __half2half2(hh[0]), yi2 = __half2half2(hh[2]), zi2 = __half2half2(hh[4]);
-			const __half2 rc2h = __float2half2_rn(bx.rc2_h);
-			int q = 0, base = 0, left = 0;   // next row; this lane's next slot and what is left of its row
-			unsigned first = 0u;             // the slot before an odd first slot belongs to another row
-			for (bool more = true; more;) {
-				// fill: blocks until a lane's words are full or the rows are done
-				for (;;) {
-					const int nblk = (__reduce_max_sync(kFull, left) + 15) >> 4;
-					if (nblk <= 0) {
-						if (q == nrows) {
-							more = false;
-							break;
-						}
-						const int r = (int) (rows >> (4 * q)) & 15;
-						q++;
-						left = 0;
-						if (act && r < 9) {
-							const int k0 = (il0 - 1) + 4 * (il1 + (r % 3) - 1) + 16 * (il2 + (r / 3) - 1);
-							const int a = S.cs[k0];
-							base = a & ~1;
-							left = S.cs[k0 + 3] - base;
-							first = (unsigned) (a & 1);
-						}
-						continue;
-					}
-					const int room = kWords - __reduce_max_sync(kFull, cnt);
-					if (room == 0) break;
-					const HalfPair* H = S.h16 + (base >> 1);
-					for (int ib = min(nblk, room); ib > 0; ib--) {
-						// bit k: slot base + 2k, bit 16 + k: slot base + 2k + 1
-						unsigned m = 0u;
-						if (left > 0) {
-#pragma unroll
-							for (int k = 0; k < 8; k++) {
-								const HalfPair P = H[k];
-								const __half2 dx = __hsub2(xi2, P.x), dy = __hsub2(yi2, P.y), dz = __hsub2(zi2, P.z);
-								const __half2 d2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
-								m |= __hlt2_mask(d2, rc2h) & ((1u << k) | (1u << (16 + k)));
-							}
-							// keep slots in [a, b)
-							if (left < 16) m &= ((1u << ((left + 1) >> 1)) - 1u) | (((1u << (left >> 1)) - 1u) << 16);
-							m &= ~first;
-						}
-						first = 0u;
-						// even slots' bits in byte 0, odd slots' in byte 1, the block's first slot above
-						words[cnt * kThreads] = __byte_perm(m, (unsigned) base, 0x5420);
-						cnt += m != 0u ? 1 : 0;
-						hits += __popc(m);
-						base += 16;
-						left -= 16;
-						H += 8;
-					}
-				}
-				evaluate();
-			}
-			if (kSingle) sums64_finish<kLjIsRc>(s64, eps24_d, shift6_d);
-			U += s64.u;
-			W += s64.w;
-			NP += (double) s64.np;
-			// the molecule's force: its lanes' sums in a fixed order
-			for (int o = 1; o < lpm; o <<= 1) {
-				s64.x += __shfl_xor_sync(kFull, s64.x, o);
-				s64.y += __shfl_xor_sync(kFull, s64.y, o);
-				s64.z += __shfl_xor_sync(kFull, s64.z, o);
-			}
-			if (act && sub == 0) {
-				fx[gi] = s64.x;
-				fy[gi] = s64.y;
-				fz[gi] = s64.z;
-				if (!(isfinite(s64.x) && isfinite(s64.y) && isfinite(s64.z))) atomicOr(status, kStatusNonFinite);
-			}
-		}
+		double sums[3];
+		pairs_in_parts<kSingle, kLjIsRc, kWords>(p, bx, brick, smem, rx, ry, rz, cid, cstart, fx, fy, fz, s_own, s_ocell,
+		                                         status, sums);
+		U = sums[0];
+		W = sums[1];
+		NP = sums[2];
 	}
-	if (same) atomicOr(status, kStatusSamePosition);
 	block_sum3_at(U, W, NP, partials, slot);
 }
 
