@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <new>
 #include <string>
 #include <vector>
@@ -406,6 +407,15 @@ int device_max_optin(int device) {
 	std::lock_guard<std::mutex> lock(mu);
 	if (cached) known[device] = v;
 	return v;
+}
+
+cudaError_t allow_dynamic_smem(const void* kernel, int device, size_t bytes) {
+	static std::mutex mu;
+	static std::map<std::pair<const void*, int>, size_t> limits;
+	std::lock_guard<std::mutex> lock(mu);
+	size_t& limit = limits[{kernel, device}];
+	if (bytes > limit) limit = bytes;
+	return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) limit);
 }
 
 int rebuild_prepare(Context* c) {

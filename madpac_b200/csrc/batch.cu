@@ -779,7 +779,7 @@ int plan(Batch* b, const Tiles& t, Launch& L) {
 		L.build_cap = bcap;
 		L.smem = std::max({brick::layout(lcap, fp64).total, brick::build_bytes(bcap), b->max_bin_bytes});
 	}
-	B_CUDA(cudaFuncSetAttribute(L.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) L.smem));
+	B_CUDA(allow_dynamic_smem((const void*) L.kern, b->device, L.smem));
 	int per_sm = 0;
 	B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, L.kern, kThreads, L.smem));
 	if (per_sm < 1) return bfail(b, MDGPU_ERR_CAPACITY, "the batched step kernel does not fit on an SM");

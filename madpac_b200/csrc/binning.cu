@@ -538,7 +538,7 @@ cudaError_t launch_bin(Context* c, bool permute_forces) {
 	cudaError_t e = cudaSuccess;
 	if (n > 0 && n <= kSmallMolecules && nc <= kSmallCells) {
 		const size_t bytes = small_bytes(n, nc);
-		e = cudaFuncSetAttribute(k_bin_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
+		e = allow_dynamic_smem((const void*) k_bin_small, c->device, bytes);
 		if (e == cudaSuccess)
 			k_bin_small<<<1, kSmallThreads, bytes, s>>>((int) n, c->g, c->p, c->q, c->cell_start, c->rank, permute_forces,
 			                                            c->status);

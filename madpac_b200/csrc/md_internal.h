@@ -237,6 +237,9 @@ int set_cuda_error(Context* c, cudaError_t e, const char* where);
 
 // cudaDevAttrMaxSharedMemoryPerBlockOptin of a device, queried once per device (api.cu).
 int device_max_optin(int device);
+// Lets the kernel be launched with `bytes` of dynamic shared memory. The limit belongs to the kernel and the device,
+// not to a launch, and containers of several host threads ask for different sizes: it is only ever raised.
+cudaError_t allow_dynamic_smem(const void* kernel, int device, size_t bytes);
 
 // Timing brackets around a group of launches (0 = binning, 1 = pairs, 2 = integration).
 void prof_begin(Context* c, int group);

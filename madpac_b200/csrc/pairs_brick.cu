@@ -304,7 +304,7 @@ bool fold_in_traversal(const Context* c, const Plan& P) { return P.nbricks <= kT
 
 template <typename K, typename... Extra>
 cudaError_t go(Context* c, const Plan& P, K kern, const int* gate, const brick::Lists& lists, Extra... extra) {
-	cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) P.bytes);
+	cudaError_t r = allow_dynamic_smem((const void*) kern, c->device, P.bytes);
 	// the list kernel runs as a resident grid over a queue of the dense bricks when the sparse ones are
 	// evaluated apart (lists.kind set, or lists.counts in the traversal); otherwise one CTA per brick
 	const bool queue = lists.kind || (lists.counts && !lists.nbr);
@@ -469,7 +469,7 @@ cudaError_t launch_pairs_skin(Context* c, int kick_mode, double dt, double* reco
 	}
 	const size_t bbytes = brick::build_bytes(s_cap);
 	const int nbricks = bb.nb[0] * bb.nb[1] * bb.nb[2];
-	cudaError_t e = cudaFuncSetAttribute(k_build_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bbytes);
+	cudaError_t e = allow_dynamic_smem((const void*) k_build_lists, c->device, bbytes);
 	const int grid = std::min(nbricks, ctas * c->num_sms);
 	if (e == cudaSuccess)
 		k_build_lists<<<grid, brick::kThreads, bbytes, c->stream>>>(bb, nbricks, s_cap, c->p.rx, c->p.ry, c->p.rz,
@@ -491,7 +491,7 @@ cudaError_t launch_pairs_skin(Context* c, int kick_mode, double dt, double* reco
 		                                 : k_pairs_list_sparse<false, false, false>));
 		const size_t sbytes = brick::kWarps * brick::sparse_warp_bytes(fp64);
 		const brick::Const ps = brick::make_const(c->sp.n, brick::kSparseCap, c->rc, c->rc_lj);
-		e = cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sbytes);
+		e = allow_dynamic_smem((const void*) ks, c->device, sbytes);
 		const int sgrid = resident_grid(c, ks, sbytes, (P.nbricks + brick::kWarps - 1) / brick::kWarps);
 		if (e == cudaSuccess)
 			ks<<<sgrid, brick::kThreads, sbytes, c->stream>>>(ps, P.bx, c->p.rx, c->p.ry, c->p.rz, c->p.cid,
