@@ -80,6 +80,11 @@ void give_lane(Lane& l) {
 	free_lane(l);
 }
 
+cudaError_t queue(cudaStream_t s, const CopySpan& c, bool to_host) {
+	return to_host ? cudaMemcpyAsync(c.host, c.dev, c.bytes, cudaMemcpyDeviceToHost, s)
+	               : cudaMemcpyAsync(c.dev, c.host, c.bytes, cudaMemcpyHostToDevice, s);
+}
+
 struct Job {
 	int device;
 	cudaStream_t stream;
@@ -112,9 +117,7 @@ void work(Job& job, Lane& l, bool to_host) {
 		const CopySpan* c = job.take();
 		if (!c) break;
 		if (!to_host) std::memcpy(l.buf[b], c->host, c->bytes);
-		const cudaError_t e = to_host ? cudaMemcpyAsync(l.buf[b], c->dev, c->bytes, cudaMemcpyDeviceToHost, job.stream)
-		                              : cudaMemcpyAsync(c->dev, l.buf[b], c->bytes, cudaMemcpyHostToDevice, job.stream);
-		if (!job.check(e)) break;
+		if (!job.check(queue(job.stream, CopySpan{l.buf[b], c->dev, c->bytes}, to_host))) break;
 		if (!job.check(cudaEventRecord(l.done[b], job.stream))) {
 			cudaStreamSynchronize(job.stream);
 			break;
@@ -137,57 +140,72 @@ bool plain_copy(const CopySpan& span) {
 	return a.type == cudaMemoryTypeDevice || (a.type == cudaMemoryTypeHost && span.bytes >= kChunk);
 }
 
-cudaError_t copy(int device, cudaStream_t s, const CopySpan* spans, int n, bool to_host) {
-	try {
-		Job job;
-		job.device = device;
-		job.stream = s;
-		bool direct = false;
-		size_t total = 0;
-		for (int k = 0; k < n; k++) {
-			if (!spans[k].host || spans[k].bytes == 0) continue;
-			if (plain_copy(spans[k])) {
-				const cudaError_t e =
-				    to_host ? cudaMemcpyAsync(spans[k].host, spans[k].dev, spans[k].bytes, cudaMemcpyDeviceToHost, s)
-				            : cudaMemcpyAsync(spans[k].dev, spans[k].host, spans[k].bytes, cudaMemcpyHostToDevice, s);
-				if (e != cudaSuccess) return e;
-				direct = true;
-				continue;
-			}
-			for (size_t o = 0; o < spans[k].bytes; o += kChunk)
-				job.chunks.push_back(CopySpan{(unsigned char*) spans[k].host + o, (unsigned char*) spans[k].dev + o,
-				                              std::min(kChunk, spans[k].bytes - o)});
-			total += spans[k].bytes;
-		}
-		if (!job.chunks.empty()) {
-			const int cores = std::max(1, (int) std::thread::hardware_concurrency() / 2);
-			const int want = std::max(1, std::min({kMaxThreads, cores, (int) (total / kPerThread)}));
-			std::vector<Lane> lanes;
-			lanes.reserve((size_t) want);
-			cudaError_t e = cudaSuccess;
-			for (int t = 0; t < want; t++) {
-				Lane l;
-				e = take_lane(device, l);
-				if (e != cudaSuccess) break;   // fewer lanes do as well
-				lanes.push_back(l);
-			}
-			if (lanes.empty()) return e;
-			std::vector<std::thread> threads;
-			threads.reserve(lanes.size());
-			try {
-				for (size_t t = 1; t < lanes.size(); t++)
-					threads.emplace_back([&job, &lanes, t, to_host] { work(job, lanes[t], to_host); });
-			} catch (...) {   // no more threads: those that run take all chunks
-			}
-			work(job, lanes[0], to_host);
-			for (auto& t : threads) t.join();
-			for (Lane& l : lanes) give_lane(l);
-			if (!job.ok()) return (cudaError_t) job.err.load();
-		}
-		return direct && to_host ? cudaStreamSynchronize(s) : cudaSuccess;
-	} catch (const std::bad_alloc&) {
-		return cudaErrorMemoryAllocation;
+// The lanes of one copy, given back at its end.
+struct Lanes {
+	std::vector<Lane> all;
+	~Lanes() {
+		for (Lane& l : all) give_lane(l);
 	}
+};
+
+// The copy; `direct` is set once one is queued that reads or writes the caller's memory by itself.
+cudaError_t copy_spans(int device, cudaStream_t s, const CopySpan* spans, int n, bool to_host, bool& direct) {
+	Job job;
+	job.device = device;
+	job.stream = s;
+	size_t total = 0;
+	for (int k = 0; k < n; k++) {
+		if (!spans[k].host || spans[k].bytes == 0) continue;
+		if (plain_copy(spans[k])) {
+			const cudaError_t e = queue(s, spans[k], to_host);
+			if (e != cudaSuccess) return e;
+			direct = true;
+			continue;
+		}
+		for (size_t o = 0; o < spans[k].bytes; o += kChunk)
+			job.chunks.push_back(CopySpan{(unsigned char*) spans[k].host + o, (unsigned char*) spans[k].dev + o,
+			                              std::min(kChunk, spans[k].bytes - o)});
+		total += spans[k].bytes;
+	}
+	if (job.chunks.empty()) return cudaSuccess;
+	const int cores = std::max(1, (int) std::thread::hardware_concurrency() / 2);
+	const int want = std::max(1, std::min({kMaxThreads, cores, (int) (total / kPerThread)}));
+	Lanes lanes;
+	lanes.all.reserve((size_t) want);
+	std::vector<std::thread> threads;
+	threads.reserve((size_t) want);
+	cudaError_t e = cudaSuccess;
+	for (int t = 0; t < want; t++) {
+		Lane l;
+		e = take_lane(device, l);
+		if (e != cudaSuccess) break;   // fewer lanes do as well
+		lanes.all.push_back(l);
+	}
+	if (lanes.all.empty()) return e;
+	try {
+		for (size_t t = 1; t < lanes.all.size(); t++)
+			threads.emplace_back([&job, &lanes, t, to_host] { work(job, lanes.all[t], to_host); });
+	} catch (...) {   // no more threads: those that run take all chunks
+	}
+	work(job, lanes.all[0], to_host);
+	for (auto& t : threads) t.join();
+	return (cudaError_t) job.err.load();
+}
+
+cudaError_t copy(int device, cudaStream_t s, const CopySpan* spans, int n, bool to_host) {
+	bool direct = false;
+	cudaError_t e;
+	try {
+		e = copy_spans(device, s, spans, n, to_host, direct);
+	} catch (const std::bad_alloc&) {
+		e = cudaErrorMemoryAllocation;
+	}
+	// what comes back is complete on return, and an error leaves no copy of the caller's memory in flight
+	if (direct && (to_host || e != cudaSuccess)) {
+		const cudaError_t es = cudaStreamSynchronize(s);
+		if (e == cudaSuccess) e = es;
+	}
+	return e;
 }
 
 }  // namespace
