@@ -174,14 +174,21 @@ cudaError_t copy_spans(int device, cudaStream_t s, const CopySpan* spans, int n,
 	lanes.all.reserve((size_t) want);
 	std::vector<std::thread> threads;
 	threads.reserve((size_t) want);
-	cudaError_t e = cudaSuccess;
 	for (int t = 0; t < want; t++) {
 		Lane l;
-		e = take_lane(device, l);
-		if (e != cudaSuccess) break;   // fewer lanes do as well
+		if (take_lane(device, l) != cudaSuccess) break;   // fewer lanes do as well
 		lanes.all.push_back(l);
 	}
-	if (lanes.all.empty()) return e;
+	if (lanes.all.empty()) {
+		// no pinned memory to be had: the driver stages the copies
+		cudaGetLastError();
+		for (const CopySpan& c : job.chunks) {
+			const cudaError_t e = queue(s, c, to_host);
+			if (e != cudaSuccess) return e;
+			direct = true;
+		}
+		return cudaSuccess;
+	}
 	try {
 		for (size_t t = 1; t < lanes.all.size(); t++)
 			threads.emplace_back([&job, &lanes, t, to_host] { work(job, lanes.all[t], to_host); });

@@ -49,6 +49,19 @@ def test_bytes(lib, sizes, to_host):
 
 
 @pytest.mark.parametrize("to_host", [False, True])
+def test_without_pinned_memory_the_driver_stages(lib, to_host):
+    lib.release()       # give the idle chunks back
+    lib.retain()
+    assert lib.fake_chunks() == 0
+    lib.fake_reset(1, -1)
+    st, in_flight, same, after = copy(lib, [20 * MB, 3, 5 * MB + 7], to_host)
+    assert st == 0 and all(after)
+    if to_host:
+        assert in_flight == 0 and all(same)
+    lib.fake_reset(0, -1)
+
+
+@pytest.mark.parametrize("to_host", [False, True])
 @pytest.mark.parametrize("fails_at", [1, 2, 3])
 def test_an_error_leaves_no_copy_of_the_callers_memory_in_flight(lib, to_host, fails_at):
     """Two arrays that the caller pinned and a pageable one; the second, third or fourth copy fails."""
