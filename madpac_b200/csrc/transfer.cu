@@ -130,14 +130,14 @@ void work(Job& job, Lane& l, bool to_host) {
 }
 
 // Whether a span goes to the driver as it is: arrays that the caller pinned (the DMA runs at the link's rate by
-// itself), and what is not host memory, which the driver judges.
+// itself), and device or managed memory, which the driver judges.
 bool plain_copy(const CopySpan& span) {
 	cudaPointerAttributes a{};
 	if (cudaPointerGetAttributes(&a, span.host) != cudaSuccess) {
 		cudaGetLastError();
 		return false;
 	}
-	return a.type == cudaMemoryTypeDevice || (a.type == cudaMemoryTypeHost && span.bytes >= kChunk);
+	return a.type != cudaMemoryTypeUnregistered && (a.type != cudaMemoryTypeHost || span.bytes >= kChunk);
 }
 
 // The lanes of one copy, given back at its end.

@@ -68,3 +68,10 @@ def test_an_error_leaves_no_copy_of_the_callers_memory_in_flight(lib, to_host, f
     lib.fake_reset(0, fails_at)
     st, in_flight, same, after = copy(lib, [2 * MB, 2 * MB, MB], to_host, [HOST, HOST, 0])
     assert st == 1 and in_flight == 0
+
+
+def test_managed_and_device_memory_go_to_the_driver(lib):
+    for t in (MANAGED, DEVICE):
+        lib.fake_reset(0, -1)
+        st, in_flight, same, after = copy(lib, [100, 3 * MB], True, [t, t])
+        assert st == 0 and in_flight == 0 and all(same) and lib.fake_plain() == 2
