@@ -10,6 +10,8 @@
 // arrays just allocated in 7 ms (25), 50 MB in in 1.9 ms (3.8); four threads 9 ms into new arrays.
 #include "transfer.h"
 
+#include <sched.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -140,6 +142,14 @@ bool plain_copy(const CopySpan& span) {
 	return a.type != cudaMemoryTypeUnregistered && (a.type != cudaMemoryTypeHost || span.bytes >= kChunk);
 }
 
+// Processors that this thread may run on (containers and batch systems give a process a part of the machine's).
+int processors() {
+	cpu_set_t set;
+	CPU_ZERO(&set);
+	if (sched_getaffinity(0, sizeof(set), &set) == 0) return std::max(1, CPU_COUNT(&set));
+	return std::max(1, (int) std::thread::hardware_concurrency());
+}
+
 // The lanes of one copy, given back at its end.
 struct Lanes {
 	std::vector<Lane> all;
@@ -168,8 +178,7 @@ cudaError_t copy_spans(int device, cudaStream_t s, const CopySpan* spans, int n,
 		total += spans[k].bytes;
 	}
 	if (job.chunks.empty()) return cudaSuccess;
-	const int cores = std::max(1, (int) std::thread::hardware_concurrency() / 2);
-	const int want = std::max(1, std::min({kMaxThreads, cores, (int) (total / kPerThread)}));
+	const int want = std::max(1, std::min({kMaxThreads, processors() / 2, (int) (total / kPerThread)}));
 	Lanes lanes;
 	lanes.all.reserve((size_t) want);
 	std::vector<std::thread> threads;

@@ -75,3 +75,15 @@ def test_managed_and_device_memory_go_to_the_driver(lib):
         lib.fake_reset(0, -1)
         st, in_flight, same, after = copy(lib, [100, 3 * MB], True, [t, t])
         assert st == 0 and in_flight == 0 and all(same) and lib.fake_plain() == 2
+
+
+def test_threads_follow_the_processors_the_process_may_use(lib):
+    """A copy of 64 MB takes up to eight threads, but on one or two processors only the calling one."""
+    allowed = os.sched_getaffinity(0)
+    try:
+        os.sched_setaffinity(0, sorted(allowed)[:2])
+        lib.fake_reset(0, -1)
+        st, in_flight, same, after = copy(lib, [64 * MB], True)
+        assert st == 0 and all(same) and lib.fake_threads() == 1
+    finally:
+        os.sched_setaffinity(0, allowed)
