@@ -573,6 +573,8 @@ int mdgpu_set_precision(mdgpu_ctx* ctx, int precision) {
 	if (!ctx) return MDGPU_ERR_ARG;
 	Context* c = &ctx->c;
 	if (precision != MDGPU_FP64 && precision != MDGPU_MIXED) return fail(c, MDGPU_ERR_ARG, "unknown precision mode");
+	// lists end with the sentinel slot of the form they were built for, whose staged capacity is its own
+	if (precision != c->precision) c->lists_valid = false;
 	c->precision = precision;
 	return MDGPU_OK;
 }

@@ -1212,6 +1212,11 @@ int mdgpu_batch_set_tiles(mdgpu_batch* h, int32_t list_cap, int32_t ctas_per_sm,
 	if (dynamic != 0 && dynamic != 1) return bfail(b, MDGPU_ERR_ARG, "dynamic must be 0 or 1");
 	if (ctas_per_sm == 2 && b->max_bin_bytes > 110 * 1024)
 		return bfail(b, MDGPU_ERR_CAPACITY, "the largest box needs one CTA per SM");
+	if (b->valid && ctas_per_sm != b->tiles.ctas) {
+		// the lists end with the sentinel slot of the other staged capacity
+		B_CUDA(cudaSetDevice(b->device));
+		B_CUDA(cudaMemsetAsync(b->valid, 0, sizeof(int), b->stream));
+	}
 	b->tiles.cap = list_cap;
 	b->tiles.ctas = ctas_per_sm;
 	b->tiles.dynamic = dynamic;
