@@ -736,6 +736,8 @@ int check_status(Batch* b) {
 	if (st & kStatusTimeout) {
 		// barrier words may be left mid-count: start them again
 		B_CUDA(cudaMemsetAsync(b->bar, 0, sizeof(unsigned) * 8, b->stream));
+		// and boxes may have been sorted whose lists were not built
+		if (b->valid) B_CUDA(cudaMemsetAsync(b->valid, 0, sizeof(int), b->stream));
 		B_CUDA(cudaStreamSynchronize(b->stream));
 		b->prepared = false;
 		return bfail(b, MDGPU_ERR_TIMEOUT, "a grid-barrier wait of the batched step kernel ran out");

@@ -74,3 +74,20 @@ def test_other_tiles_build_again(precision, tol):
             ref.close()
             assert rms(st["F"][k] - F) <= tol * rms(F)
     b.close()
+
+
+def test_a_wait_that_ran_out_builds_again():
+    """The step that gave up may have sorted boxes without building their lists."""
+    systems = [box(n, 2.5, n) for n in (600, 1500, 3000)]
+    b = M.Batch.from_systems(systems, M.FP64)
+    b.setSkin(0.3)
+    b.prepare()
+    builds = b.skinBuilds()
+    b.setBarrierTimeout(0)
+    with pytest.raises(M.MdgpuError) as ei:
+        b.run(1, DT)
+    assert ei.value.code == 9
+    b.setBarrierTimeout(2_000_000_000)
+    b.prepare()
+    assert b.skinBuilds() == builds + len(systems)
+    b.close()
