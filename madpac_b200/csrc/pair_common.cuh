@@ -14,10 +14,13 @@
 
 namespace mdgpu {
 
-// 1/x for a positive normal x: the hardware's approximation y (rcp.approx.ftz.f64, about 20 bits) and
-// one step of Chebyshev's third-order iteration, y + y (e + e^2) with e = 1 - x y: e^3 is below 2^-58,
-// so what is left is the last rounding. Three FP64 instructions and no branch; the correctly rounded
-// intrinsic, with its branch for special operands, made the whole FP64 evaluation a fifth slower.
+// 1/x for a positive normal x whose reciprocal is normal: the hardware's approximation y (rcp.approx.ftz.f64, about
+// 20 bits) and one step of Chebyshev's third-order iteration (J. F. Traub, Iterative Methods for the Solution of
+// Equations, 1964, for f(y) = 1/y - x), y + y (e + e^2) with e = 1 - x y: e^3 is below 2^-57, so what is left is
+// the last rounding, and the result is the nearest double or its neighbour (exponents from 2^-1000 to
+// 2^1000 tested). Zero gives a NaN, not infinity: a force that was infinite or NaN with the division is a NaN.
+// Three FP64 instructions and no branch; the correctly rounded intrinsic, with its branch for special operands,
+// made the whole FP64 evaluation a fifth slower.
 __device__ __forceinline__ double rcp64(double x) {
 	double y;
 	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
