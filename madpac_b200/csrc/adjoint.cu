@@ -62,6 +62,10 @@ __global__ void __launch_bounds__(kReduceBlock) k_adjoint(int64_t n, Particles p
 	}
 	__syncthreads();
 	const double cut2 = fmin(pp->rc2, pp->rclj2), gU6 = gU / 6.0;
+	// the scan tests the shifted molecule against the candidates as they are, which rounds differently from the
+	// traversal's image of the candidate: it lists a little more, and the pair evaluation decides as the
+	// traversal does. The forms differ by less than 1e-15 L^2.
+	const double near2 = cut2 + 1e-14 * (g.L[0] * g.L[0] + g.L[1] * g.L[1] + g.L[2] * g.L[2]);
 	// kAdjLanes consecutive lanes per molecule, each taking every kAdjLanes-th candidate of a cell
 	const int64_t i = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / kAdjLanes;
 	const int sub = threadIdx.x % kAdjLanes;
@@ -100,8 +104,10 @@ __global__ void __launch_bounds__(kReduceBlock) k_adjoint(int64_t n, Particles p
 		int32_t* aj = s_aj + threadIdx.x;
 		uint8_t* ai = s_ai + threadIdx.x;
 		auto eval_pair = [&](int j, double sx, double sy, double sz) {
-			const double d0 = xi - (p.rx[j] + sx), d1 = yi - (p.ry[j] + sy), d2 = zi - (p.rz[j] + sz);
-			const double q = d0 * d0 + d1 * d1 + d2 * d2;
+			const double d0 = __dsub_rn(xi, __dadd_rn(p.rx[j], sx)), d1 = __dsub_rn(yi, __dadd_rn(p.ry[j], sy));
+			const double d2 = __dsub_rn(zi, __dadd_rn(p.rz[j], sz));
+			const double q = __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
+			if (!(q < cut2)) return;
 			const int pk = ti * ns + p.cid[j];
 			const double w0 = wix - gfx[j], w1 = wiy - gfy[j], w2 = wiz - gfz[j];
 			const double c6 = s_c6[pk], c6s = s_c6s[pk];
@@ -194,7 +200,7 @@ __global__ void __launch_bounds__(kReduceBlock) k_adjoint(int64_t n, Particles p
 					for (int j = start[nb] + sub; j < j1; j += kAdjLanes) {
 						if (j == i && !shifted) continue;
 						const double d0 = xs - p.rx[j], d1 = ys - p.ry[j], d2 = zs - p.rz[j];
-						if (!(d0 * d0 + d1 * d1 + d2 * d2 < cut2)) continue;
+						if (!(d0 * d0 + d1 * d1 + d2 * d2 < near2)) continue;
 						aj[acnt * kReduceBlock] = j;
 						ai[acnt * kReduceBlock] = img;
 						if (++acnt == kAdjList) flush();
