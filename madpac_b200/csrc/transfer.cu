@@ -185,12 +185,14 @@ cudaError_t copy_spans(int device, cudaStream_t s, const CopySpan* spans, int n,
 	threads.reserve((size_t) want);
 	for (int t = 0; t < want; t++) {
 		Lane l;
-		if (take_lane(device, l) != cudaSuccess) break;   // fewer lanes do as well
+		if (take_lane(device, l) != cudaSuccess) {
+			cudaGetLastError();   // fewer lanes do as well: not an error of this call
+			break;
+		}
 		lanes.all.push_back(l);
 	}
 	if (lanes.all.empty()) {
 		// no pinned memory to be had: the driver stages the copies
-		cudaGetLastError();
 		for (const CopySpan& c : job.chunks) {
 			const cudaError_t e = queue(s, c, to_host);
 			if (e != cudaSuccess) return e;

@@ -28,7 +28,7 @@ size_t done = 0;
 std::map<const void*, cudaMemoryType> types;
 std::set<void*> chunks;
 std::set<long> threads;
-int fail_alloc = 0, fail_copy_at = -1, copies = 0, plain = 0;
+int fail_alloc = -1, allocs = 0, fail_copy_at = -1, copies = 0, plain = 0, last = 0;
 
 void run_to(size_t n) {
 	for (; done < n && done < ops.size(); done++) std::memcpy(ops[done].dst, ops[done].src, ops[done].bytes);
@@ -42,7 +42,7 @@ bool own(const void* p) {
 
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) {
 	std::lock_guard<std::mutex> l(mu);
-	if (fail_alloc) return cudaErrorMemoryAllocation;
+	if (fail_alloc >= 0 && allocs++ >= fail_alloc) return last = cudaErrorMemoryAllocation;
 	*p = ::operator new(bytes);
 	chunks.insert(*p);
 	return cudaSuccess;
@@ -78,7 +78,7 @@ cudaError_t cudaStreamSynchronize(cudaStream_t) {
 }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpyKind, cudaStream_t) {
 	std::lock_guard<std::mutex> l(mu);
-	if (copies++ == fail_copy_at) return cudaErrorInvalidValue;
+	if (copies++ == fail_copy_at) return last = cudaErrorInvalidValue;
 	threads.insert(syscall(SYS_gettid));
 	const bool mine = own(dst) || own(src);
 	plain += mine ? 0 : 1;
@@ -91,12 +91,17 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
 	a->type = it == types.end() ? cudaMemoryTypeUnregistered : it->second;
 	return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+	const int e = last;
+	last = 0;
+	return e;
+}
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 
 #include "transfer.cu"
 
 extern "C" {
+// alloc_fails: the first pinned allocation that fails, as do all after it (-1: none)
 void fake_reset(int alloc_fails, int copy_fails_at) {
 	std::lock_guard<std::mutex> l(mu);
 	ops.clear();
@@ -105,11 +110,12 @@ void fake_reset(int alloc_fails, int copy_fails_at) {
 	threads.clear();
 	fail_alloc = alloc_fails;
 	fail_copy_at = copy_fails_at;
-	copies = plain = 0;
+	copies = plain = allocs = last = 0;
 }
 void fake_type(const void* p, int type) { types[p] = (cudaMemoryType) type; }
 int fake_in_flight() { return (int) (ops.size() - done); }
 int fake_plain() { return plain; }
+int fake_last_error() { return last; }
 int fake_threads() { return (int) threads.size(); }
 int fake_chunks() { return (int) chunks.size(); }
 void fake_finish() { cudaStreamSynchronize(nullptr); }

@@ -43,7 +43,7 @@ def copy(lib, sizes, to_host, types=None):
 @pytest.mark.parametrize("to_host", [False, True])
 @pytest.mark.parametrize("sizes", [[1], [8, 0, 24], [MB // 2, MB // 2 + 1], [20 * MB, 3, 5 * MB + 7]])
 def test_bytes(lib, sizes, to_host):
-    lib.fake_reset(0, -1)
+    lib.fake_reset(-1, -1)
     st, in_flight, same, after = copy(lib, sizes, to_host)
     assert st == 0 and in_flight == 0 and all(same) and lib.fake_plain() == 0
 
@@ -53,26 +53,38 @@ def test_without_pinned_memory_the_driver_stages(lib, to_host):
     lib.release()       # give the idle chunks back
     lib.retain()
     assert lib.fake_chunks() == 0
-    lib.fake_reset(1, -1)
+    lib.fake_reset(0, -1)
     st, in_flight, same, after = copy(lib, [20 * MB, 3, 5 * MB + 7], to_host)
     assert st == 0 and all(after)
     if to_host:
         assert in_flight == 0 and all(same)
-    lib.fake_reset(0, -1)
+    lib.fake_reset(-1, -1)
+
+
+@pytest.mark.parametrize("alloc_fails", [0, 1, 2, 5])
+def test_a_copy_that_succeeds_leaves_no_error_behind(lib, alloc_fails):
+    """Some pinned chunks are to be had, others not: the copy does with fewer, and the next call that looks for the
+    errors of its own launches finds none."""
+    lib.release()
+    lib.retain()
+    lib.fake_reset(alloc_fails, -1)
+    st, in_flight, same, after = copy(lib, [20 * MB], True)
+    assert st == 0 and all(same) and lib.fake_last_error() == 0
+    lib.fake_reset(-1, -1)
 
 
 @pytest.mark.parametrize("to_host", [False, True])
 @pytest.mark.parametrize("fails_at", [1, 2, 3])
 def test_an_error_leaves_no_copy_of_the_callers_memory_in_flight(lib, to_host, fails_at):
     """Two arrays that the caller pinned and a pageable one; the second, third or fourth copy fails."""
-    lib.fake_reset(0, fails_at)
+    lib.fake_reset(-1, fails_at)
     st, in_flight, same, after = copy(lib, [2 * MB, 2 * MB, MB], to_host, [HOST, HOST, 0])
     assert st == 1 and in_flight == 0
 
 
 def test_managed_and_device_memory_go_to_the_driver(lib):
     for t in (MANAGED, DEVICE):
-        lib.fake_reset(0, -1)
+        lib.fake_reset(-1, -1)
         st, in_flight, same, after = copy(lib, [100, 3 * MB], True, [t, t])
         assert st == 0 and in_flight == 0 and all(same) and lib.fake_plain() == 2
 
@@ -82,7 +94,7 @@ def test_threads_follow_the_processors_the_process_may_use(lib):
     allowed = os.sched_getaffinity(0)
     try:
         os.sched_setaffinity(0, sorted(allowed)[:2])
-        lib.fake_reset(0, -1)
+        lib.fake_reset(-1, -1)
         st, in_flight, same, after = copy(lib, [64 * MB], True)
         assert st == 0 and all(same) and lib.fake_threads() == 1
     finally:
