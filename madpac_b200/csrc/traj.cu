@@ -273,6 +273,7 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 	if (!c->traj) c->traj = new Traj();
 	Traj* t = c->traj;
 	const int64_t n = c->n;
+	t->valid = false;   // nothing to go backward on until this pass is through
 	t->n = n;
 	t->nsteps = nsteps;
 	t->every = std::min(checkpoint_every, nsteps);
@@ -285,6 +286,7 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 	if (need_snaps > t->cap_snaps) {
 		cudaFree(t->snaps);
 		t->snaps = nullptr;
+		t->cap_snaps = 0;
 		e = cudaMalloc(&t->snaps, sizeof(double) * need_snaps);
 		if (e != cudaSuccess) return set_cuda_error(c, e, "cudaMalloc (trajectory snapshots)");
 		t->cap_snaps = need_snaps;
@@ -292,6 +294,7 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 	if (need_seg > t->cap_seg) {
 		cudaFree(t->seg);
 		t->seg = nullptr;
+		t->cap_seg = 0;
 		e = cudaMalloc(&t->seg, sizeof(double) * need_seg);
 		if (e != cudaSuccess) return set_cuda_error(c, e, "cudaMalloc (trajectory segment)");
 		t->cap_seg = need_seg;
@@ -300,6 +303,7 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 		cudaFree(t->rbar);
 		cudaFree(t->gs);
 		t->rbar = t->gs = nullptr;
+		t->cap_n = 0;
 		// rbar, vbar, Fbar (3n each), cm (n), rows (6n); gs, os (3n each), pgrad, par
 		e = cudaMalloc(&t->rbar, sizeof(double) * 16 * n);
 		if (e == cudaSuccess) e = cudaMalloc(&t->gs, sizeof(double) * (6 * n + nb * 2 * KK + 2 * KK));

@@ -1,0 +1,43 @@
+"""The device memory of the trajectory adjoint: what a pass keeps, and a pass that gets none."""
+import numpy as np
+import pytest
+
+from madpac_b200 import mdgpu as M
+from madpac_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+DT = 0.002
+
+
+def cluster(length, n=1000, species=2):
+    """n molecules of a liquid in the middle of a box of the given edge."""
+    s = W.lj_fcc_box(7, 0.7, 1.0, 5, 2.5, W.two_species() if species == 2 else [W.Component(1.0, 1.0, 1.0, True)], n_atoms=n)
+    rng = np.random.default_rng(6)
+    r = s.r + rng.uniform(-0.05, 0.05, s.r.shape) - s.length / 2
+    lc = M.LinkedCells([length] * 3, 2.5, s.components, s.mix)
+    lc.addParticles(s.ids, s.cid, np.ascontiguousarray(r + length / 2), s.v)
+    return lc
+
+
+def gradient(lc, steps, every):
+    n = lc.n
+    lc.trajForward(steps, every, DT)
+    return lc.trajBackward(np.random.default_rng(7).standard_normal((n, 3)), 1.0)
+
+
+def starve(lc):
+    """A segment of tens of terabytes."""
+    with pytest.raises(M.MdgpuError) as ei:
+        lc.trajForward(2_000_000_000, 2_000_000_000, DT)
+    assert ei.value.code == 2
+
+
+def test_a_pass_without_memory_leaves_nothing_to_go_backward_on():
+    lc = cluster(20.0)
+    lc.trajForward(6, 3, DT)
+    starve(lc)
+    with pytest.raises(M.MdgpuError) as ei:
+        lc.trajBackward(np.zeros((lc.n, 3)), 1.0)
+    assert ei.value.code == 3
+    lc.close()
