@@ -110,6 +110,7 @@ int fail(Context* c, int code, const std::string& msg) {
 
 int cuda_fail(Context* c, cudaError_t e, const char* where) {
 	c->err = std::string(where) + ": " + cudaGetErrorString(e);
+	cudaGetLastError();   // reported here, not again by the check behind a later launch
 	return MDGPU_ERR_CUDA;
 }
 

@@ -691,6 +691,7 @@ int bfail(Batch* b, int code, const std::string& msg) {
 		cudaError_t e_ = (call);                                                \
 		if (e_ != cudaSuccess) {                                                \
 			b->err = std::string(#call) + ": " + cudaGetErrorString(e_);        \
+			cudaGetLastError(); /* reported here, not again by a later check */ \
 			return MDGPU_ERR_CUDA;                                              \
 		}                                                                       \
 	} while (0)

@@ -41,3 +41,16 @@ def test_a_pass_without_memory_leaves_nothing_to_go_backward_on():
         lc.trajBackward(np.zeros((lc.n, 3)), 1.0)
     assert ei.value.code == 3
     lc.close()
+
+
+def test_a_failed_call_is_reported_once():
+    """The same pass afterwards, and another container, do not see the error of the call that failed."""
+    lc = cluster(20.0)
+    want = gradient(lc, 6, 3)
+    lc.close()
+    lc = cluster(20.0)
+    starve(lc)
+    for got in (gradient(lc, 6, 3), gradient(cluster(20.0), 6, 3)):
+        for a, b in zip(got[:4], want[:4]):
+            np.testing.assert_array_equal(a, b)
+    lc.close()
