@@ -62,7 +62,9 @@ __global__ void k_restore(int64_t n, const int32_t* __restrict__ uidx, const dou
 }
 
 // One step of a segment as the binning left it: sorted positions, caller indices, components and cell starts,
-// so that the backward pass needs no binning of its own (16,384 molecules: 18 us of 137 per backward step).
+// so that the backward pass needs no binning of its own (16,384 molecules: 18 us of 137 per backward step). It
+// takes 32 bytes per molecule and 4 per cell; boxes of more than two cells per molecule (a liquid has a twelfth),
+// and passes for which that is more than can be had, keep the positions only (24 bytes) and bin again.
 struct Kept {
 	double* r;          // three planes
 	int32_t *uidx, *cid, *start;
@@ -165,7 +167,8 @@ struct Traj {
 	double dt = 0.0;
 	std::vector<int> starts;   // checkpointed steps
 	double* snaps = nullptr;   // starts.size() x (r, v) planes (6 n)
-	double* seg = nullptr;     // every kept steps
+	double* seg = nullptr;     // every kept steps, or their positions (3 n)
+	bool binned = false;       // which of the two
 	double *rbar = nullptr, *vbar = nullptr, *Fbar = nullptr, *cm = nullptr;
 	double *gs = nullptr, *os = nullptr, *pgrad = nullptr, *par = nullptr, *rows = nullptr;
 	int64_t cap_snaps = 0, cap_seg = 0, cap_n = 0;
@@ -204,11 +207,11 @@ cudaError_t traj_step(Context* c, double dt) {
 	return e;
 }
 
-cudaError_t traj_snap(Context* c, double* dst) {
+cudaError_t traj_snap(Context* c, double* dst, bool with_v) {
 	const int64_t n = c->n;
 	k_snap<<<nblk(n), kT, 0, c->stream>>>(n, c->p.uidx, c->p.rx, c->p.ry, c->p.rz, dst);
-	k_snap<<<nblk(n), kT, 0, c->stream>>>(n, c->p.uidx, c->p.vx, c->p.vy, c->p.vz, dst + 3 * n);
-	count_launches(c, 2);
+	if (with_v) k_snap<<<nblk(n), kT, 0, c->stream>>>(n, c->p.uidx, c->p.vx, c->p.vy, c->p.vz, dst + 3 * n);
+	count_launches(c, with_v ? 2 : 1);
 	return cudaGetLastError();
 }
 
@@ -219,11 +222,11 @@ cudaError_t traj_keep(Context* c, double* dst) {
 	return cudaGetLastError();
 }
 
-cudaError_t traj_restore(Context* c, const double* src) {
+cudaError_t traj_restore(Context* c, const double* src, bool with_v) {
 	const int64_t n = c->n;
 	k_restore<<<nblk(n), kT, 0, c->stream>>>(n, c->p.uidx, src, c->p.rx, c->p.ry, c->p.rz);
-	k_restore<<<nblk(n), kT, 0, c->stream>>>(n, c->p.uidx, src + 3 * n, c->p.vx, c->p.vy, c->p.vz);
-	count_launches(c, 2);
+	if (with_v) k_restore<<<nblk(n), kT, 0, c->stream>>>(n, c->p.uidx, src + 3 * n, c->p.vx, c->p.vy, c->p.vz);
+	count_launches(c, with_v ? 2 : 1);
 	return cudaGetLastError();
 }
 
@@ -282,7 +285,8 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 	for (int k = 0; k < nsteps; k += t->every) t->starts.push_back(k);
 	const int64_t nb = adjoint_blocks(n);
 	const int64_t need_snaps = (int64_t) t->starts.size() * 6 * n;
-	const int64_t need_seg = t->every * kept_size(n, c->g.ncells);
+	t->binned = c->g.ncells <= 2 * n;
+	int64_t need_seg = t->every * (t->binned ? kept_size(n, c->g.ncells) : 3 * n);
 	if (need_snaps > t->cap_snaps) {
 		cudaFree(t->snaps);
 		t->snaps = nullptr;
@@ -296,6 +300,12 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 		t->seg = nullptr;
 		t->cap_seg = 0;
 		e = cudaMalloc(&t->seg, sizeof(double) * need_seg);
+		if (e == cudaErrorMemoryAllocation && t->binned) {
+			cudaGetLastError();
+			t->binned = false;
+			need_seg = (int64_t) t->every * 3 * n;
+			e = cudaMalloc(&t->seg, sizeof(double) * need_seg);
+		}
 		if (e != cudaSuccess) return set_cuda_error(c, e, "cudaMalloc (trajectory segment)");
 		t->cap_seg = need_seg;
 	}
@@ -320,11 +330,11 @@ int mdgpu_traj_forward(mdgpu_ctx* ctx, int32_t nsteps, int32_t checkpoint_every,
 	// forces of the start, then the steps; every `every` steps a snapshot (r, v)
 	e = traj_bin(c);
 	if (e == cudaSuccess) e = launch_pairs(c);
-	if (e == cudaSuccess) e = traj_snap(c, t->snaps);
+	if (e == cudaSuccess) e = traj_snap(c, t->snaps, true);
 	size_t si = 1;
 	for (int k = 1; k <= nsteps && e == cudaSuccess; k++) {
 		e = traj_step(c, dt);
-		if (e == cudaSuccess && si < t->starts.size() && t->starts[si] == k) e = traj_snap(c, t->snaps + 6 * n * si++);
+		if (e == cudaSuccess && si < t->starts.size() && t->starts[si] == k) e = traj_snap(c, t->snaps + 6 * n * si++, true);
 	}
 	if (e != cudaSuccess) return set_cuda_error(c, e, "trajectory forward");
 	double sc[3];
@@ -348,7 +358,7 @@ int mdgpu_traj_backward(mdgpu_ctx* ctx, const double* gF, double gU, double* dL_
 	cudaError_t e = cudaSetDevice(c->device);
 	if (e != cudaSuccess) return set_cuda_error(c, e, "cudaSetDevice");
 	const int64_t n = c->n;
-	const int64_t kept = kept_size(n, c->g.ncells);
+	const int64_t kept = t->binned ? kept_size(n, c->g.ncells) : 3 * n;
 	const double dt = t->dt;
 	// cotangents of the final state: Fbar = gF, rbar = vbar = 0; parameter sums 0
 	const CopySpan in{(void*) gF, t->rows, sizeof(double) * 3 * n};
@@ -371,16 +381,24 @@ int mdgpu_traj_backward(mdgpu_ctx* ctx, const double* gF, double gU, double* dL_
 		const int k0 = t->starts[si];
 		const int k1 = si + 1 < (int) t->starts.size() ? t->starts[si + 1] : t->nsteps;
 		// the segment from its snapshot: forces of r_k0, then steps k0+1 .. k1, positions kept
-		e = traj_restore(c, t->snaps + 6 * n * si);
+		e = traj_restore(c, t->snaps + 6 * n * si, true);
 		if (e == cudaSuccess) e = traj_bin(c);
 		if (e == cudaSuccess) e = launch_pairs(c);
 		for (int k = k0 + 1; k <= k1 && e == cudaSuccess; k++) {
 			e = traj_step(c, dt);
-			if (e == cudaSuccess) e = traj_keep(c, t->seg + kept * (k - k0 - 1));
+			double* const at = t->seg + kept * (k - k0 - 1);
+			if (e == cudaSuccess) e = t->binned ? traj_keep(c, at) : traj_snap(c, at, false);
 			t->recomputed++;
 		}
 		// backwards through the segment: F_k = F(r_k) for k = k1 .. k0 + 1
 		for (int k = k1; k > k0 && e == cudaSuccess; k--) {
+			if (!t->binned) {
+				e = traj_restore(c, t->seg + kept * (k - k0 - 1), false);
+				if (e == cudaSuccess) e = traj_bin(c);
+				if (e == cudaSuccess) e = traj_vjp(c, t, gUk, true, true);
+				gUk = 0.0;
+				continue;
+			}
 			// (the kernels of the step read the kept arrays in the place of the context's)
 			const Kept at = kept_at(t->seg + kept * (k - k0 - 1), n);
 			const Particles own = c->p;
@@ -398,7 +416,7 @@ int mdgpu_traj_backward(mdgpu_ctx* ctx, const double* gF, double gU, double* dL_
 		}
 	}
 	// the start: rbar += J(r_0)^T Fbar
-	if (e == cudaSuccess) e = traj_restore(c, t->snaps);
+	if (e == cudaSuccess) e = traj_restore(c, t->snaps, true);
 	if (e == cudaSuccess) e = traj_bin(c);
 	if (e == cudaSuccess) e = traj_vjp(c, t, gUk, false, false);
 	double par[2 * KK];

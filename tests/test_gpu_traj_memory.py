@@ -54,3 +54,34 @@ def test_a_failed_call_is_reported_once():
         for a, b in zip(got[:4], want[:4]):
             np.testing.assert_array_equal(a, b)
     lc.close()
+
+
+@pytest.mark.parametrize("species", [1, 2])
+def test_a_dilute_box_keeps_positions_only(species):
+    """1,000 molecules in 64,000 cells: 200 steps of a segment take no more than their positions (24 bytes per molecule
+    and step; 16 MB for the rest and the allocator's steps), not the cell starts of every step (51 MB more)."""
+    import torch
+
+    lc = cluster(100.0, species=species)
+    lc.update()
+    lc.traversePairs()
+    lc.trajForward(1, 1, DT)
+    free = torch.cuda.mem_get_info()[0]
+    lc.trajForward(200, 200, DT)
+    assert free - torch.cuda.mem_get_info()[0] <= 200 * 24 * lc.n + (16 << 20)
+    lc.close()
+
+
+@pytest.mark.parametrize("species", [1, 2])
+@pytest.mark.parametrize("every", [2, 7])
+def test_both_forms_give_the_same_gradient(species, every):
+    """The molecules alone in the middle of a small box, which keeps binned states, and of a large one, which bins again:
+    the same pairs with coordinates 40 larger, whose rounding (1e-14) the seven steps amplify by less than 1e2."""
+    out = []
+    for length in (20.0, 100.0):
+        lc = cluster(length, species=species)
+        assert (np.prod(lc.geometry()["box_cells"]) <= 2 * lc.n) == (length == 20.0)
+        out.append(gradient(lc, 7, every))
+        lc.close()
+    for a, b in zip(out[0][:4], out[1][:4]):
+        assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(a))
