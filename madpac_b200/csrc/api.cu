@@ -177,7 +177,7 @@ void free_particles(Context* c) {
 	c->q = Particles{};
 }
 
-// Staging buffer for AoS transfers (n x 3 doubles), reused between calls.
+// Staging buffer for transfers in the caller's order, reused between calls.
 struct Staging {
 	void* ptr = nullptr;
 	size_t bytes = 0;
@@ -661,19 +661,24 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 	}
 	c->n = n;
 	void* st;
-	MD_CUDA(staging(c, x->stage, sizeof(double) * 11 * n, &st));   // as much as a read-back of every field takes
+	// (as much as a read-back of every field takes)
+	const bool whole = n <= kStageWhole;
+	MD_CUDA(staging(c, x->stage, sizeof(double) * (whole ? 11 : 3) * n, &st));
 	double* aos = (double*) st;
 	const size_t b3 = sizeof(double) * 3 * n;
-	const CopySpan in[5] = {{(void*) r, aos, b3},
-	                        {(void*) v, aos + 3 * n, b3},
-	                        {(void*) F, aos + 6 * n, b3},
-	                        {(void*) id, c->p.id, sizeof(uint64_t) * n},
-	                        {(void*) cid, c->p.cid, sizeof(int32_t) * n}};
-	MD_CUDA(copy_to_device(c->device, c->stream, in, 5));
+	const int64_t next = whole ? 3 * n : 0;
+	const CopySpan in[5] = {{(void*) id, c->p.id, sizeof(uint64_t) * n},
+	                        {(void*) cid, c->p.cid, sizeof(int32_t) * n},
+	                        {(void*) r, aos, b3},
+	                        {(void*) v, aos + next, b3},
+	                        {(void*) F, aos + 2 * next, b3}};
+	MD_CUDA(copy_to_device(c->device, c->stream, in, whole ? 5 : 3));
 	k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, nullptr, c->p.rx, c->p.ry, c->p.rz);
-	k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 3 * n, nullptr, c->p.vx, c->p.vy, c->p.vz);
+	if (!whole) MD_CUDA(copy_to_device(c->device, c->stream, in + 3, 1));
+	k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + next, nullptr, c->p.vx, c->p.vy, c->p.vz);
 	if (F) {
-		k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 6 * n, nullptr, c->p.fx, c->p.fy, c->p.fz);
+		if (!whole) MD_CUDA(copy_to_device(c->device, c->stream, in + 4, 1));
+		k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 2 * next, nullptr, c->p.fx, c->p.fy, c->p.fz);
 	} else {
 		MD_CUDA(cudaMemsetAsync(c->p.fx, 0, sizeof(double) * n, c->stream));
 		MD_CUDA(cudaMemsetAsync(c->p.fy, 0, sizeof(double) * n, c->stream));
@@ -711,11 +716,21 @@ int mdgpu_get_particles(mdgpu_ctx* ctx, int64_t n, uint64_t* id, int32_t* cid, d
 	if (!ctx) return MDGPU_ERR_ARG;
 	Context* c = &ctx->c;
 	if (n != c->n) return fail(c, MDGPU_ERR_ARG, "n does not match the loaded molecules");
+	if (n > kStageWhole && (r ? 1 : 0) + (v ? 1 : 0) + (F ? 1 : 0) + (id ? 1 : 0) + (cid ? 1 : 0) > 1) {
+		int e = MDGPU_OK;
+		if (r) e = mdgpu_get_particles(ctx, n, nullptr, nullptr, r, nullptr, nullptr);
+		if (v && !e) e = mdgpu_get_particles(ctx, n, nullptr, nullptr, nullptr, v, nullptr);
+		if (F && !e) e = mdgpu_get_particles(ctx, n, nullptr, nullptr, nullptr, nullptr, F);
+		if (id && !e) e = mdgpu_get_particles(ctx, n, id, nullptr, nullptr, nullptr, nullptr);
+		if (cid && !e) e = mdgpu_get_particles(ctx, n, nullptr, cid, nullptr, nullptr, nullptr);
+		return e;
+	}
 	MD_CUDA(cudaSetDevice(c->device));
 	// the fields asked for one after another in the staging buffer, packed by one kernel
 	void* st;
 	const size_t b3 = sizeof(double) * 3 * n;
-	MD_CUDA(staging(c, extra(c)->stage, ((r ? 3 : 0) + (v ? 3 : 0) + (F ? 3 : 0) + 2) * sizeof(double) * n, &st));
+	const int planes = (r ? 3 : 0) + (v ? 3 : 0) + (F ? 3 : 0) + (id ? 1 : 0) + (cid ? 1 : 0);
+	MD_CUDA(staging(c, extra(c)->stage, sizeof(double) * planes * n, &st));
 	Packed o{};
 	CopySpan out[5];
 	int k = 0;

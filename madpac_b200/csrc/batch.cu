@@ -1104,7 +1104,9 @@ int mdgpu_batch_set_particles(mdgpu_batch* h, int64_t ntotal, const uint64_t* id
 	for (int64_t i = 0; i < ntotal; i++)
 		if (cid[i] < 0 || cid[i] >= b->sp.n) return bfail(b, MDGPU_ERR_ARG, "component id out of range");
 	B_CUDA(cudaSetDevice(b->device));
-	const size_t need = sizeof(double) * 11 * ntotal;   // a read-back's r, v, F, id and cid
+	// a read-back's r, v, F, id and cid, or one of them
+	const bool whole = ntotal <= kStageWhole;
+	const size_t need = sizeof(double) * (whole ? 11 : 3) * ntotal;
 	if (b->stage_bytes < need) {
 		cudaFree(b->stage);
 		b->stage = nullptr;
@@ -1115,13 +1117,15 @@ int mdgpu_batch_set_particles(mdgpu_batch* h, int64_t ntotal, const uint64_t* id
 	b->cur = 0;
 	Particles& p = b->buf[0];
 	const size_t b3 = sizeof(double) * 3 * ntotal;
-	const CopySpan in[4] = {{(void*) r, b->stage, b3},
-	                        {(void*) v, b->stage + 3 * ntotal, b3},
-	                        {(void*) id, p.id, sizeof(uint64_t) * ntotal},
-	                        {(void*) cid, p.cid, sizeof(int32_t) * ntotal}};
-	B_CUDA(copy_to_device(b->device, b->stream, in, 4));
+	double* const stage_v = b->stage + (whole ? 3 * ntotal : 0);
+	const CopySpan in[4] = {{(void*) id, p.id, sizeof(uint64_t) * ntotal},
+	                        {(void*) cid, p.cid, sizeof(int32_t) * ntotal},
+	                        {(void*) r, b->stage, b3},
+	                        {(void*) v, stage_v, b3}};
+	B_CUDA(copy_to_device(b->device, b->stream, in, whole ? 4 : 3));
 	k_load3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, b->stage, p.rx, p.ry, p.rz);
-	k_load3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, b->stage + 3 * ntotal, p.vx, p.vy, p.vz);
+	if (!whole) B_CUDA(copy_to_device(b->device, b->stream, in + 3, 1));
+	k_load3<<<blocks(ntotal), kThreads, 0, b->stream>>>(ntotal, stage_v, p.vx, p.vy, p.vz);
 	B_CUDA(cudaMemsetAsync(p.fx, 0, sizeof(double) * ntotal, b->stream));
 	B_CUDA(cudaMemsetAsync(p.fy, 0, sizeof(double) * ntotal, b->stream));
 	B_CUDA(cudaMemsetAsync(p.fz, 0, sizeof(double) * ntotal, b->stream));
@@ -1140,6 +1144,15 @@ int mdgpu_batch_get_particles(mdgpu_batch* h, int64_t ntotal, uint64_t* id, int3
 	Batch* b = &h->b;
 	if (ntotal != b->ntotal) return bfail(b, MDGPU_ERR_ARG, "ntotal must equal the sum of the box counts");
 	if (!b->loaded) return bfail(b, MDGPU_ERR_STATE, "no molecules loaded");
+	if (ntotal > kStageWhole && (r ? 1 : 0) + (v ? 1 : 0) + (F ? 1 : 0) + (id ? 1 : 0) + (cid ? 1 : 0) > 1) {
+		int e = MDGPU_OK;
+		if (r) e = mdgpu_batch_get_particles(h, ntotal, nullptr, nullptr, r, nullptr, nullptr);
+		if (v && !e) e = mdgpu_batch_get_particles(h, ntotal, nullptr, nullptr, nullptr, v, nullptr);
+		if (F && !e) e = mdgpu_batch_get_particles(h, ntotal, nullptr, nullptr, nullptr, nullptr, F);
+		if (id && !e) e = mdgpu_batch_get_particles(h, ntotal, id, nullptr, nullptr, nullptr, nullptr);
+		if (cid && !e) e = mdgpu_batch_get_particles(h, ntotal, nullptr, cid, nullptr, nullptr, nullptr);
+		return e;
+	}
 	B_CUDA(cudaSetDevice(b->device));
 	const Particles& p = b->buf[b->cur];
 	CopySpan out[5];

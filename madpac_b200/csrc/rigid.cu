@@ -1193,7 +1193,7 @@ struct mdgpu_rigid {
 	std::vector<mdgpu_site> sites_in;
 	std::vector<mdgpu_charge> charges_in;
 	std::vector<double> inertia_in, mix_in;
-	double* stage = nullptr;    // kRigidPlanes x cap host <-> device staging
+	double* stage = nullptr;    // host <-> device staging, stage_planes(cap) x cap
 	double* partials = nullptr; // per-block reduction partials (4 doubles per block of the pair kernel)
 	double* scal = nullptr;     // [0..2] pair sums, [3..4] kinetic sums
 	double* steps = nullptr;    // 5 doubles per step of mdgpu_rigid_run
@@ -1529,6 +1529,9 @@ int setup_rigid(Context* c, int ncomp, const int32_t* nlj, const mdgpu_site* sit
 	return MDGPU_OK;
 }
 
+// q, D and M together, or the widest of them
+int64_t stage_planes(int64_t n) { return n <= kStageWhole ? kRigidPlanes : 4; }
+
 int ensure_capacity(mdgpu_rigid* h, int64_t n) {
 	Context* c = ctx_of(h);
 	if (n <= h->cap) return MDGPU_OK;
@@ -1554,7 +1557,7 @@ int ensure_capacity(mdgpu_rigid* h, int64_t n) {
 	RG_CUDA(cudaMalloc(&h->es, sizeof(double) * 3 * std::max(1, h->hp.ns_max) * n));
 	RG_CUDA(cudaMalloc(&h->rec, sizeof(float4) * kRecFloat4 * n));
 	RG_CUDA(cudaMalloc(&h->ss, sizeof(double) * 2 * kRigidPlanes * n));
-	RG_CUDA(cudaMalloc(&h->stage, sizeof(double) * kRigidPlanes * n));
+	RG_CUDA(cudaMalloc(&h->stage, sizeof(double) * stage_planes(n) * n));
 	RG_CUDA(cudaMalloc(&h->partials, sizeof(double) * 4 * nblocks(n * kRigidLanes)));
 	h->cap = n;
 	return MDGPU_OK;
@@ -1836,11 +1839,13 @@ int mdgpu_rigid_set_particles(mdgpu_rigid* h, int64_t n, const uint64_t* id, con
 	st = ensure_capacity(h, n);
 	if (st) return st;
 	const unsigned nb4 = (unsigned) nblocks(4 * n), nb3 = (unsigned) nblocks(3 * n);
-	const CopySpan in[2] = {{(void*) q, h->stage, sizeof(double) * 4 * n},
-	                        {(void*) D, h->stage + 4 * n, sizeof(double) * 3 * n}};
-	RG_CUDA(copy_to_device(c->device, c->stream, in, 2));
+	const bool whole = h->cap <= kStageWhole;
+	double* const stage_D = h->stage + (whole ? 4 * n : 0);
+	const CopySpan in[2] = {{(void*) q, h->stage, sizeof(double) * 4 * n}, {(void*) D, stage_D, sizeof(double) * 3 * n}};
+	RG_CUDA(copy_to_device(c->device, c->stream, in, whole ? 2 : 1));
 	k_scatter_soa<double><<<nb4, kRigidThreads, 0, c->stream>>>(n, 4, h->stage, h->q);
-	k_scatter_soa<double><<<nb3, kRigidThreads, 0, c->stream>>>(n, 3, h->stage + 4 * n, h->D);
+	if (!whole) RG_CUDA(copy_to_device(c->device, c->stream, in + 1, 1));
+	k_scatter_soa<double><<<nb3, kRigidThreads, 0, c->stream>>>(n, 3, stage_D, h->D);
 	RG_CUDA(cudaMemsetAsync(h->M, 0, sizeof(double) * 3 * n, c->stream));
 	RG_CUDA(cudaGetLastError());
 	RG_CUDA(cudaStreamSynchronize(c->stream));
@@ -1867,7 +1872,13 @@ int mdgpu_rigid_get_particles(mdgpu_rigid* h, int64_t n, uint64_t* id, int32_t* 
 		if (!s.out) continue;
 		k_gather_soa<double><<<(unsigned) nblocks(s.k * n), kRigidThreads, 0, c->stream>>>(n, s.k, s.src, at);
 		out[k++] = CopySpan{s.out, at, sizeof(double) * s.k * n};
-		at += s.k * n;
+		if (h->cap <= kStageWhole) {
+			at += s.k * n;
+		} else {
+			RG_CUDA(cudaGetLastError());
+			RG_CUDA(copy_to_host(c->device, c->stream, out, k));
+			k = 0;
+		}
 	}
 	RG_CUDA(cudaGetLastError());
 	RG_CUDA(copy_to_host(c->device, c->stream, out, k));

@@ -4,8 +4,14 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdint>
 
 namespace mdgpu {
+
+// Most molecules whose fields pass through a staging buffer that holds all of them at once (88 bytes per molecule,
+// 369 MB). Of larger boxes one field after another does, in the room of the widest: a copy of 100 MB has nothing to
+// gain from being queued with the next.
+constexpr int64_t kStageWhole = int64_t(1) << 22;
 
 struct CopySpan {
 	void* host;
