@@ -636,6 +636,9 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 	MD_CUDA(cudaSetDevice(c->device));
 	MD_CUDA(cudaStreamSynchronize(c->stream));
 	if (n > c->cap) {
+		c->n = 0;   // until the new arrays are there
+		c->cells_valid = false;
+		c->lists_valid = false;
 		free_particles(c);
 		cudaFree(c->cell);
 		cudaFree(c->rank);

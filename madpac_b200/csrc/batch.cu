@@ -991,6 +991,38 @@ int upload_table(Batch* b) {
 	return MDGPU_OK;
 }
 
+void free_lists(Batch* b) {
+	void* lists[] = {b->nbr, b->nbr_count, b->r_ref, b->box_flag, b->rebuild, b->valid, b->builds};
+	for (void* x : lists) cudaFree(x);
+	b->nbr = b->nbr_count = nullptr;
+	b->r_ref = nullptr;
+	b->box_flag = b->valid = nullptr;
+	b->rebuild = nullptr;
+	b->builds = nullptr;
+}
+
+// The buffers of the Verlet-skin mode.
+int alloc_lists(Batch* b, double skin) {
+	// list capacity from the densest box (x 1.5 for local fluctuations)
+	double rho = 0.0;
+	for (int k = 0; k < b->nboxes; k++)
+		rho = std::max(rho, b->h_count[k] / (b->h_len[3 * k] * b->h_len[3 * k + 1] * b->h_len[3 * k + 2]));
+	const double rl = b->rc + skin;
+	int cap = (int) std::ceil(1.25 * 4.18879020478639 * rl * rl * rl * rho * 1.5) + 32;
+	cap = std::min((cap + 31) & ~31, 65504);
+	b->list_cap = cap;
+	B_CUDA(cudaMalloc(&b->nbr, sizeof(unsigned short) * (size_t) cap * b->ntotal));
+	B_CUDA(cudaMalloc(&b->nbr_count, sizeof(unsigned short) * b->ntotal));
+	B_CUDA(cudaMalloc(&b->r_ref, sizeof(double) * 3 * b->ntotal));
+	B_CUDA(cudaMalloc(&b->box_flag, sizeof(int) * b->nboxes));
+	B_CUDA(cudaMalloc(&b->rebuild, sizeof(int32_t) * b->nboxes));
+	B_CUDA(cudaMalloc(&b->valid, sizeof(int)));
+	B_CUDA(cudaMemset(b->valid, 0, sizeof(int)));
+	B_CUDA(cudaMalloc(&b->builds, sizeof(unsigned long long)));
+	B_CUDA(cudaMemset(b->builds, 0, sizeof(unsigned long long)));
+	return MDGPU_OK;
+}
+
 }  // namespace
 }  // namespace mdgpu
 
@@ -1337,33 +1369,20 @@ int mdgpu_batch_set_skin(mdgpu_batch* h, double skin) {
 		return st;
 	}
 	if (b->max_bin_bytes > 110 * 1024) b->tiles.ctas = 1;
-	void* lists[] = {b->nbr, b->nbr_count, b->r_ref, b->box_flag, b->rebuild, b->valid, b->builds};
-	for (void* x : lists) cudaFree(x);
-	b->nbr = b->nbr_count = nullptr;
-	b->r_ref = nullptr;
-	b->box_flag = b->valid = nullptr;
-	b->rebuild = nullptr;
-	b->builds = nullptr;
-	if (skin > 0.0) {
-		// list capacity from the densest box (x 1.5 for local fluctuations)
-		double rho = 0.0;
-		for (int k = 0; k < b->nboxes; k++)
-			rho = std::max(rho, b->h_count[k] / (b->h_len[3 * k] * b->h_len[3 * k + 1] * b->h_len[3 * k + 2]));
-		const double rl = b->rc + skin;
-		int cap = (int) std::ceil(1.25 * 4.18879020478639 * rl * rl * rl * rho * 1.5) + 32;
-		cap = std::min((cap + 31) & ~31, 65504);
-		b->list_cap = cap;
-		B_CUDA(cudaMalloc(&b->nbr, sizeof(unsigned short) * (size_t) cap * b->ntotal));
-		B_CUDA(cudaMalloc(&b->nbr_count, sizeof(unsigned short) * b->ntotal));
-		B_CUDA(cudaMalloc(&b->r_ref, sizeof(double) * 3 * b->ntotal));
-		B_CUDA(cudaMalloc(&b->box_flag, sizeof(int) * b->nboxes));
-		B_CUDA(cudaMalloc(&b->rebuild, sizeof(int32_t) * b->nboxes));
-		B_CUDA(cudaMalloc(&b->valid, sizeof(int)));
-		B_CUDA(cudaMemset(b->valid, 0, sizeof(int)));
-		B_CUDA(cudaMalloc(&b->builds, sizeof(unsigned long long)));
-		B_CUDA(cudaMemset(b->builds, 0, sizeof(unsigned long long)));
-	}
+	free_lists(b);
 	b->prepared = false;
+	if (skin > 0.0) {
+		st = alloc_lists(b, skin);
+		if (st) {
+			// without its lists there is no skin mode
+			free_lists(b);
+			b->skin = 0.0;
+			const std::string why = b->err;
+			if (!box_table(b)) upload_table(b);
+			b->err = why;
+			return st;
+		}
+	}
 	return MDGPU_OK;
 }
 

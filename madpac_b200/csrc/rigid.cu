@@ -1837,7 +1837,10 @@ int mdgpu_rigid_set_particles(mdgpu_rigid* h, int64_t n, const uint64_t* id, con
 	int st = mdgpu_set_particles(h->inner, n, id, cid, r, v, nullptr);
 	if (st) return st;
 	st = ensure_capacity(h, n);
-	if (st) return st;
+	if (st) {
+		c->n = 0;   // no orientations to go with the molecules
+		return st;
+	}
 	const unsigned nb4 = (unsigned) nblocks(4 * n), nb3 = (unsigned) nblocks(3 * n);
 	const bool whole = h->cap <= kStageWhole;
 	double* const stage_D = h->stage + (whole ? 4 * n : 0);
