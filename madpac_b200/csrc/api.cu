@@ -38,6 +38,31 @@ __global__ void k_load_aos(int64_t n, const double* __restrict__ aos, const int3
 }
 
 // sorted SoA -> caller order (AoS)
+// New positions behind pruned lists: as k_load_aos, with the largest squared displacement (float bits, rounded up)
+// in st->jump.
+__global__ void k_load_moved(int64_t n, const double* __restrict__ aos, const int32_t* __restrict__ uidx, double* x, double* y,
+                             double* z, PruneState* st) {
+	const int64_t s = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+	unsigned d2 = 0u;
+	if (s < n) {
+		const int64_t u = uidx[s];
+		const double r[3] = {aos[3 * u], aos[3 * u + 1], aos[3 * u + 2]};
+		const double d[3] = {r[0] - x[s], r[1] - y[s], r[2] - z[s]};
+		x[s] = r[0];
+		y[s] = r[1];
+		z[s] = r[2];
+		d2 = __float_as_uint(__double2float_ru(d[0] * d[0] + d[1] * d[1] + d[2] * d[2])) & 0x7fffffffu;
+	}
+	d2 = __reduce_max_sync(0xffffffffu, d2);
+	if ((threadIdx.x & 31) == 0 && d2 > 0u) atomicMax(&st->jump, d2);
+}
+
+// The displacement joins the drifts since the last prune (a NaN makes the next step prune).
+__global__ void k_add_jump(PruneState* st) {
+	st->acc += sqrt((double) __uint_as_float(st->jump));
+	st->jump = 0u;
+}
+
 __global__ void k_store_aos(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, const int32_t* __restrict__ uidx, double* __restrict__ aos) {
 	int64_t s = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
@@ -706,7 +731,13 @@ int mdgpu_set_state(mdgpu_ctx* ctx, int64_t n, const double* r, const double* v)
 	const CopySpan in[2] = {{(void*) r, aos, sizeof(double) * 3 * n}, {(void*) v, aos + 3 * n, sizeof(double) * 3 * n}};
 	MD_CUDA(copy_to_device(c->device, c->stream, in, 2));
 	if (r) {
-		k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, c->p.uidx, c->p.rx, c->p.ry, c->p.rz);
+		if (pruning(c) && c->lists_valid && c->prune_st) {
+			k_load_moved<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, c->p.uidx, c->p.rx, c->p.ry, c->p.rz, c->prune_st);
+			k_add_jump<<<1, 1, 0, c->stream>>>(c->prune_st);
+			count_launches(c, 1);
+		} else {
+			k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos, c->p.uidx, c->p.rx, c->p.ry, c->p.rz);
+		}
 		c->cells_valid = false;
 	}
 	if (v) k_load_aos<<<blocks_for(n), kThreads, 0, c->stream>>>(n, aos + 3 * n, c->p.uidx, c->p.vx, c->p.vy, c->p.vz);

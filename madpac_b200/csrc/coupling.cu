@@ -257,6 +257,7 @@ int mdgpu_reflect_boundary(mdgpu_ctx* ctx, int32_t dim, int32_t stream_out_dir, 
 	const int st = check_device_status(c);
 	if (st) return st;
 	c->cells_valid = false;   // positions changed: bin again (LinkedCells::update) before the forces
+	if (pruning(c)) c->lists_valid = false;   // a displacement that the pruned lists did not see
 	if (streamed_out) *streamed_out = (int64_t) h;
 	return MDGPU_OK;
 }

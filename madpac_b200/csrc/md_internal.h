@@ -53,6 +53,7 @@ struct PruneState {
 	int pruned;                 // id of the step whose inner lists were last made
 	double acc;                 // summed largest drifts since the positions of the last prune
 	unsigned long long count;   // prunes so far
+	unsigned jump;              // float bits of the largest squared displacement of a state set from outside
 };
 
 // LinkedCells geometry. The device keeps only the box's own cells (nc per dimension, no halo

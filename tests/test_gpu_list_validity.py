@@ -91,3 +91,33 @@ def test_a_wait_that_ran_out_builds_again():
     b.prepare()
     assert b.skinBuilds() == builds + len(systems)
     b.close()
+
+
+@pytest.mark.parametrize("precision,tol", [(M.FP64, 1e-11), (M.MIXED, 1e-5)])
+def test_positions_set_behind_pruned_lists(precision, tol):
+    """Displacements below half the skin keep the lists, but not the inner lists within the cutoff + 0.15: two molecules
+    may be 0.34 closer."""
+    s = box(4000, 2.5, 8)
+    lc = M.LinkedCells.from_system(s, precision)
+    lc.update()
+    lc.traversePairs()
+    lc.setSkin(0.4)
+    lc.setListPrune(0.15)
+    rng = np.random.default_rng(9)
+    lc.run(3, DT)
+    for k in range(3):
+        st = lc.getParticles()
+        builds = lc.skinBuilds()
+        r = st["r"] + rng.uniform(-0.1, 0.1, st["r"].shape) * (1.0 if k == 0 else 0.2)
+        r = np.where((r >= 0.0) & (r < s.length), r, st["r"])
+        lc.setState(r=r)
+        lc.run(1, DT)
+        st = lc.getParticles()
+        ref = M.LinkedCells.from_system(s, M.FP64)
+        ref.setState(st["r"], st["v"])
+        ref.update()
+        ref.traversePairs()
+        F = ref.getParticles()["F"]
+        ref.close()
+        assert rms(st["F"] - F) <= tol * rms(F), (k, lc.skinBuilds() - builds)
+    lc.close()
