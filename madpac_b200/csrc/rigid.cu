@@ -355,6 +355,7 @@ struct RigidOut {
 constexpr int kRigidLanes = MDGPU_RIGID_LANES;
 constexpr int kScan = 4;   // list entries of a lane tested at a time
 constexpr int kRigidList = MDGPU_RIGID_LIST;
+static_assert(kRigidList >= kScan, "a round of the list scan fits in a lane's list of accepted partners");
 static_assert(kRigidLanes == 1 || kRigidLanes == 2 || kRigidLanes == 4 || kRigidLanes == 8, "lanes per molecule");
 
 // kRigidLanes lanes per sorted molecule i: force and torque from every molecule of the 27 cells
