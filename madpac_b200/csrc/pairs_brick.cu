@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(brick::kThreads, kTraverseMinBlocks)
                   const double* __restrict__ rz, const int32_t* __restrict__ cid,
                   const int32_t* __restrict__ cstart, const PairParams* __restrict__ pp,
                   double* __restrict__ fx, double* __restrict__ fy, double* __restrict__ fz,
-                  double* __restrict__ partials, int* __restrict__ status, const int* __restrict__ gate,
+                  double* __restrict__ partials, int* __restrict__ status,
                   brick::Lists lists, unsigned* ticket, double* scalars) {
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ int s_item;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(brick::kThreads, kListMinBlocks)
                  const double* __restrict__ rz, const int32_t* __restrict__ cid,
                  const int32_t* __restrict__ cstart, const PairParams* __restrict__ pp,
                  double* __restrict__ fx, double* __restrict__ fy, double* __restrict__ fz,
-                 double* __restrict__ partials, int* __restrict__ status, const int* __restrict__ gate,
+                 double* __restrict__ partials, int* __restrict__ status,
                  brick::Lists lists, unsigned* tickets, double* scalars, brick::Kick kick, double* record,
                  brick::PruneOut po, double half_prune) {
 	if (lists.pst) {
@@ -303,7 +303,7 @@ Plan plan(Context* c, const Grid& g, double filter_radius, int kind) {
 bool fold_in_traversal(const Context* c, const Plan& P) { return P.nbricks <= kTraverseMinBlocks * c->num_sms; }
 
 template <typename K, typename... Extra>
-cudaError_t go(Context* c, const Plan& P, K kern, const int* gate, const brick::Lists& lists, Extra... extra) {
+cudaError_t go(Context* c, const Plan& P, K kern, const brick::Lists& lists, Extra... extra) {
 	cudaError_t r = allow_dynamic_smem((const void*) kern, c->device, P.bytes);
 	// the list kernel runs as a resident grid over a queue of the dense bricks when the sparse ones are
 	// evaluated apart (lists.kind set, or lists.counts in the traversal); otherwise one CTA per brick
@@ -312,13 +312,13 @@ cudaError_t go(Context* c, const Plan& P, K kern, const int* gate, const brick::
 	if (r == cudaSuccess)
 		kern<<<grid, brick::kThreads, P.bytes, c->stream>>>(P.p, P.bx, c->p.rx, c->p.ry, c->p.rz, c->p.cid,
 		                                                         c->cell_start, c->d_pp, c->p.fx, c->p.fy, c->p.fz,
-		                                                         c->partials, c->status, gate, lists, extra...);
+		                                                         c->partials, c->status, lists, extra...);
 	return r;
 }
 
 // kind 0: plain traversal, 2: list evaluation of the skin mode (kPr: its prune variant)
 template <int kKind, bool kPr = false>
-cudaError_t dispatch(Context* c, const Plan& P, const int* gate, const brick::Lists& lists,
+cudaError_t dispatch(Context* c, const Plan& P, const brick::Lists& lists,
                      const brick::Kick& kick = brick::Kick{}, double* record = nullptr,
                      const brick::PruneOut& po = brick::PruneOut{}, double half_prune = 0.0) {
 	const bool fp64 = c->precision == MDGPU_FP64;
@@ -327,26 +327,26 @@ cudaError_t dispatch(Context* c, const Plan& P, const int* gate, const brick::Li
 		unsigned* t = c->tickets;
 		double* out = c->scalars;
 		if (fp64 && ljrc)
-			return single ? go(c, P, k_pairs_list<true, true, true, kPr>, gate, lists, t, out, kick, record, po, half_prune)
-			              : go(c, P, k_pairs_list<true, false, true, kPr>, gate, lists, t, out, kick, record, po,
+			return single ? go(c, P, k_pairs_list<true, true, true, kPr>, lists, t, out, kick, record, po, half_prune)
+			              : go(c, P, k_pairs_list<true, false, true, kPr>, lists, t, out, kick, record, po,
 			                   half_prune);
 		if (fp64)
-			return single ? go(c, P, k_pairs_list<true, true, false, kPr>, gate, lists, t, out, kick, record, po, half_prune)
-			              : go(c, P, k_pairs_list<true, false, false, kPr>, gate, lists, t, out, kick, record, po,
+			return single ? go(c, P, k_pairs_list<true, true, false, kPr>, lists, t, out, kick, record, po, half_prune)
+			              : go(c, P, k_pairs_list<true, false, false, kPr>, lists, t, out, kick, record, po,
 			                   half_prune);
 		if (ljrc)
-			return single ? go(c, P, k_pairs_list<false, true, true, kPr>, gate, lists, t, out, kick, record, po, half_prune)
-			              : go(c, P, k_pairs_list<false, false, true, kPr>, gate, lists, t, out, kick, record, po,
+			return single ? go(c, P, k_pairs_list<false, true, true, kPr>, lists, t, out, kick, record, po, half_prune)
+			              : go(c, P, k_pairs_list<false, false, true, kPr>, lists, t, out, kick, record, po,
 			                   half_prune);
-		return single ? go(c, P, k_pairs_list<false, true, false, kPr>, gate, lists, t, out, kick, record, po, half_prune)
-		              : go(c, P, k_pairs_list<false, false, false, kPr>, gate, lists, t, out, kick, record, po,
+		return single ? go(c, P, k_pairs_list<false, true, false, kPr>, lists, t, out, kick, record, po, half_prune)
+		              : go(c, P, k_pairs_list<false, false, false, kPr>, lists, t, out, kick, record, po,
 		                   half_prune);
 	}
 	unsigned* t = fold_in_traversal(c, P) ? c->tickets + 2 : nullptr;
-	if (ljrc) return single ? go(c, P, k_pairs_brick<true, true>, gate, lists, t, c->scalars)
-	                        : go(c, P, k_pairs_brick<false, true>, gate, lists, t, c->scalars);
-	return single ? go(c, P, k_pairs_brick<true, false>, gate, lists, t, c->scalars)
-	              : go(c, P, k_pairs_brick<false, false>, gate, lists, t, c->scalars);
+	if (ljrc) return single ? go(c, P, k_pairs_brick<true, true>, lists, t, c->scalars)
+	                        : go(c, P, k_pairs_brick<false, true>, lists, t, c->scalars);
+	return single ? go(c, P, k_pairs_brick<true, false>, lists, t, c->scalars)
+	              : go(c, P, k_pairs_brick<false, false>, lists, t, c->scalars);
 }
 
 brick::Lists lists_of(Context* c) {
@@ -397,7 +397,7 @@ cudaError_t launch_pairs_brick(Context* c) {
 			    P.p, P.bx, P.nbricks, c->p.rx, c->p.ry, c->p.rz, c->p.cid, c->cell_start, c->d_pp, c->p.fx, c->p.fy,
 			    c->p.fz, c->partials, c->status, l);
 	}
-	if (e == cudaSuccess) e = dispatch<0>(c, P, nullptr, l);
+	if (e == cudaSuccess) e = dispatch<0>(c, P, l);
 	if (e == cudaSuccess) e = cudaGetLastError();
 	prof_end(c, 1, sparse ? 2 : 1);
 	if (e != cudaSuccess || fold_in_traversal(c, P)) return e;
@@ -501,9 +501,9 @@ cudaError_t launch_pairs_skin(Context* c, int kick_mode, double dt, double* reco
 	if (e == cudaSuccess && prune) {
 		Plan Pp = P;
 		Pp.bytes += brick::kPruneRingBytes;
-		e = dispatch<2, true>(c, Pp, nullptr, ld, kick, record, po, half_prune);
+		e = dispatch<2, true>(c, Pp, ld, kick, record, po, half_prune);
 	}
-	if (e == cudaSuccess) e = dispatch<2>(c, P, nullptr, prune ? ldi : ld, kick, record);
+	if (e == cudaSuccess) e = dispatch<2>(c, P, prune ? ldi : ld, kick, record);
 	if (e == cudaSuccess) e = cudaGetLastError();
 	prof_end(c, 1, sparse ? launches + 1 : launches);
 	return e;
