@@ -424,8 +424,9 @@ def run_ours(args, dist: Dist):
     tk, cnt, rec2 = time_kernels(lc, system, args.steps)
     rebuilds = (lc.skinBuilds() - builds0) if args.skin > 0 else args.steps
     prunes = (lc.listPrunes() - prunes0) if args.skin > 0 else 0
-    # one rebinning pass alone: the same state set again before each of a few single steps, so that
-    # every step rebins (the binning group then holds exactly one active k_rebuild per step)
+    # one rebinning pass alone: the same state set again before each of a few single steps, and the skin with
+    # it, which asks for new lists, so that every step rebins (the binning group then holds exactly one active
+    # k_rebuild per step)
     bin_pass_ms = None
     if args.skin > 0:
         st_b = lc.getParticles()
@@ -433,6 +434,7 @@ def run_ours(args, dist: Dist):
         lc.profileEnable(True)
         for _ in range(5):
             lc.setState(r=st_b["r"], v=st_b["v"])
+            lc.setSkin(args.skin)
             lc.run(1, system.dt, record=False)
         bin_pass_ms = lc.profileRead(reset=True)[0][0] / 5
         lc.profileEnable(False)
