@@ -34,7 +34,9 @@ extern "C" {
 #define MDGPU_ERR_CAPACITY 10        /* a workload exceeds a fixed device buffer */
 
 /* ---- precision modes ---------------------------------------------------------------------- */
-#define MDGPU_FP64 0   /* every pair in double precision, same operation order as PotForceLJ */
+#define MDGPU_FP64 0   /* every pair in double precision: distances and cutoff tests with the reference's operations
+                        * (the same pairs), the force law contracted, with a reciprocal within one unit in the last
+                        * place (forces within 1e-12 of PotForceLJ's, relative to their rms) */
 #define MDGPU_MIXED 1  /* pair arithmetic in FP32, forces/energy/virial accumulated in FP64 (the traversal of
                         * the per-step binning, where FP32 gains nothing, evaluates in FP64 in both modes) */
 
@@ -75,7 +77,10 @@ int mdgpu_set_pair_kernel(mdgpu_ctx* ctx, int kind);
  * io/InputOldstyle.cpp:324-378, LinkedCells.cpp:182-204). F may be NULL (zero forces). */
 int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int32_t* cid,
                         const double* r, const double* v, const double* F);
-/* Overwrite positions and velocities of the loaded molecules (caller order). */
+/* Overwrite positions and velocities of the loaded molecules (caller order; r or v may be NULL). Pageable arrays,
+ * and arrays below 512 KB, have been read on return. Larger arrays that the caller pinned, and device or managed
+ * memory, are read in stream order, as with cudaMemcpyAsync: leave them alone until a call that returns results, or
+ * mdgpu_synchronize, is back. */
 int mdgpu_set_state(mdgpu_ctx* ctx, int64_t n, const double* r, const double* v);
 /* Read molecules back in caller order (replaces iteration with ParticleContainer::begin/next,
  * ParticleContainer.h:100-113). Any output pointer may be NULL. */

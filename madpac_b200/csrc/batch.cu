@@ -27,8 +27,7 @@
 // bricks of the other boxes, whose lists still hold, and only then those of the flagged boxes, which wait
 // for their box (long since done), build their lists and evaluate them. The list evaluation applies the
 // closing kick. A barrier between rebuilding and evaluating kept the whole device waiting for the largest
-// rebuilt box, 300 of a step's 850 us:
-// 512 boxes of 1.17 M molecules took 852 us per step, now 712.
+// rebuilt box, 300 of a step's 850 us: 512 boxes of 1.27 M molecules took 852 us per step, now 712.
 //
 // Each wait (barrier or box) is bounded by a time limit; a wait that runs out sets the timeout status, the
 // CTA skips the rest of the step, and every later launch returns at once until the host has read the status.

@@ -604,8 +604,10 @@ struct Lists {
 	unsigned long long* builds;        // incremented once per build
 	int sentinel;                      // staged slot of the list kernel's far-away sentinel
 	unsigned char* kind;               // per brick: 1 = sparse (evaluated one warp per brick)
-	unsigned* counts;                  // sparse [0] and dense [1] bricks of the build (or null)
-	int32_t* blist;                    // dense bricks at [0, nbricks), sparse ones from nbricks on
+	// list kernels: sparse [0] and dense [1] bricks of the build (or null); traversal: bricks that are not
+	// sparse [0] and the queue over them [1] (or null: no sparse bricks looked for)
+	unsigned* counts;
+	int32_t* blist;                    // dense bricks at [0, nbricks), sparse ones (lists only) from nbricks on
 	int nbricks;
 	PruneState* pst;                   // pruned lists: their state (the evaluation's last CTA updates it)
 	int step;                          // id of the step being evaluated
@@ -1574,7 +1576,7 @@ __device__ __forceinline__ void list_chunk(const Const& p, const Box& bx, const 
 // structure, at the current positions: staging as in pairs, then the molecules of the brick's
 // own cells, 32 per warp regardless of their cell, each evaluate their list with the exact cutoff.
 // Chunks of 64 entries are summed in FP32 and added to FP64 accumulators.
-// Shared memory: layout(s_cap, kFP64, 0, false) (no filter lists, no half-precision copy).
+// Shared memory: layout(s_cap, kFP64) (no hit words, no half-precision copy).
 // kPrune: a prune step (the build lists in, the inner lists out through po).
 template <bool kFP64, bool kSingle, bool kLjIsRc, bool kWide = true, bool kPrune = false>
 __device__ __forceinline__ void list_pairs(const Const& p, const Box& bx, int brick, int64_t slot,

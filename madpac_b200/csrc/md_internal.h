@@ -169,9 +169,9 @@ struct Context {
 	int64_t prof_count[4] = {0, 0, 0, 0};
 };
 
-// Whether the Verlet-skin steps evaluate pruned lists (an inner radius between rc and rc + skin).
 // Fewest bricks of a traversal that looks for sparse ones first: two rounds of resident CTAs (three per SM).
 inline int64_t sparse_min_bricks(const Context* c) { return 6 * (int64_t) c->num_sms; }
+// Whether the Verlet-skin steps evaluate pruned lists (an inner radius between rc and rc + skin).
 inline bool pruning(const Context* c) { return c->skin > 0.0 && c->prune > 0.0 && c->prune < c->skin; }
 
 // ---- launch helpers implemented in the .cu files -------------------------------------------

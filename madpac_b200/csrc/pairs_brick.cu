@@ -21,9 +21,9 @@
 namespace mdgpu {
 namespace {
 
-// Resident CTAs per SM of the traversal (registers and the usual shared memory are sized for it). Two,
-// with 128 registers, took 168 us against 144 for 250,047 molecules at rc = 2.5 (and 220 against 235 at
-// rc = 3.0), four, with 64, 213.
+// Resident CTAs per SM of the traversal (registers and the usual shared memory are sized for it). 250,047
+// molecules at rc = 2.5, us per traversal: three, with 80 registers, 125; two, with 128, 146; four, with 64, 137.
+// At rc = 3.0, where the regions leave room for two in each case: 187, 179 and 226.
 constexpr int kTraverseMinBlocks = 3;
 
 template <bool kSingle, bool kLjIsRc>

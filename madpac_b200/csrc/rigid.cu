@@ -25,8 +25,8 @@
 //   with the quaternion algebra of Quaternion.cpp (rotate, differentiate, normalisation) and the
 //   sums m v^2 and I w^2 of Leapfrog::transition2to3 (integrators/Leapfrog.cpp:52-99).
 //
-// MDGPU_FP64 evaluates everything in double with the reference's operation order and no
-// contraction; MDGPU_MIXED evaluates the centre pairs of a molecule pair in float (from the double
+// MDGPU_FP64 evaluates everything in double with the reference's operation order and no contraction, but for
+// the reciprocals of squared site distances (rcp64, within one unit in the last place); MDGPU_MIXED evaluates the centre pairs of a molecule pair in float (from the double
 // centre distance) and adds their sums to double accumulators once per molecule pair.
 #include <cuda_runtime.h>
 
