@@ -258,16 +258,17 @@ size_t share(const Context* c, int ctas) {
 
 // Whether a capacity of s_cap staged molecules, that of `ctas` CTAs per SM, holds a region of 64 cells with
 // room for its fluctuations. The kernels take the most CTAs per SM for which it does: of a region above the
-// capacity the traversal stages the parts one by one (30,000 molecules loaded at a density of 0.1 and then set to a
-// droplet: 117 us per step), and the list kernels gather the candidates from global memory, ten times as slow. The skin cells of a small box can be
-// much larger than the radius asks for (3 or 4 along an edge, two or three times the molecules), so the lists'
-// last step is the whole SM for one CTA. A grid of one CTA per SM or less loses nothing by it and asks for the most
-// room (with 3 cells along an edge a region holds some of them twice); a larger one asks for little (a liquid's
-// regions differ by a percent or two, and the density around a molecule of a lattice is 6 % high already: with 1.15
-// for the step to three CTAs the FP64 form with pruned lists took two for 1,048,576 molecules, whose regions
-// of 2,048 three hold: 0.445 ms per step against 0.374). 20 steps of FP64 runs with skin 0.3, at a
-// density of 0.7 and a cutoff of 2.5, in ms, with one fixed capacity and with this rule: 1,500 molecules
-// 11.2 and 1.5, 3,300 10.0 and 1.3, 5,000 23.7 and 1.8 (FP32 25.3 and 1.5), 8,000 4.8 and 1.3.
+// capacity the traversal stages the parts one by one (30,000 molecules loaded at a density of 0.1 and then set
+// to a droplet: 117 us per step), and the list kernels gather the candidates from global memory, ten times as
+// slow. The skin cells of a small box can be much larger than the radius asks for (3 or 4 along an edge, two or
+// three times the molecules), so the lists' last step is the whole SM for one CTA. A grid of one CTA per SM or
+// less loses nothing by it and asks for the most room (with 3 cells along an edge a region holds some of them
+// twice); a larger one asks for little (a liquid's regions differ by a percent or two, and the density around a
+// molecule of a lattice is 6 % high already: with 1.15 for the step to three CTAs the FP64 form with pruned
+// lists took two for 1,048,576 molecules, whose regions of 2,048 three hold: 0.445 ms per step against 0.374).
+// 20 steps of FP64 runs with skin 0.3, at a density of 0.7 and a cutoff of 2.5, in ms, with one fixed capacity
+// and with this rule: 1,500 molecules 11.2 and 1.4, 3,300 10.0 and 1.3, 5,000 23.7 and 1.7 (FP32 25.3 and
+// 1.5), 8,000 4.8 and 1.3.
 bool region_fits(const Context* c, const Grid& g, int kind, int ctas, int s_cap) {
 	const double rho = c->rho_typ > 0.0 ? c->rho_typ : (double) c->n / (g.L[0] * g.L[1] * g.L[2]);
 	const double region = 64.0 * rho * g.cell_length[0] * g.cell_length[1] * g.cell_length[2];
