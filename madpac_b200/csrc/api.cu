@@ -660,10 +660,10 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 	}
 	MD_CUDA(cudaSetDevice(c->device));
 	MD_CUDA(cudaStreamSynchronize(c->stream));
+	c->n = 0;   // until the new molecules are in place
+	c->cells_valid = false;
+	c->lists_valid = false;
 	if (n > c->cap) {
-		c->n = 0;   // until the new arrays are there
-		c->cells_valid = false;
-		c->lists_valid = false;
 		free_particles(c);
 		cudaFree(c->cell);
 		cudaFree(c->rank);
@@ -687,7 +687,6 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 		}
 		c->cap = n;
 	}
-	c->n = n;
 	void* st;
 	// (as much as a read-back of every field takes)
 	const bool whole = n <= kStageWhole;
@@ -715,8 +714,7 @@ int mdgpu_set_particles(mdgpu_ctx* ctx, int64_t n, const uint64_t* id, const int
 	k_iota<<<blocks_for(n), kThreads, 0, c->stream>>>(n, c->p.uidx);
 	MD_CUDA(cudaGetLastError());
 	MD_CUDA(cudaStreamSynchronize(c->stream));
-	c->cells_valid = false;
-	c->lists_valid = false;
+	c->n = n;
 	return MDGPU_OK;
 }
 

@@ -51,6 +51,24 @@ def test_a_container_that_could_not_grow_holds_no_molecules():
     lc.close()
 
 
+def test_a_container_whose_copies_got_no_memory_holds_no_molecules():
+    """The arrays fit (190 MB), the staging buffer (88 MB) does not: they hold nothing yet."""
+    s = box(1_000_000)
+    lc = M.LinkedCells(s.length, 2.5, s.components)
+    with Full(240 << 20):
+        with pytest.raises(M.MdgpuError) as ei:
+            lc.addParticles(s.ids, s.cid, s.r, s.v)
+        assert ei.value.code == 2
+    for call in (lc.update, lambda: lc.run(1, DT), lc.traversePairs):
+        with pytest.raises(M.MdgpuError) as ei:
+            call()
+        assert ei.value.code == 3
+    lc.addParticles(s.ids, s.cid, s.r, s.v)
+    lc.update()
+    np.testing.assert_array_equal(lc.getParticles()["r"], s.r)
+    lc.close()
+
+
 def test_a_rigid_container_without_orientations_holds_no_molecules():
     s = W.rigid_fcc_box(16, 0.3, 2.0, 11, 3.0, [W.two_centre()])
     big = W.rigid_fcc_box(64, 0.3, 2.0, 11, 3.0, [W.two_centre()])      # 1,048,576 molecules: 230 and 500 MB
