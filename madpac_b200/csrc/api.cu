@@ -438,10 +438,14 @@ int device_max_optin(int device) {
 cudaError_t allow_dynamic_smem(const void* kernel, int device, size_t bytes) {
 	static std::mutex mu;
 	static std::map<std::pair<const void*, int>, size_t> limits;
-	std::lock_guard<std::mutex> lock(mu);
-	size_t& limit = limits[{kernel, device}];
-	if (bytes > limit) limit = bytes;
-	return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) limit);
+	try {
+		std::lock_guard<std::mutex> lock(mu);
+		size_t& limit = limits[{kernel, device}];
+		if (bytes > limit) limit = bytes;
+		return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) limit);
+	} catch (...) {   // no exception leaves a C entry
+		return cudaErrorMemoryAllocation;
+	}
 }
 
 int rebuild_prepare(Context* c) {
